@@ -50,6 +50,10 @@ __device__ __forceinline__ bool finite_bits(double x) { return (__double2hiint(x
 __device__ __forceinline__ double plus_zero(double x) {
   return (__double_as_longlong(x) << 1) == 0 ? 0.0 : x;
 }
+// whether any component has a bit other than its sign set (is not +-0)
+__device__ __forceinline__ bool some_bits(V a) {
+  return ((__double_as_longlong(a.x) | __double_as_longlong(a.y) | __double_as_longlong(a.z)) << 1) != 0;
+}
 __device__ __forceinline__ float plus_zero(float x) { return (__float_as_int(x) << 1) == 0 ? 0.0f : x; }
 
 constexpr double kPi = 3.14159265358979323846;
@@ -67,29 +71,129 @@ __device__ __forceinline__ double f2d_exact(float f) {
                                           ((uint64_t)(u & 0x7FFFFFu) << 29)));
 }
 
+// -------------------------------------------- FP64 roots and quotients
+// GB300's FP64 pipe takes a warp instruction every 16 clocks of an SM, and the
+// library's sqrt, 1/x and a/b measured 144, 178 and about 190 of them (9, 11
+// and 12 FP64 instructions) in kernels that this pipe bounds. Here the
+// hardware's seeds (rsqrt / rcp.approx.ftz.f64: MUFU instructions, off that
+// pipe) take one third-order step (Householder: y (1 + e/2 + 3 e^2/8) with
+// e = 1 - x y^2, and y (1 + e + e^2) with e = 1 - x y), which leaves 2^-60 of a
+// seed good to 2^-20, and the result is corrected by its exact residual
+// (Markstein 1990: x - s^2 and a - b q are representable). The corrected value
+// carries an error of ~2^-50 ulp before its last rounding, so it is the
+// correctly rounded one that the library gives: 8 FP64 instructions for a root,
+// 2 more for its reciprocal, 6 for a quotient. Together with the integer
+// comparisons below this took the pair kernel of a 1,048,576-sphere Hertz bed
+// from 206 to 194 million FP64 thread instructions (461 to 435 us), and the
+// reference's JKR Newton on 262,144 spheres from 2.82 to 2.67 ms a step. Zero, negative, infinite, NaN
+// and very large or small arguments go to the library.
+__device__ __forceinline__ bool exponent_in(double x, uint32_t lo, uint32_t hi) {
+  return (uint32_t)__double2hiint(x) - lo < hi - lo;
+}
+__device__ __forceinline__ double rsqrt_seed(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+__device__ __forceinline__ double rcp_step(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+// sqrt(x) and 1/sqrt(x) to an ulp (2^-766 <= x < 2^767; not checked)
+__device__ __forceinline__ double sqrt_step(double x, double& inv) {
+  const double y = rsqrt_seed(x);
+  const double r = x * y;
+  const double e = fma(-r, y, 1.0);
+  const double q = e * fma(e, 0.375, 0.5);
+  inv = fma(y, q, y);
+  const double s = fma(r, q, r);
+  const double half_inv = __hiloint2double(__double2hiint(inv) - 0x00100000, __double2loint(inv));
+  return fma(fma(-s, s, x), half_inv, s);
+}
+constexpr uint32_t EXP_LO = 0x10100000u, EXP_HI = 0x6FE00000u;      // 2^-766 .. 2^767
+constexpr uint32_t QUOT_LO = 0x30000000u, QUOT_HI = 0x4FF00000u;    // 2^-255 .. 2^256
+__device__ __forceinline__ double sqrt_rn(double x) {
+  if (!exponent_in(x, EXP_LO, EXP_HI)) return sqrt(x);
+  double inv;
+  return sqrt_step(x, inv);
+}
+__device__ __forceinline__ float sqrt_rn(float x) { return sqrt(x); }
+// sqrt(x) and the rounded 1/sqrt(x) of that rounded root
+__device__ __forceinline__ double sqrt_rn(double x, double& inv) {
+  if (!exponent_in(x, EXP_LO, EXP_HI)) {
+    const double s = sqrt(x);
+    inv = 1.0 / s;
+    return s;
+  }
+  double y;
+  const double s = sqrt_step(x, y);
+  inv = fma(y, fma(-s, y, 1.0), y);
+  return s;
+}
+__device__ __forceinline__ double div_rn(double a, double b) {
+  if (!(exponent_in(fabs(a), QUOT_LO, QUOT_HI) && exponent_in(fabs(b), QUOT_LO, QUOT_HI))) return a / b;
+  const double y = rcp_step(b);
+  const double q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
+__device__ __forceinline__ float div_rn(float a, float b) { return a / b; }
+// Comparisons of FP64 values as integers, off the FP64 pipe (a comparison
+// there costs as much as an addition): the bits of non-negative values order
+// as the values do.
+// max(x, 0), 0 for NaN (as fmax)
+__device__ __forceinline__ double relu(double x) {
+  const long long b = __double_as_longlong(x);
+  return b > 0 && b <= 0x7FF0000000000000ll ? x : 0.0;
+}
+__device__ __forceinline__ float relu(float x) { return fmax(x, 0.0f); }
+// a < b for a >= 0 or NaN (false) and b >= 0
+__device__ __forceinline__ bool less_nn(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b);
+}
+__device__ __forceinline__ bool less_nn(float a, float b) { return a < b; }
+// x <= 0 (false for a NaN with a clear sign bit, as the comparison)
+__device__ __forceinline__ bool not_positive(double x) { return __double_as_longlong(x) <= 0; }
+__device__ __forceinline__ bool not_positive(float x) { return x <= 0.0f; }
+// whether an overlap exceeds 0.2 min(r_i, r_j); below an eighth of both radii
+// the exponents decide it
+__device__ __forceinline__ bool is_excess(double overlap, double ri, double rj) {
+  if (__double2hiint(overlap) + 0x00300000 < min(__double2hiint(ri), __double2hiint(rj))) return false;
+  return overlap > 0.2 * fmin(ri, rj);
+}
+__device__ __forceinline__ bool is_excess(float overlap, float ri, float rj) { return overlap > 0.2f * fmin(ri, rj); }
+__device__ __forceinline__ double dot_fma(V a, V b) { return fma(a.z, b.z, fma(a.y, b.y, a.x * b.x)); }
+// a x b, each component one product and one fused multiply-add
+__device__ __forceinline__ V cross_fma(V a, V b) {
+  return V{fma(a.y, b.z, -(b.y * a.z)), fma(a.z, b.x, -(b.z * a.x)), fma(a.x, b.y, -(b.x * a.y))};
+}
+__device__ __forceinline__ V mad(double s, V a, V b) { return V{fma(s, a.x, b.x), fma(s, a.y, b.y), fma(s, a.z, b.z)}; }
+
 // ------------------------------------------------------------- force laws
 // src/physics.rs:49-70
 template <typename R>
 __device__ __forceinline__ R lsd_mag(R overlap, R vn, R kn, R gn) {
-  return fmax(kn * overlap - gn * vn, R(0));
+  return relu(kn * overlap - gn * vn);
 }
 // src/physics.rs:86-129. With s = sqrt(R* delta): the elastic term
 // (4/3) E* sqrt(R*) delta^1.5 = (4/3) E* s delta and the tangent stiffness
 // 2 E* sqrt(R* delta) = 2 E* s share one square root.
 template <typename R>
 __device__ __forceinline__ R hertz_mag(R overlap, R vn, R es, R rs, R ms, R beta_abs) {
-  if (overlap <= R(0)) return R(0);
-  R s = sqrt(rs * overlap);
+  if (not_positive(overlap)) return R(0);
+  R s = sqrt_rn(rs * overlap);
   R fe = R(4.0 / 3.0) * es * s * overlap;
   R kt = R(2) * es * s;
-  R cn = R(2) * sqrt(ms * kt) * beta_abs;
+  R cn = R(2) * sqrt_rn(ms * kt) * beta_abs;
   R fd = -cn * vn;
-  return fmax(fe + fd, R(0));
+  return relu(fe + fd);
 }
 template <typename R>
 __device__ __forceinline__ R hertz_elastic_mag(R overlap, R es, R rs) {
-  R kn = R(4.0 / 3.0) * es * sqrt(rs);
-  return overlap > R(0) ? kn * (overlap * sqrt(overlap)) : R(0);
+  if (not_positive(overlap)) return R(0);
+  R kn = R(4.0 / 3.0) * es * sqrt_rn(rs);
+  return kn * (overlap * sqrt_rn(overlap));
 }
 // src/physics.rs:132-219 (Newton on a^2/R* - sqrt(C a) - delta = 0).
 // `near` (FP32 callers) is set when a cut-off decision lies within rounding.
@@ -99,23 +203,23 @@ __device__ __forceinline__ R jkr_mag(R overlap, R es, R rs, R gamma, bool* near 
   const R eight_pi = R(8) * R(kPi);
   R c_val = eight_pi * gamma / es;
   R sqrt_c = sqrt(c_val);
-  R a = overlap > R(0) ? sqrt(rs * overlap) : rs * R(0.5);
+  R a = overlap > R(0) ? sqrt_rn(rs * overlap) : rs * R(0.5);
   for (int it = 0; it < 20; ++it) {
-    if (a <= R(0)) a = R(1e-9);
-    R ts = sqrt(c_val * a);
-    R f_val = a * a / rs - ts - overlap;
-    R df = R(2) * a / rs - R(0.5) * sqrt_c / sqrt(a);
-    if (fabs(df) < R(1e-9)) break;
-    R da = f_val / df;
+    if (not_positive(a)) a = R(1e-9);
+    R ts = sqrt_rn(c_val * a);
+    R f_val = div_rn(a * a, rs) - ts - overlap;
+    R df = div_rn(R(2) * a, rs) - div_rn(R(0.5) * sqrt_c, sqrt_rn(a));
+    if (less_nn(fabs(df), R(1e-9))) break;
+    R da = div_rn(f_val, df);
     R max_step = a * R(0.5);
     R step = da;
     if (step < -max_step) step = -max_step;
     if (step > max_step) step = max_step;
     a = a - step;
-    if (fabs(step) < R(1e-6) * rs) break;
+    if (less_nn(fabs(step), R(1e-6) * rs)) break;
   }
-  R ts = sqrt(c_val * a);
-  R f_val = a * a / rs - ts - overlap;
+  R ts = sqrt_rn(c_val * a);
+  R f_val = div_rn(a * a, rs) - ts - overlap;
   if (near && fabs(fabs(f_val) - R(1e-3) * rs) <= R(1e-5) * rs) *near = true;
   if (fabs(f_val) > R(1e-3) * rs) return R(0);
   if (a <= R(0)) return R(0);
@@ -222,11 +326,13 @@ template <typename R>
 __device__ __forceinline__ R sjkr_mag(R overlap, R vn, R es, R rs, R gamma) {
   if (gamma <= R(0)) return hertz_elastic_mag(overlap, es, rs);
   R f_pull = R(1.5) * R(kPi) * gamma * rs;
-  R term = R(3) * (R(kPi) * R(kPi)) * (gamma * gamma) * rs / (es * es);
-  R delta_c = -sqrt(term);
-  if (overlap < delta_c) return R(0);
+  if (!not_positive(-overlap)) {  // a gap: only one can lie beyond delta_c <= 0
+    R term = R(3) * (R(kPi) * R(kPi)) * (gamma * gamma) * rs / (es * es);
+    R delta_c = -sqrt(term);
+    if (overlap < delta_c) return R(0);
+  }
   R coh = vn > R(0) ? R(1) : R(0);
-  R fh = overlap > R(0) ? R(4.0 / 3.0) * es * sqrt(rs) * (overlap * sqrt(overlap)) : R(0);
+  R fh = not_positive(overlap) ? R(0) : R(4.0 / 3.0) * es * sqrt_rn(rs) * (overlap * sqrt_rn(overlap));
   return fh - coh * f_pull;
 }
 
@@ -241,7 +347,7 @@ __device__ __forceinline__ R normal_mag(int model, R overlap, T3<R> n, T3<R> rv,
     case 1: m = hertz_mag(overlap, dot(rv, n), es, rs, ms, beta_abs); break;
     case 0: {
       R kn = es * rs;
-      R gn = R(0.5) * sqrt(ms * kn);
+      R gn = R(0.5) * sqrt_rn(ms * kn);
       m = lsd_mag(overlap, dot(rv, n), kn, gn);
     } break;
     case 2: {
@@ -264,7 +370,7 @@ __device__ __forceinline__ R normal_mag_vn(int model, R overlap, T3<R> n, R vn, 
     case 1: return hertz_mag(overlap, vn, es, rs, ms, beta_abs);
     case 0: {
       R kn = es * rs;
-      R gn = R(0.5) * sqrt(ms * kn);
+      R gn = R(0.5) * sqrt_rn(ms * kn);
       return lsd_mag(overlap, vn, kn, gn);
     }
     case 2: return lsd_mag(overlap, dot(t3(R(0), R(0), R(0)), n), es * rs, R(0));
@@ -284,7 +390,7 @@ template <typename R>
 __device__ __forceinline__ T3<R> coulomb_force(R fn, T3<R> rv, T3<R> n, R mu) {
   T3<R> vt = rv - dot(rv, n) * n;
   const R vt2 = dot(vt, vt);
-  if (vt2 < R(1e-8)) return t3(R(0), R(0), R(0));
+  if (less_nn(vt2, R(1e-8))) return t3(R(0), R(0), R(0));
   R inv = rsqrt(vt2);
   T3<R> dir = vt * inv;
   return (-mu * fn) * dir;
@@ -343,11 +449,11 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
   V nd;         // the unit normal in FP64 (FP32 form: to ~1e-14, for the relative velocity below)
   double ovd;   // the overlap in FP64 (FP32 form: to ~1e-14 of r_sum)
   if (sizeof(R) == sizeof(double)) {
-    const double dist = sqrt(d2);
+    double inv;
+    const double dist = sqrt_rn(d2, inv);
     overlap = (R)(rsum - dist);
     ovd = (double)overlap;
-    const double inv = 1.0 / dist;
-    const V nd = dist > 1e-6 ? d * inv : vmk(0.0, 1.0, 0.0);
+    const V nd = less_nn(1e-6, dist) ? d * inv : vmk(0.0, 1.0, 0.0);
     n = cvt<R>(nd);
   } else {
     bool far_enough;
@@ -373,7 +479,7 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
     overlap = (R)ovd;
   }
   const R rir = (R)ri, rjr = (R)rj;
-  if (overlap > R(0.2) * fmin(rir, rjr)) excess = true;
+  if (is_excess(overlap, rir, rjr)) excess = true;
   const T3<R> ra = (-n) * rir;
   const T3<R> rb = n * rjr;
   T3<R> rv, vt;
@@ -402,8 +508,8 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
     vn = (R)vnd;
     vt = cvt<R>(rvd - vnd * nd);
   }
-  const R rs = (rir * rjr) / (rir + rjr);
-  const R ms = ((R)mi * (R)mj) / ((R)mi + (R)mj);
+  const R rs = div_rn(rir * rjr, rir + rjr);
+  const R ms = div_rn((R)mi * (R)mj, (R)mi + (R)mj);
   R fmag;
   int jkind = JKR_FALLBACK;
   if (P.nmodel == 3 && P.jkr_solver != 0 && !newton && L.gamma_pp > 0.0) {
@@ -498,6 +604,130 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
   return true;
 }
 
+// Normal force magnitude of a particle pair in physical mode in FP64, with
+// fused multiply-adds and shared roots (the laws of src/physics.rs:49-129,
+// 234-325). JKR goes to jkr_mag or jkr_learned.
+__device__ __forceinline__ double normal_mag_fused(int model, const Law& L, double overlap, double vn, double rs,
+                                                   double mi, double mj) {
+  const double es = L.es_pp;
+  if (model == 1) {
+    // (4/3) E* s delta = (2/3) k_t delta with k_t = 2 E* s, s = sqrt(R* delta)
+    if (overlap <= 0.0) return 0.0;
+    const double ms = div_rn(mi * mj, mi + mj);
+    const double kt = (2.0 * es) * sqrt_rn(rs * overlap);
+    const double cn = sqrt_rn(ms * kt) * (2.0 * L.beta_abs);
+    return relu(fma(-cn, vn, (kt * overlap) * (2.0 / 3.0)));
+  }
+  if (model == 0) {
+    const double ms = div_rn(mi * mj, mi + mj);
+    const double kn = es * rs;
+    return relu(fma(kn, overlap, -(0.5 * sqrt_rn(ms * kn)) * vn));
+  }
+  if (model == 2) return relu((es * rs) * overlap);  // the pair law sees no relative velocity
+  // sJKR; without surface energy the elastic Hertz law
+  const double fh = overlap > 0.0 ? ((4.0 / 3.0) * es * sqrt_rn(rs * overlap)) * overlap : 0.0;
+  const double gamma = L.gamma_pp;
+  if (gamma <= 0.0) return fh;
+  if (overlap < 0.0) {  // delta_c <= 0: only a gap can lie beyond it
+    const double term = 3.0 * (kPi * kPi) * (gamma * gamma) * rs / (es * es);
+    if (overlap < -sqrt(term)) return 0.0;
+  }
+  return vn > 0.0 ? fma(-(1.5 * kPi * gamma), rs, fh) : fh;
+}
+
+// pair_contact for physical mode in FP64: the same contact with fused
+// multiply-adds and only the parts that the configured laws use. Parity mode
+// repeats the reference's roundings operation by operation (a dense bed with
+// Coulomb friction chatters, and any other rounding grows tenfold every three
+// steps); physical mode has no such counterpart, and each operation here rounds
+// once where the separate form rounds twice. Both are bound by the FP64 pipe
+// whatever a warp's lanes do, so what counts is FP64 instructions a contact.
+// The cutoff decision is the caller's and stays unfused. On a 163,843-sphere
+// bed with linear springs the pair kernel went from 62.7 to 43.8 million FP64
+// thread instructions and from 210 to 130 us.
+//   nf = n x f, from which the caller forms both torques: -r_i (n x f) on i
+// and, the other end's force being -f, -r_j (n x f) on j; the normal force
+// adds nothing to it.
+// Springs, `deferred` and `newton` as in pair_contact.
+template <bool HIST>
+__device__ __forceinline__ void pair_contact_fused(const StepParams& P, const Law& L, V d, double d2, double rsum,
+                                                   double ri, double rj, double mi, double mj, V vi, V vj, V wi, V wj,
+                                                   double* hist, size_t plane, V& f_out, V& nf_out, bool& excess,
+                                                   float guess = -1.0f, uint32_t* tally = nullptr,
+                                                   bool* deferred = nullptr, bool newton = false) {
+  V n;
+  double overlap;
+  if (d2 > 1.001e-12) {
+    double inv;
+    overlap = rsum - sqrt_rn(d2, inv);
+    n = d * inv;
+  } else {  // next to the reference's |d| > 1e-6 decision, which it takes on the rounded root
+    const double dist = sqrt(d2);
+    overlap = rsum - dist;
+    n = dist > 1e-6 ? d * (1.0 / dist) : vmk(0.0, 1.0, 0.0);
+  }
+  if (is_excess(overlap, ri, rj)) excess = true;
+  // (v_i - v_j) - (w_i r_i + w_j r_j) x n
+  const V W = mad(rj, wj, wi * ri);
+  const V u = vi - vj;
+  const V rv = vmk(fma(n.y, W.z, fma(-W.y, n.z, u.x)), fma(n.z, W.x, fma(-W.z, n.x, u.y)),
+                   fma(n.x, W.y, fma(-W.x, n.y, u.z)));
+  const double vn = dot_fma(rv, n);
+  const V vt = mad(-vn, n, rv);
+  const double rs = div_rn(ri * rj, rsum);
+  double fm = 0.0;
+  if (P.nmodel == 3) {
+    int kind = JKR_FALLBACK;
+    if (P.jkr_solver != 0 && !newton && L.gamma_pp > 0.0) {
+      uint32_t it = 0;
+      kind = jkr_learned(P, L, overlap, rs, guess, fm, it);
+      if (tally) {
+        tally[kind == JKR_CONVERGES ? 0 : (kind == JKR_ZERO ? 1 : (kind == JKR_WALK ? 5 : 2))] += 1;
+        tally[4] += it;
+      }
+      if (kind == JKR_FALLBACK && deferred) {
+        *deferred = true;
+        return;
+      }
+    }
+    if (kind == JKR_FALLBACK) fm = jkr_mag<double>(overlap, L.es_pp, rs, L.gamma_pp);
+  } else {
+    fm = normal_mag_fused(P.nmodel, L, overlap, vn, rs, mi, mj);
+  }
+  V f = fm * n, nf = vmk(0.0, 0.0, 0.0);
+  if (P.tmodel == 0) {
+    const double vt2 = dot_fma(vt, vt);
+    if (!(vt2 < 1e-8)) {
+      const double g = (-L.mu * fabs(fm)) * rsqrt(vt2);
+      nf = g * cross_fma(n, vt);
+      f = mad(g, vt, f);
+    }
+  } else {
+    V xi = vmk(0.0, 0.0, 0.0);
+    if (overlap > 0.0) {
+      const double kt = P.tmodel == 2 ? (8.0 * L.gs_pp) * sqrt_rn(rs * overlap) : L.gs_pp * rs;
+      if (HIST) xi = vmk(hist[0], hist[plane], hist[2 * plane]);
+      xi = mad(P.dt, vt, mad(-dot_fma(xi, n), n, xi));
+      const V trial = (-kt) * xi;
+      const double t2 = dot_fma(trial, trial), fc = L.mu * fabs(fm);
+      V ft = trial;
+      if (t2 > fc * fc) {
+        ft = t2 > 1e-12 ? (fc * rsqrt(t2)) * trial : vmk(0.0, 0.0, 0.0);
+        xi = (-div_rn(1.0, kt)) * ft;
+      }
+      nf = cross_fma(n, ft);
+      f = f + ft;
+    }
+    if (HIST) {
+      hist[0] = xi.x;
+      hist[plane] = xi.y;
+      hist[2 * plane] = xi.z;
+    }
+  }
+  f_out = vmk(plus_zero(f.x), plus_zero(f.y), plus_zero(f.z));
+  nf_out = nf;
+}
+
 // Kahan-compensated s += d with residual r (src/particle.rs:12-18 and the
 // reference's integrator): y = d - r, t = s + y, r = (t - s) - y, s = t.
 __device__ __forceinline__ void kahan_add(V& s, V& r, V d) {
@@ -569,6 +799,7 @@ __global__ void __launch_bounds__(256) k_first_half(StepParams P) {
     const bool moving = !(fl & PF_FIXED);
     V vres = vmk(0.0, 0.0, 0.0), wres = vres, xres = vres, dv = vres, dw = vres;
     double inv_inertia = 0.0, inv_mass = 0.0;
+    bool spin = false, own_spin = false;
     if (moving) {
       // the fused second half of the previous step and this step's first
       // half kick with the same a and tau: the increments are computed once
@@ -587,10 +818,16 @@ __global__ void __launch_bounds__(256) k_first_half(StepParams P) {
       // first half kick into one kick of a dt
       const double kdt = (!KAHAN && FUSE) ? dt : hdt;
       dv = a * kdt;
-      dw = KAHAN ? (tau * inv_inertia) * kdt : tau * (inv_inertia * kdt);
+      // without a torque and a residual (a particle in flight) the spin keeps
+      // its value, adding zeros to it: two of the seven 32-byte stores fall
+      // away and, where that holds for a whole warp, 30 of the ~90 FP64
+      // instructions (decided by the warp: lanes going apart cost more)
+      own_spin = some_bits(tau) || (KAHAN && some_bits(wres));
+      spin = __any_sync(__activemask(), own_spin);
+      if (spin) dw = KAHAN ? (tau * inv_inertia) * kdt : tau * (inv_inertia * kdt);
       if (KAHAN && FUSE) {
         kahan_add(v, vres, dv);
-        kahan_add(w, wres, dw);
+        if (spin) kahan_add(w, wres, dw);
       }
     }
     // the FP32 mirror of x (written with it) decides most wrap and removal
@@ -622,18 +859,19 @@ __global__ void __launch_bounds__(256) k_first_half(StepParams P) {
       if (KAHAN) {
         kahan_add(v, vres, dv);
         kahan_add(x, xres, v * dt);
-        kahan_add(w, wres, dw);
         B.vres[k] = D4{vres.x, vres.y, vres.z, inv_mass};
         B.xres[k] = D4{xres.x, xres.y, xres.z, 0.0};
-        B.wres[k] = D4{wres.x, wres.y, wres.z, inv_inertia};
+        if (spin) kahan_add(w, wres, dw);
+        if (own_spin) B.wres[k] = D4{wres.x, wres.y, wres.z, inv_inertia};
       } else {
         v = v + dv;
         x = x + v * dt;
-        w = w + dw;
+        if (spin) w = w + dw;
       }
       B.vm[k] = D4{v.x, v.y, v.z, vm.w};
       wc.x = w.x; wc.y = w.y; wc.z = w.z;
     }
+    const double code = wc.w;
     const float4 xf = make_float4((float)x.x, (float)x.y, (float)x.z, (float)xr.w);
     if (P.mode == 0) {
       const int32_t c0 = ref_axis_fast(x.x, xf.x, P.bmin[0], bminf[0], P.href, P.inv_href, inv_hf);
@@ -641,7 +879,7 @@ __global__ void __launch_bounds__(256) k_first_half(StepParams P) {
       const int32_t c2 = ref_axis_fast(x.z, xf.z, P.bmin[2], bminf[2], P.href, P.inv_href, inv_hf);
       wc.w = __longlong_as_double((long long)pack_code(c0, c1, c2));
     }
-    B.wc[k] = wc;
+    if (own_spin || __double_as_longlong(code) != __double_as_longlong(wc.w)) B.wc[k] = wc;
     B.xr[k] = D4{x.x, x.y, x.z, xr.w};
     B.xf[k] = xf;
     float4 r0 = B.xref[k];
@@ -886,10 +1124,18 @@ __global__ void __launch_bounds__(128) k_force(StepParams P) {
           const D4 vj4 = B.vm[j];
           V fc, tc, nrm;
           T3<R> fr, tr, nr;
-          if (pair_contact<R, PHYS, HIST>(P, lw, d, d2, rsum, ri, rj, mi, vj4.w, vi, xyz(vj4), wi, xyz(wj4),
+          if constexpr (PHYS && sizeof(R) == sizeof(double)) {
+            pair_contact_fused<HIST>(P, lw, d, d2, rsum, ri, rj, mi, vj4.w, vi, xyz(vj4), wi, xyz(wj4),
+                                     HIST ? B.hist + hi : nullptr, plane, fc, nrm, excess);
+            tc = (-ri) * nrm;
+          } else if (pair_contact<R, PHYS, HIST>(P, lw, d, d2, rsum, ri, rj, mi, vj4.w, vi, xyz(vj4), wi, xyz(wj4),
                                           HIST ? B.hist + hi : nullptr, plane, fr, tr, nr, excess)) {
             fc = cvt<double>(fr);
             tc = cvt<double>(tr);
+          } else if constexpr (PHYS) {
+            pair_contact_fused<HIST>(P, lw, d, d2, rsum, ri, rj, mi, vj4.w, vi, xyz(vj4), wi, xyz(wj4),
+                                     HIST ? B.hist + hi : nullptr, plane, fc, nrm, excess);
+            tc = (-ri) * nrm;
           } else {
             pair_contact<double, PHYS, HIST>(P, lw, d, d2, rsum, ri, rj, mi, vj4.w, vi, xyz(vj4), wi, xyz(wj4),
                                              HIST ? B.hist + hi : nullptr, plane, fc, tc, nrm, excess);
@@ -1329,25 +1575,43 @@ __device__ __forceinline__ bool contact_eval(const StepParams& P, const Bank& B,
   const double d2 = dot(d, d);
   const double rsum = xi4.w + xj4.w;
   const double cut = rsum + (adh ? rsum * 0.5 : 0.0);
-  const bool in = d2 < cut * cut;
+  const bool in = less_nn(d2, cut * cut);
   const size_t hik = (size_t)k * P.cap + m;
   double* hk = HIST ? B.hist + hik : nullptr;
-  T3<R> fc = t3(R(0), R(0), R(0)), tc = fc, nrm = fc;
+  T3<R> fc = t3(R(0), R(0), R(0)), tc = fc, tc2 = fc, nrm = fc;  // tc2: the torque on the other end
   if (in) {
     const D4 vi4 = B.vm[k], wi4 = B.wc[k], vj4 = B.vm[j], wj4 = B.wc[j];
     const Law lw = law_of(P, B, (int)k);
     bool deferred = false;
     const bool can_defer = first_pass && P.jfb != nullptr;
-    if (!pair_contact<R, PHYS, HIST>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4), xyz(wi4),
-                                     xyz(wj4), hk, plane, fc, tc, nrm, excess, guess, tally,
-                                     can_defer ? &deferred : nullptr, !first_pass)) {
-      V fd, td, nd;
-      pair_contact<double, PHYS, HIST>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4),
-                                       xyz(wi4), xyz(wj4), hk, plane, fd, td, nd, excess, guess, nullptr, nullptr,
-                                       !first_pass);
-      fc = cvt<R>(fd);
-      tc = cvt<R>(td);
-      nrm = cvt<R>(nd);
+    if constexpr (PHYS && sizeof(R) == sizeof(double)) {
+      pair_contact_fused<HIST>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4), xyz(wi4), xyz(wj4),
+                               hk, plane, fc, nrm, excess, guess, tally, can_defer ? &deferred : nullptr,
+                               !first_pass);
+      tc = (-xi4.w) * nrm;
+      tc2 = (-xj4.w) * nrm;
+    } else {
+      bool done = pair_contact<R, PHYS, HIST>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4),
+                                              xyz(wi4), xyz(wj4), hk, plane, fc, tc, nrm, excess, guess, tally,
+                                              can_defer ? &deferred : nullptr, !first_pass);
+      if (!done) {  // FP32 cannot decide the pair
+        V fd, td, nd;
+        if constexpr (PHYS) {
+          pair_contact_fused<HIST>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4), xyz(wi4),
+                                   xyz(wj4), hk, plane, fd, nd, excess, guess, nullptr, nullptr, !first_pass);
+          fc = cvt<R>(fd);
+          tc = cvt<R>((-xi4.w) * nd);
+          tc2 = cvt<R>((-xj4.w) * nd);
+        } else {
+          pair_contact<double, PHYS, HIST>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4),
+                                           xyz(wi4), xyz(wj4), hk, plane, fd, td, nd, excess, guess, nullptr,
+                                           nullptr, !first_pass);
+          fc = cvt<R>(fd);
+          tc = cvt<R>(td);
+          nrm = cvt<R>(nd);
+        }
+      }
+      if (done || !PHYS) tc2 = cross(nrm * (R)xj4.w, -fc);
     }
     if (deferred) return true;
     if (HIST && m < 64) atomicOr(B.hmask + k, 1ull << m);
@@ -1363,9 +1627,7 @@ __device__ __forceinline__ bool contact_eval(const StepParams& P, const Bank& B,
     const CRec* rj = P.crec + (size_t)j * P.cap;
     for (uint32_t c2 = 0; c2 < nj; ++c2) {
       if (rj[c2].j != k) continue;
-      const T3<R> f2 = -fc;
-      const T3<R> t2 = cross(nrm * (R)xj4.w, f2);
-      put_result(P, P.coff[j] + c2, f2, t2, vji);
+      put_result(P, P.coff[j] + c2, -fc, tc2, vji);
       const size_t h2 = (size_t)j * P.cap + (rj[c2].mv & 0xFFFFu);
       if (HIST) {
         B.hist[h2] = -hk[0];
