@@ -126,7 +126,7 @@ void Engine::free_device() {
   dfree(warena_); dfree(wres_); dfree(wok_); dfree(woff_); dfree(wcnt_);
   dfree(ctot_);
   dfree(tri_d_); dfree(tstart_d_); dfree(titems_d_); dfree(glaw_d_); dfree(motions_d_);
-  dfree(mlp_d_); dfree(jq_); dfree(jguess_); dfree(jfb_);
+  dfree(mlp_d_); dfree(jq_); dfree(jguess_); dfree(jfb_); dfree(jhard_);
   dfree(io_buf_); dfree(slot_of_); dfree(io_flag_); dfree(id_live_); dfree(id_pos_); dfree(slot_of_id_);
   dfree(id_part_);
   io_n_ = 0;
@@ -139,6 +139,10 @@ void Engine::free_device() {
   if (ev1_) cudaEventDestroy(ev1_);
   for (cudaEvent_t e : fev_) cudaEventDestroy(e);
   fev_.clear();
+  if (side_.fork) cudaEventDestroy(side_.fork);
+  if (side_.join) cudaEventDestroy(side_.join);
+  if (side_.stream) cudaStreamDestroy(side_.stream);
+  side_ = SideStream{};
   if (stream_) cudaStreamDestroy(stream_);
   stream_ = nullptr;
   ev0_ = ev1_ = nullptr;
@@ -174,6 +178,9 @@ int Engine::ensure_gpu() {
   CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
   CK(cudaEventCreate(&ev0_));
   CK(cudaEventCreate(&ev1_));
+  CK(cudaStreamCreateWithFlags(&side_.stream, cudaStreamNonBlocking));
+  CK(cudaEventCreateWithFlags(&side_.fork, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&side_.join, cudaEventDisableTiming));
   TRY(dalloc(&ctrl_, 1));
   CK(cudaMallocHost((void**)&ctrl_h_, sizeof(Ctrl)));
   TRY(dalloc(&ke_, 1));
@@ -408,10 +415,12 @@ int Engine::ensure_jkr_buffers() {
     const size_t need = std::max<size_t>(n_alloc_ * (size_t)std::max(cap_, 1), 1);
     if (jfb_alloc_ < need) {
       TRY(dalloc(&jfb_, need));
+      TRY(dalloc(&jhard_, need));
       jfb_alloc_ = need;
       graph_dirty_ = true;
     }
     P_.jfb = jfb_;
+    P_.jhard = jhard_;
   } else {
     P_.jfb = nullptr;
   }
@@ -500,12 +509,13 @@ int Engine::build_params() {
   P.pm = pm;
   P.wm = wm;
   // per-group law constants (group 0: the particle material)
+  std::vector<Law> laws;
   {
     uint32_t ng = 1;
     for (const HostParticle& p : hp_) ng = std::max(ng, p.group + 1);
     for (uint32_t g : tri_group_)
       if (g != GROUP_ALL) ng = std::max(ng, g + 1);
-    std::vector<Law> laws(ng);
+    laws.resize(ng);
     for (uint32_t g = 0; g < ng; ++g) {
       const Material& m = (g > 0 && g < gmat_.size() && gmat_set_[g]) ? gmat_[g] : pm;
       laws[g] = make_law(m);
@@ -554,6 +564,28 @@ int Engine::build_params() {
       }
     P.pretest = ok ? 1 : 0;
     P.lmax = (float)lm;
+    // The adhesive laws' cutoff is 1.5 r_sum (src/simulation.rs:343-357), but
+    // their force ends much sooner: JKR's at a gap of kappa C^(2/3) R*^(1/3) +
+    // 1e-3 R* (the ZERO certificate of rp_mlp.cuh) and sJKR's at |delta_c|, both
+    // largest for two of the largest spheres (R* = r_max / 2). Where such pairs
+    // are left out, the lists end there too: rows of 27 entries become 9 on
+    // spheres of 5-20 um at solid fraction 0.35. The relative 1e-3 covers the
+    // rounding of the laws next to the bound.
+    P.drop_zero = adh > 1.0 && P.pretest && !debug && (tmodel == RP_TANGENTIAL_COULOMB || mode == RP_MODE_PHYSICAL);
+    P.cut_a = (float)adh;
+    P.cut_b = INFINITY;
+    if (P.drop_zero) {
+      const double rs = 0.5 * rmax, kappa = std::pow(16.0, -1.0 / 6.0) - std::pow(16.0, -2.0 / 3.0);
+      double zone = 0.0;
+      for (const Law& L : laws) {
+        if (!(L.gamma_pp > 0.0)) continue;  // the elastic law: no force across a gap
+        const double z = nmodel == RP_NORMAL_JKR
+                             ? kappa * std::cbrt(L.jkr_C * L.jkr_C * rs) + 1e-3 * rs
+                             : std::sqrt(3.0 * (kPiH * kPiH) * (L.gamma_pp * L.gamma_pp) * rs / (L.es_pp * L.es_pp));
+        zone = std::max(zone, std::isfinite(z) ? z : INFINITY);
+      }
+      P.cut_b = (float)(zone * 1.001);
+    }
   }
   // fine cells at least the largest list radius, with a relative 1e-7 to
   // spare for the rounding of the cell lookup (fine_cell)
@@ -586,6 +618,14 @@ int Engine::build_params() {
     xb = std::max(xb, std::max(std::fabs(bmin[k]), std::fabs(bmax[k])) + 1.0);
   }
   P.rmaxf = (float)rmax;
+  P.cutmaxf = (float)(2.0 * rmax * adh);
+  {
+    // PF_NOIMAGE, PF_ONECELL: the pretest's own margin at the box's coordinates
+    // and the rounding of an FP32 cell coordinate, several times over
+    double lm = 0.0;
+    for (int k = 0; k < 3; ++k) lm = std::max(lm, P.bsize[k]);
+    P.home_margin = (float)(2e-6 * (xb + lm + 4.0 * rmax * adh + href));
+  }
   P.xbound = (float)xb;
   P.fncells = (uint32_t)((uint64_t)P.fdims[0] * P.fdims[1] * P.fdims[2]);
   rb_.key_bits = bits_for(P.fncells);
@@ -979,7 +1019,7 @@ int Engine::finish_step_accounting() {
 int Engine::recover_halt() {
   while (ctrl_h_->halt) {
     if (ctrl_h_->halt & HALT_LISTS) {
-      int newcap = std::max<int>(cap_ + 8, (int)(ctrl_h_->max_count * 5 / 4 + 8));
+      int newcap = grown_capacity(ctrl_h_->max_count);
       TRY(alloc_lists(newcap, true));
       tot_.status |= ST_NLIST_GROW;
     }
@@ -995,7 +1035,7 @@ int Engine::recover_halt() {
     CK(cudaMemcpyAsync(&ctrl_->wall_need, &zu, sizeof(unsigned), cudaMemcpyHostToDevice, stream_));
     CK(cudaStreamSynchronize(stream_));
     launches_ += launch_rebuild(P_, rb_, stream_);
-    launches_ += launch_force(P_, stream_);
+    launches_ += launch_force(P_, stream_, side_);
     launches_ += launch_end_step(P_, stream_);
     CK(cudaGetLastError());
     TRY(sync_ctrl());
@@ -1057,7 +1097,7 @@ int Engine::build_graph() {
   chain_kernels_ = launch_rebuild(P_, rb_, cap_stream2_);
   cudaGraph_t t2 = nullptr;
   CK(cudaStreamEndCapture(cap_stream2_, &t2));
-  sk += launch_force(P_, cap_stream_);
+  sk += launch_force(P_, cap_stream_, side_);
   sk += launch_end_step_loop(P_, hloop, cap_stream_);
   step_kernels_ = sk;
   cudaGraph_t t1 = nullptr;
@@ -1128,7 +1168,7 @@ int Engine::launch_steps(uint64_t n) {
       launches_ += launch_first_half(P_, stream_);
       launches_ += launch_rebuild(P_, rb_, stream_);
       if (profiling) CK(cudaEventRecord(fev_[2 * s], stream_));
-      launches_ += launch_force(P_, stream_);
+      launches_ += launch_force(P_, stream_, side_);
       if (profiling) CK(cudaEventRecord(fev_[2 * s + 1], stream_));
       launches_ += launch_end_step(P_, stream_);
     }
@@ -1205,7 +1245,7 @@ int Engine::compact_removed() {
     }
     // a list outgrew its capacity in that rebuild (the bank did not flip):
     // grow the lists and run the rebuild again from the same bank
-    const int newcap = std::max<int>(cap_ + 8, (int)(ctrl_h_->max_count * 5 / 4 + 8));
+    const int newcap = grown_capacity(ctrl_h_->max_count);
     TRY(alloc_lists(newcap, true));
     tot_.status |= ST_NLIST_GROW;
     const int zero = 0;
@@ -1744,11 +1784,11 @@ int Engine::autotune(rp_tune_report* rep) {
   std::memcpy(&saved, ctrl_h_, sizeof(Ctrl));
   int tried = 0;
   auto time_pass = [&](float* out) -> int {
-    for (int w = 0; w < 2; ++w) launch_force(P_, stream_);
+    for (int w = 0; w < 2; ++w) launch_force(P_, stream_, side_);
     float t[5];
     for (int r = 0; r < 5; ++r) {
       CK(cudaEventRecord(ev0_, stream_));
-      launch_force(P_, stream_);
+      launch_force(P_, stream_, side_);
       CK(cudaEventRecord(ev1_, stream_));
       CK(cudaEventSynchronize(ev1_));
       CK(cudaEventElapsedTime(&t[r], ev0_, ev1_));

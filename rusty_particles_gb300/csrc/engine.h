@@ -3,6 +3,7 @@
 // (src/simulation.rs:16-51) with GPU-resident state.
 #pragma once
 #include <cstdint>
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -84,6 +85,10 @@ class Engine {
   int jkr_get_network(float* params, float* norm, float* domain);
   bool jkr_has_network() const { return jkr_have_net_; }
   int jkr_counters(uint64_t out[6]);
+  // row capacity for lists of up to max_count entries (rows on 16 bytes)
+  int grown_capacity(unsigned max_count) const {
+    return (std::max(cap_ + 8, (int)(max_count * 5 / 4 + 8)) + 3) & ~3;
+  }
   void config_changed() { dev_valid_ = false; }  // forces a fresh upload before the next step
   void set_capacity(int c) {
     if (!host_valid_) download();
@@ -163,7 +168,9 @@ class Engine {
   uint2* jq_ = nullptr;
   float* jguess_ = nullptr;
   size_t jq_alloc_ = 0;
-  uint32_t* jfb_ = nullptr;  // pairs deferred to the reference-Newton pass
+  uint32_t* jfb_ = nullptr;    // pairs deferred to the reference-Newton pass
+  uint32_t* jhard_ = nullptr;  // pairs that the filter sends to it at once
+  SideStream side_;
   size_t jfb_alloc_ = 0;
   int ensure_jkr_buffers();
   int step_kernels_ = 4;  // kernels of one device-loop step outside the rebuild chain

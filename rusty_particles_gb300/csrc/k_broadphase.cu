@@ -55,6 +55,14 @@ __global__ void k_hash_fine(StepParams P, uint32_t* keys, uint32_t* vals) {
     else {
       D4 x = B.xr[k];
       key = fine_cell(P, x.x, x.y, x.z);
+      // a step's drift leaves particles beyond a periodic face until the next step wraps them
+      const float4 xf = B.xf[k];
+      const float p[3] = {xf.x, xf.y, xf.z};
+      float out = 0.0f;
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+        if (P.periodic[a]) out = fmaxf(out, fmaxf((float)P.bmin[a] - p[a], p[a] - (float)P.bmax[a]));
+      if (out > 0.0f) atomicMax(&P.ctrl->xout, __float_as_uint(out));
     }
     keys[k] = key;
     vals[k] = (uint32_t)k;
@@ -314,7 +322,7 @@ __global__ void k_reorder(StepParams P, const uint32_t* perm) {
 
 // --------------------------------------------------------- neighbour lists
 // One thread per slot scans the 27 (deduplicated) fine cells around it and
-// keeps every other particle within (cutoff + skin), tested in FP32 on the
+// keeps every other particle within reach (cut_a, cut_b) + skin, tested in FP32 on the
 // FP64 difference with a small relative margin, so the list is a superset of
 // every pair the exact FP64 cutoff test can accept before the next rebuild.
 // A neighbouring cell farther from the particle than its largest list radius
@@ -325,7 +333,6 @@ __global__ void k_build_nlist(StepParams P, const uint32_t* cstart, const uint32
   if (gate_closed(P.ctrl)) return;
   const int b = P.ctrl->bank;
   const Bank O = P.bank[b], B = P.bank[b ^ 1];
-  const float adh = (P.nmodel == 3 || P.nmodel == 4) ? 1.5f : 1.0f;
   const float skin = (float)P.skin;
   const size_t plane_new = (size_t)P.n * P.cap;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < P.n; k += gridDim.x * blockDim.x) {
@@ -349,7 +356,7 @@ __global__ void k_build_nlist(StepParams P, const uint32_t* cstart, const uint32
     // is a periodic image) plus the rounding of an FP32 distance again,
     // grown by 1e-4; the cell gaps keep a thousandth of a cell for the
     // rounding of the lookup
-    const float rb = (ri + P.rmaxf) * adh + skin;
+    const float rb = fminf((ri + P.rmaxf) * P.cut_a, (ri + P.rmaxf) + P.cut_b) + skin;
     const float Xe = fmaxf(Xi + 2.0f * rb, P.xbound);
     const float rlm = (rb * P.list_scale + 5e-7f * (2.0f * Xe + P.lmax + rb)) * 1.0001f;
     const double pq[3] = {xi.x, xi.y, xi.z};
@@ -411,7 +418,8 @@ __global__ void k_build_nlist(StepParams P, const uint32_t* cstart, const uint32
             if (P.periodic[2] && fabsf(fz * P.binvf[2]) > 0.49f) fz -= P.bsizef[2] * rintf(fz / P.bsizef[2]);
             float d2 = fx * fx + fy * fy + fz * fz;
             const float X = fmaxf(Xi, fmaxf(fmaxf(fabsf(xj.x), fabsf(xj.y)), fabsf(xj.z)));
-            float rl = (ri + xj.w) * adh + skin;
+            const float rsum = ri + xj.w;
+            float rl = fminf(rsum * P.cut_a, rsum + P.cut_b) + skin;
             rl = rl * P.list_scale + 2.5e-7f * (2.0f * X + P.lmax);
             if (d2 < rl * rl) {
               if (cnt < (uint32_t)P.cap) {
@@ -451,6 +459,7 @@ __global__ void k_rebuild_finish(StepParams P) {
   if (c->rebuild == 0 || c->halt != 0) return;
   c->bank ^= 1;
   c->rebuild = 0;
+  c->xout = 0;
   c->rebuilds += 1;
 }
 

@@ -303,12 +303,8 @@ __global__ void k_mlp_reduce_adam(const float* __restrict__ partial, int ntiles,
 // Tensor-core inference over rows of normalised features (one row per lane).
 __global__ void __launch_bounds__(128) k_mlp_infer_rows(const MlpInfer* __restrict__ Mg, const float* __restrict__ featn,
                                                         size_t n, float* __restrict__ out) {
-  __shared__ MlpInfer M;
-  {
-    const uint4* src = reinterpret_cast<const uint4*>(Mg);
-    uint4* dst = reinterpret_cast<uint4*>(&M);
-    for (int i = threadIdx.x; i < (int)(sizeof(MlpInfer) / 16); i += blockDim.x) dst[i] = src[i];
-  }
+  __shared__ MlpShared M;
+  mlp_stage(M, Mg);
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const size_t warps = (size_t)gridDim.x * (blockDim.x >> 5);

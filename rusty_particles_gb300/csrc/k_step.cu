@@ -224,8 +224,8 @@ __device__ __forceinline__ R jkr_mag(R overlap, R es, R rs, R gamma, bool* near 
   if (fabs(f_val) > R(1e-3) * rs) return R(0);
   if (a <= R(0)) return R(0);
   R a3 = a * a * a;
-  R term1 = R(4) * es * a3 / (R(3) * rs);
-  R term2 = sqrt(eight_pi * gamma * es * a3);
+  R term1 = div_rn(R(4) * es * a3, R(3) * rs);
+  R term2 = sqrt_rn(eight_pi * gamma * es * a3);
   R fm = term1 - term2;
   R f_pull = R(-2.0 / 3.0) * R(kPi) * gamma * rs;
   if (near && fabs(fm - f_pull) <= R(1e-5) * (term1 + term2)) *near = true;
@@ -237,13 +237,16 @@ __device__ __forceinline__ R jkr_mag(R overlap, R es, R rs, R gamma, bool* near 
 // certificates (rp_mlp.cuh) either prove the reference returns zero or that
 // its iteration converges to the root on the increasing branch; the root is
 // then found in FP32 (solver 1: two Newton steps from the network's `guess`;
-// solver 2: Newton from the reference's own start), accepted only when its
+// solver 2, and pairs without a good guess: Newton from the reference's own
+// start; `missed` marks the latter with solver 1, their steps not counted as
+// the network's), accepted only when its
 // FP64 residual is <= 1e-6 of the terms, corrected by one FP64-accurate Newton
 // step, and turned into the reference's force 4 E* a^3/(3 R*) - sqrt(8 pi
 // gamma E* a^3) = E* a (4 a^2/(3 R*) - sqrt(C a)). The pull-off cut is decided
 // in FP64 and left to the reference's loop when within 1e-7 of the terms.
 __device__ __forceinline__ int jkr_learned(const StepParams& P, const Law& L, double overlap, double rs, float guess,
-                                           double& fm, uint32_t& iters) {
+                                           double& fm, uint32_t& iters, bool& missed) {
+  missed = false;
   const float rsf = (float)rs;
   const float x = (float)overlap / rsf;
   const float c = L.jkr_Cf / rsf;
@@ -258,21 +261,22 @@ __device__ __forceinline__ int jkr_learned(const StepParams& P, const Law& L, do
     // operation for operation in FP64
     const double es = L.es_pp, gamma = L.gamma_pp;
     const double eight_pi = 8.0 * kPi;
-    const double c_val = eight_pi * gamma / es;
-    double a = sqrt(rs * overlap);
+    const double c_val = L.jkr_C;  // 8 pi gamma / E*
+    double a = sqrt_rn(rs * overlap);
     const double lim = 1e-6 * rs;
-    for (int it = 0; it < 20; ++it) {
-      const double st = a * 0.5;
-      a = a - st;
-      if (st < lim) break;
-    }
-    const double ts = sqrt(c_val * a);
-    const double f_val = a * a / rs - ts - overlap;
+    // a / 2^k with the first k in 1..20 that takes it below lim, from the
+    // exponents and mantissas (both are positive and normal here); the loop
+    // itself took up to 60 of the pass's FP64 instructions
+    const long long ab = __double_as_longlong(a), lb = __double_as_longlong(lim), M = 0x000FFFFFFFFFFFFFll;
+    const int k = (int)(ab >> 52) - (int)(lb >> 52) + ((ab & M) < (lb & M) ? 0 : 1);
+    a = __longlong_as_double(ab - ((long long)min(max(k, 1), 20) << 52));
+    const double ts = sqrt_rn(c_val * a);
+    const double f_val = div_rn(a * a, rs) - ts - overlap;
     fm = 0.0;
     if (fabs(f_val) > 1e-3 * rs || a <= 0.0) return JKR_WALK;
     const double a3 = a * a * a;
-    const double term1 = 4.0 * es * a3 / (3.0 * rs);
-    const double term2 = sqrt(eight_pi * gamma * es * a3);
+    const double term1 = div_rn(4.0 * es * a3, 3.0 * rs);
+    const double term2 = sqrt_rn(eight_pi * gamma * es * a3);
     const double fmv = term1 - term2;
     const double f_pull = (-2.0 / 3.0) * kPi * gamma * rs;
     fm = fmv < f_pull ? 0.0 : fmv;
@@ -280,15 +284,18 @@ __device__ __forceinline__ int jkr_learned(const StepParams& P, const Law& L, do
   }
   if (cls != JKR_CONVERGES) return JKR_FALLBACK;
   float u;
-  if (P.jkr_solver == 1) {
-    if (!(guess > 0.0f && guess < 1e30f)) return JKR_FALLBACK;
-    u = jkr_newton_f32(jkr_newton_f32(guess, x, c), x, c);
-    iters += 2;
-  } else {
+  missed = P.jkr_solver == 1 && !(guess > 0.0f && guess < 1e30f);
+  if (P.jkr_solver == 1 && !missed) {
+    const float u1 = jkr_newton_f32(guess, x, c);
+    u = jkr_newton_f32(u1, x, c);
+    missed = !(fabsf(u - u1) <= 1e-3f * u);  // a prediction two quadratic steps do not make good
+    if (!missed) iters += 2;
+  }
+  if (P.jkr_solver != 1 || missed) {
     u = overlap > 0.0 ? sqrtf(x) : 0.5f;
     for (int k = 0; k < 40; ++k) {
       const float un = jkr_newton_f32(u, x, c);
-      ++iters;
+      if (!missed) ++iters;
       const bool done = fabsf(un - u) <= 1e-6f * un;
       u = un;
       if (done) break;
@@ -339,9 +346,10 @@ __device__ __forceinline__ R sjkr_mag(R overlap, R vn, R es, R rs, R gamma) {
 // Normal force vector for the configured model. The reference passes
 // Vec3::ZERO as the relative velocity to the hysteretic particle-particle law
 // (src/simulation.rs:409-411) and the real one for walls (:495-501).
-template <typename R>
+template <typename R, bool JKR>
 __device__ __forceinline__ R normal_mag(int model, R overlap, T3<R> n, T3<R> rv, R es, R rs, R ms, R beta_abs,
                                        R gamma, bool wall) {
+  if (JKR) return jkr_mag(overlap, es, rs, gamma);
   R m;
   switch (model) {
     case 1: m = hertz_mag(overlap, dot(rv, n), es, rs, ms, beta_abs); break;
@@ -355,14 +363,13 @@ __device__ __forceinline__ R normal_mag(int model, R overlap, T3<R> n, T3<R> rv,
       R vn = wall ? dot(rv, n) : dot(t3(R(0), R(0), R(0)), n);
       m = lsd_mag(overlap, vn, kn, R(0));
     } break;
-    case 3: m = jkr_mag(overlap, es, rs, gamma); break;
     default: m = sjkr_mag(overlap, dot(rv, n), es, rs, gamma); break;
   }
   return m;
 }
 // The same with the normal relative speed given (vn = rv . n; the FP32 form
 // forms it in FP64). The hysteretic particle-particle law keeps the
-// reference's zero velocity.
+// reference's zero velocity. JKR has no damping and is the caller's.
 template <typename R>
 __device__ __forceinline__ R normal_mag_vn(int model, R overlap, T3<R> n, R vn, R es, R rs, R ms, R beta_abs,
                                           R gamma) {
@@ -374,15 +381,14 @@ __device__ __forceinline__ R normal_mag_vn(int model, R overlap, T3<R> n, R vn, 
       return lsd_mag(overlap, vn, kn, gn);
     }
     case 2: return lsd_mag(overlap, dot(t3(R(0), R(0), R(0)), n), es * rs, R(0));
-    case 3: return jkr_mag(overlap, es, rs, gamma);
     default: return sjkr_mag(overlap, vn, es, rs, gamma);
   }
 }
 // The vector form, f n, as the reference returns it.
-template <typename R>
+template <typename R, bool JKR>
 __device__ __forceinline__ T3<R> normal_force(int model, R overlap, T3<R> n, T3<R> rv, R es, R rs, R ms, R beta_abs,
                                               R gamma, bool wall) {
-  return normal_mag<R>(model, overlap, n, rv, es, rs, ms, beta_abs, gamma, wall) * n;
+  return normal_mag<R, JKR>(model, overlap, n, rv, es, rs, ms, beta_abs, gamma, wall) * n;
 }
 
 // src/physics.rs:385-397 (direction by one reciprocal square root)
@@ -436,7 +442,8 @@ __device__ __forceinline__ T3<R> spring_coulomb(R fn, T3<R> rv, T3<R> n, T3<R>& 
 // and FP32 Newton steps when not null). A pair that needs the reference's
 // Newton iteration sets *deferred and returns at once, touching nothing, when
 // `deferred` is given; `newton` forces the reference's iteration.
-template <typename R, bool PHYS, bool HIST>
+// JKR: the law is JKR's (a kernel of its own; the others hold fewer registers).
+template <typename R, bool PHYS, bool HIST, bool JKR>
 __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, V d, double d2, double rsum, double ri,
                                              double rj, double mi, double mj, V vi, V vj, V wi, V wj, double* hist,
                                              size_t plane, T3<R>& fc_out, T3<R>& tc_out, T3<R>& n_out,
@@ -512,13 +519,14 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
   const R ms = div_rn((R)mi * (R)mj, (R)mi + (R)mj);
   R fmag;
   int jkind = JKR_FALLBACK;
-  if (P.nmodel == 3 && P.jkr_solver != 0 && !newton && L.gamma_pp > 0.0) {
+  if (JKR && P.jkr_solver != 0 && !newton && L.gamma_pp > 0.0) {
     double fmd = 0.0;
     uint32_t it = 0;
-    jkind = jkr_learned(P, L, ovd, (double)rs, guess, fmd, it);
+    bool missed;
+    jkind = jkr_learned(P, L, ovd, (double)rs, guess, fmd, it, missed);
     if (jkind != JKR_FALLBACK) fmag = (R)fmd;
     if (tally) {
-      tally[jkind == JKR_CONVERGES ? 0 : (jkind == JKR_ZERO ? 1 : (jkind == JKR_WALK ? 5 : 2))] += 1;
+      tally[jkind == JKR_CONVERGES ? (missed ? 2 : 0) : (jkind == JKR_ZERO ? 1 : (jkind == JKR_WALK ? 5 : 2))] += 1;
       tally[4] += it;
     }
     if (jkind == JKR_FALLBACK && deferred) {
@@ -527,7 +535,9 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
     }
   }
   if (jkind != JKR_FALLBACK) {
-  } else if (F32 && P.nmodel == 3) {
+  } else if (JKR && !F32) {
+    fmag = jkr_mag<R>(overlap, (R)L.es_pp, rs, (R)L.gamma_pp);
+  } else if (JKR) {
     // The contact radius has a square-root fold next to the pull-off: there
     // the FP32 iteration cannot resolve the root (an FP32 residual moves it by
     // ~sqrt(1e-7) relative) and the pair is evaluated in FP64. Elsewhere the
@@ -542,7 +552,7 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
   } else {
     fmag = normal_mag_vn<R>(P.nmodel, overlap, n, vn, (R)L.es_pp, rs, ms, (R)L.beta_abs, (R)L.gamma_pp);
   }
-  if (F32 && P.nmodel == 4 && L.gamma_pp > 0.0) {
+  if (F32 && !JKR && P.nmodel == 4 && L.gamma_pp > 0.0) {
     const R gamma = (R)L.gamma_pp, es = (R)L.es_pp;
     const R f_pull = R(1.5) * R(kPi) * gamma * rs;
     const R delta_c = -sqrt(R(3) * (R(kPi) * R(kPi)) * (gamma * gamma) * rs / (es * es));
@@ -649,7 +659,7 @@ __device__ __forceinline__ double normal_mag_fused(int model, const Law& L, doub
 // and, the other end's force being -f, -r_j (n x f) on j; the normal force
 // adds nothing to it.
 // Springs, `deferred` and `newton` as in pair_contact.
-template <bool HIST>
+template <bool HIST, bool JKR>
 __device__ __forceinline__ void pair_contact_fused(const StepParams& P, const Law& L, V d, double d2, double rsum,
                                                    double ri, double rj, double mi, double mj, V vi, V vj, V wi, V wj,
                                                    double* hist, size_t plane, V& f_out, V& nf_out, bool& excess,
@@ -676,13 +686,14 @@ __device__ __forceinline__ void pair_contact_fused(const StepParams& P, const La
   const V vt = mad(-vn, n, rv);
   const double rs = div_rn(ri * rj, rsum);
   double fm = 0.0;
-  if (P.nmodel == 3) {
+  if (JKR) {
     int kind = JKR_FALLBACK;
     if (P.jkr_solver != 0 && !newton && L.gamma_pp > 0.0) {
       uint32_t it = 0;
-      kind = jkr_learned(P, L, overlap, rs, guess, fm, it);
+      bool missed;
+      kind = jkr_learned(P, L, overlap, rs, guess, fm, it, missed);
       if (tally) {
-        tally[kind == JKR_CONVERGES ? 0 : (kind == JKR_ZERO ? 1 : (kind == JKR_WALK ? 5 : 2))] += 1;
+        tally[kind == JKR_CONVERGES ? (missed ? 2 : 0) : (kind == JKR_ZERO ? 1 : (kind == JKR_WALK ? 5 : 2))] += 1;
         tally[4] += it;
       }
       if (kind == JKR_FALLBACK && deferred) {
@@ -790,6 +801,7 @@ __global__ void __launch_bounds__(256) k_first_half(StepParams P) {
   const double hdt = 0.5 * dt;
   const float bminf[3] = {(float)P.bmin[0], (float)P.bmin[1], (float)P.bmin[2]};
   const float inv_hf = (float)P.inv_href;
+  const unsigned xmax = C->xmax;
   bool want_rebuild = false;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < P.n; k += gridDim.x * blockDim.x) {
     uint32_t fl = B.flags[k];
@@ -882,6 +894,11 @@ __global__ void __launch_bounds__(256) k_first_half(StepParams P) {
     if (own_spin || __double_as_longlong(code) != __double_as_longlong(wc.w)) B.wc[k] = wc;
     B.xr[k] = D4{x.x, x.y, x.z, xr.w};
     B.xf[k] = xf;
+    // the largest |coordinate| sets the filter's rounding margin (the bits of
+    // non-negative floats order as the floats do; NaN stays out)
+    const float far = fmaxf(fmaxf(fabsf(xf.x), fabsf(xf.y)), fabsf(xf.z));
+    const unsigned lanes = __activemask(), top = __reduce_max_sync(lanes, far >= 0.0f ? __float_as_uint(far) : 0u);
+    if (top > xmax && (threadIdx.x & 31) == __ffs(lanes) - 1) atomicMax(&C->xmax, top);
     float4 r0 = B.xref[k];
     float ddx = xf.x - r0.x, ddy = xf.y - r0.y, ddz = xf.z - r0.z;
     if (P.periodic[0]) ddx -= P.bsizef[0] * rintf(ddx / P.bsizef[0]);
@@ -969,6 +986,7 @@ __device__ __forceinline__ bool wall_pretest(const TriRec& tr, uint32_t gi, floa
 // The FP64 contact of a sphere with a triangle that passed the pretest:
 // force fc and torque r_a x fc on the sphere, or false (outputs untouched)
 // when it does not touch the triangle.
+template <bool JKR>
 __device__ __forceinline__ bool wall_contact(const StepParams& P, const Law& L, const TriRec& tr, V xi, V vi, V wi,
                                              double ri, double mi, V& fc_out, V& tc_out, bool& excess) {
   // closest point, src/mesh.rs:45-117 (same regions and clamps)
@@ -1022,7 +1040,7 @@ __device__ __forceinline__ bool wall_contact(const StepParams& P, const Law& L, 
     const V vw = vmk(M.v[0], M.v[1], M.v[2]) + cross(vmk(M.w[0], M.w[1], M.w[2]), cp - vmk(M.c[0], M.c[1], M.c[2]));
     rv = rv - vw;
   }
-  const V fnv = normal_force<double>(P.nmodel, pen, n, rv, L.es_pw, ri, mi, L.beta_abs, L.gamma_pw, true);
+  const V fnv = normal_force<double, JKR>(P.nmodel, pen, n, rv, L.es_pw, ri, mi, L.beta_abs, L.gamma_pw, true);
   const V fc = fnv + coulomb_force<double>(len(fnv), rv, n, L.mu);
   fc_out = fc;
   tc_out = cross(ra, fc);
@@ -1030,6 +1048,7 @@ __device__ __forceinline__ bool wall_contact(const StepParams& P, const Law& L, 
 }
 
 // All wall contacts of one particle in mesh order.
+template <bool JKR>
 __device__ __forceinline__ void wall_forces(const StepParams& P, const Law& L, uint32_t gi, V xi, float4 xf, V vi,
                                             V wi, double ri, double mi, V& F, V& T, bool& excess) {
   uint32_t s, e;
@@ -1039,11 +1058,35 @@ __device__ __forceinline__ void wall_forces(const StepParams& P, const Law& L, u
     const TriRec& tr = P.tri[P.titems[t]];
     if (!wall_pretest(tr, gi, xf, xmag)) continue;
     V fc, tc;
-    if (wall_contact(P, L, tr, xi, vi, wi, ri, mi, fc, tc, excess)) {
+    if (wall_contact<JKR>(P, L, tr, xi, vi, wi, ri, mi, fc, tc, excess)) {
       F = F + fc;
       T = T + tc;
     }
   }
+}
+
+// FP32 pretest on the position mirror. With u = 2^-24 each FP32 difference of
+// a pair inside the cutoff is within e = u (2X + 2 cut + L) of the FP64 one (X
+// the largest coordinate, L the largest periodic length), so d2f <= cut^2 +
+// 3.47 e cut + 3 e^2 + 12 u cut^2 there; (cut + m)^2 with m = 2.1 e + 1e-6 cut
+// lies above that, and a pair beyond it is certainly outside the exact FP64
+// test. One margin for all pairs (the largest X and cut) keeps the test short
+// and symmetric bit for bit, so both ends keep a pair or drop it together.
+__device__ __forceinline__ float pretest_margin(const StepParams& P, const Ctrl* C) {
+  const float X = __uint_as_float(C->xmax);
+  return 2.1f * (6.0e-8f * (2.0f * X + 2.0f * P.cutmaxf + P.lmax)) + 1.0e-6f * P.cutmaxf;
+}
+__device__ __forceinline__ bool pretest_near(const StepParams& P, float4 xi, float4 xj, bool image, float margin) {
+  float fx = xi.x - xj.x, fy = xi.y - xj.y, fz = xi.z - xj.z;
+  if (image) {
+    if (P.periodic[0]) { const float L = P.bsizef[0]; if (fx > 0.5f * L) fx -= L; else if (fx < -0.5f * L) fx += L; }
+    if (P.periodic[1]) { const float L = P.bsizef[1]; if (fy > 0.5f * L) fy -= L; else if (fy < -0.5f * L) fy += L; }
+    if (P.periodic[2]) { const float L = P.bsizef[2]; if (fz > 0.5f * L) fz -= L; else if (fz < -0.5f * L) fz += L; }
+  }
+  const float d2 = fx * fx + fy * fy + fz * fz;
+  const float rsum = xi.w + xj.w;
+  const float t = fminf(rsum * P.cut_a, rsum + P.cut_b) + margin;
+  return !(d2 > t * t);  // NaN (a removed partner) stays: the exact test drops it
 }
 
 // ---------------------------------------------------------------- forces
@@ -1052,13 +1095,14 @@ __device__ __forceinline__ void wall_forces(const StepParams& P, const Law& L, u
 // pair laws of src/simulation.rs:358-460 (in R), the wall triangles of
 // src/simulation.rs:464-523 from the triangle grid, then a = g + F/m and
 // tau = T (src/simulation.rs:265-271, 532-536). v and omega are only read.
-template <bool PHYS, bool HIST, typename R>
+template <bool PHYS, bool HIST, typename R, bool JKR>
 __global__ void __launch_bounds__(128) k_force(StepParams P) {
   Ctrl* C = P.ctrl;
   if (C->halt) return;
   const Bank B = P.bank[C->bank];
   const bool adh = (P.nmodel == 3 || P.nmodel == 4);
   const size_t plane = (size_t)P.n * P.cap;
+  const float margin = pretest_margin(P, C);
   bool excess = false;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < P.n; k += gridDim.x * blockDim.x) {
     const uint32_t fl = B.flags[k];
@@ -1074,27 +1118,10 @@ __global__ void __launch_bounds__(128) k_force(StepParams P) {
     const uint32_t* row = B.nbr + (size_t)k * P.cap;
     unsigned long long hm = 0ull;  // springs this row writes (the live-spring mask)
     const float4 xif = B.xf[k];
-    const float Xi = fmaxf(fmaxf(fabsf(xif.x), fabsf(xif.y)), fabsf(xif.z));
     for (uint32_t m = 0; m < cnt; ++m) {
       const uint32_t j = row[m];
       if (P.pretest) {
-        // FP32 pretest on the position mirror: with u = 2^-24, each FP32
-        // difference is within e = u (2X + 2 cut + L) of the FP64 one when the
-        // pair is inside the cutoff, so d2f <= cut^2 + 3.47 e cut + 3 e^2 +
-        // 12 u cut^2 there. Beyond the (larger) band below the pair is
-        // certainly outside and the exact FP64 test is skipped.
-        const float4 xjf = B.xf[j];
-        float fx = xif.x - xjf.x, fy = xif.y - xjf.y, fz = xif.z - xjf.z;
-        if (P.periodic[0]) { const float L = P.bsizef[0]; if (fx > 0.5f * L) fx -= L; else if (fx < -0.5f * L) fx += L; }
-        if (P.periodic[1]) { const float L = P.bsizef[1]; if (fy > 0.5f * L) fy -= L; else if (fy < -0.5f * L) fy += L; }
-        if (P.periodic[2]) { const float L = P.bsizef[2]; if (fz > 0.5f * L) fz -= L; else if (fz < -0.5f * L) fz += L; }
-        const float d2f = fx * fx + fy * fy + fz * fz;
-        const float rsf = xif.w + xjf.w;
-        const float cutf = adh ? rsf * 1.5f : rsf;
-        const float X = fmaxf(Xi, fmaxf(fmaxf(fabsf(xjf.x), fabsf(xjf.y)), fabsf(xjf.z)));
-        const float e = 6.0e-8f * (2.0f * X + 2.0f * cutf + P.lmax);
-        const float band = 4.1f * cutf * e + 3.0f * e * e + 1.0e-6f * cutf * cutf;
-        if (d2f > cutf * cutf + band) {
+        if (!pretest_near(P, xif, B.xf[j], true, margin)) {
           const size_t hi = (size_t)k * P.cap + m;
           if (HIST) {
             B.hist[hi] = 0.0;
@@ -1125,19 +1152,19 @@ __global__ void __launch_bounds__(128) k_force(StepParams P) {
           V fc, tc, nrm;
           T3<R> fr, tr, nr;
           if constexpr (PHYS && sizeof(R) == sizeof(double)) {
-            pair_contact_fused<HIST>(P, lw, d, d2, rsum, ri, rj, mi, vj4.w, vi, xyz(vj4), wi, xyz(wj4),
+            pair_contact_fused<HIST, JKR>(P, lw, d, d2, rsum, ri, rj, mi, vj4.w, vi, xyz(vj4), wi, xyz(wj4),
                                      HIST ? B.hist + hi : nullptr, plane, fc, nrm, excess);
             tc = (-ri) * nrm;
-          } else if (pair_contact<R, PHYS, HIST>(P, lw, d, d2, rsum, ri, rj, mi, vj4.w, vi, xyz(vj4), wi, xyz(wj4),
+          } else if (pair_contact<R, PHYS, HIST, JKR>(P, lw, d, d2, rsum, ri, rj, mi, vj4.w, vi, xyz(vj4), wi, xyz(wj4),
                                           HIST ? B.hist + hi : nullptr, plane, fr, tr, nr, excess)) {
             fc = cvt<double>(fr);
             tc = cvt<double>(tr);
           } else if constexpr (PHYS) {
-            pair_contact_fused<HIST>(P, lw, d, d2, rsum, ri, rj, mi, vj4.w, vi, xyz(vj4), wi, xyz(wj4),
+            pair_contact_fused<HIST, JKR>(P, lw, d, d2, rsum, ri, rj, mi, vj4.w, vi, xyz(vj4), wi, xyz(wj4),
                                      HIST ? B.hist + hi : nullptr, plane, fc, nrm, excess);
             tc = (-ri) * nrm;
           } else {
-            pair_contact<double, PHYS, HIST>(P, lw, d, d2, rsum, ri, rj, mi, vj4.w, vi, xyz(vj4), wi, xyz(wj4),
+            pair_contact<double, PHYS, HIST, JKR>(P, lw, d, d2, rsum, ri, rj, mi, vj4.w, vi, xyz(vj4), wi, xyz(wj4),
                                              HIST ? B.hist + hi : nullptr, plane, fc, tc, nrm, excess);
           }
           if (HIST && m < 64) hm |= 1ull << m;
@@ -1155,7 +1182,7 @@ __global__ void __launch_bounds__(128) k_force(StepParams P) {
       if (P.debug) P.dbgMult[hi] = (uint8_t)visits;
     }
     if (HIST && hm) B.hmask[k] |= hm;
-    wall_forces(P, lw, gi, xi, xif, vi, wi, ri, mi, F, T, excess);
+    wall_forces<JKR>(P, lw, gi, xi, xif, vi, wi, ri, mi, F, T, excess);
     if (P.debug) {
       P.dbgF[3 * (size_t)k] = F.x; P.dbgF[3 * (size_t)k + 1] = F.y; P.dbgF[3 * (size_t)k + 2] = F.z;
       P.dbgT[3 * (size_t)k] = T.x; P.dbgT[3 * (size_t)k + 1] = T.y; P.dbgT[3 * (size_t)k + 2] = T.z;
@@ -1179,24 +1206,6 @@ __global__ void __launch_bounds__(128) k_force(StepParams P) {
 // visit counts); the pair laws run one thread per pair, each pair once, and a
 // last pass sums every particle's contact results in list order.
 
-// FP32 pretest on the position mirror: with u = 2^-24, each FP32 difference
-// is within e = u (2X + 2 cut + L) of the FP64 one when the pair is inside the
-// cutoff, so d2f <= cut^2 + 3.47 e cut + 3 e^2 + 12 u cut^2 there; beyond the
-// larger band below the pair is certainly outside the exact FP64 test.
-__device__ __forceinline__ bool pretest_far(const StepParams& P, float4 xif, float Xi, float4 xjf, bool adh) {
-  float fx = xif.x - xjf.x, fy = xif.y - xjf.y, fz = xif.z - xjf.z;
-  if (P.periodic[0]) { const float L = P.bsizef[0]; if (fx > 0.5f * L) fx -= L; else if (fx < -0.5f * L) fx += L; }
-  if (P.periodic[1]) { const float L = P.bsizef[1]; if (fy > 0.5f * L) fy -= L; else if (fy < -0.5f * L) fy += L; }
-  if (P.periodic[2]) { const float L = P.bsizef[2]; if (fz > 0.5f * L) fz -= L; else if (fz < -0.5f * L) fz += L; }
-  const float d2f = fx * fx + fy * fy + fz * fz;
-  const float rsf = xif.w + xjf.w;
-  const float cutf = adh ? rsf * 1.5f : rsf;
-  const float X = fmaxf(Xi, fmaxf(fmaxf(fabsf(xjf.x), fabsf(xjf.y)), fabsf(xjf.z)));
-  const float e = 6.0e-8f * (2.0f * X + 2.0f * cutf + P.lmax);
-  const float band = 4.1f * cutf * e + 3.0f * e * e + 1.0e-6f * cutf * cutf;
-  return d2f > cutf * cutf + band;
-}
-
 // Minimum image on the periodic axes. A difference whose magnitude has a
 // smaller high word than bsize/4 is below bsize/4 (and NaN is not), so it
 // needs no FP64 comparison.
@@ -1210,12 +1219,14 @@ __device__ __forceinline__ V mic(const StepParams& P, V d) {
   return d;
 }
 
-// Whether a JKR pair goes to the network queue: jkr_learned's certificate on
-// the FP32 position mirror, its xi thresholds widened by the mirror's
-// rounding (~2.4e-7 of the coordinates). A queued pair the exact test rejects
-// only wastes a network row; a converging pair without a row falls back to the
-// reference's Newton.
-__device__ __forceinline__ bool jkr_net_hint(const StepParams& P, float Cf, float4 xif, float4 xjf) {
+// Where a JKR pair of the certified solvers goes, from jkr_certify on the FP32
+// position mirror: CREC_HARD to the list of pairs next to the fold, whose force
+// needs the reference's Newton, CREC_NET to the network queue (both with a
+// margin for the mirror's rounding, ~2.4e-7 of the coordinates). Both are hints,
+// the exact certificates decide: a queued pair they reject only wastes a
+// network row, a converging pair without a row falls back to the reference's
+// Newton, and one that needs it outside the list is deferred.
+__device__ __forceinline__ uint32_t jkr_hint(const StepParams& P, float Cf, float4 xif, float4 xjf, bool learn) {
   float fx = xif.x - xjf.x, fy = xif.y - xjf.y, fz = xif.z - xjf.z;
   if (P.periodic[0]) { const float L = P.bsizef[0]; if (fx > 0.5f * L) fx -= L; else if (fx < -0.5f * L) fx += L; }
   if (P.periodic[1]) { const float L = P.bsizef[1]; if (fy > 0.5f * L) fy -= L; else if (fy < -0.5f * L) fy += L; }
@@ -1223,19 +1234,23 @@ __device__ __forceinline__ bool jkr_net_hint(const StepParams& P, float Cf, floa
   const float rsum = xif.w + xjf.w;
   const float rs = xif.w * xjf.w / rsum;
   const float c = Cf / rs;
-  if (!(c >= kJkrCMin && c <= kJkrCMax)) return false;
+  if (!(c >= kJkrCMin && c <= kJkrCMax)) return CREC_HARD;
   const float c23 = jkr_c23(c);
   const float x = (rsum - sqrtf(fx * fx + fy * fy + fz * fz)) / rs;
+  const float xi = x / c23;
   const float X = fmaxf(fmaxf(fmaxf(fabsf(xif.x), fabsf(xif.y)), fabsf(xif.z)),
                         fmaxf(fmaxf(fabsf(xjf.x), fabsf(xjf.y)), fabsf(xjf.z)));
-  const float m = 0.02f + 2.4e-7f * (2.0f * X + rsum + P.lmax) / (rs * c23);
-  const float xi = x / c23;
-  if (xi < kJkrXiNeg - m) return false;
-  if (xi > m && xi < kJkrXiPos - m) return false;
+  const float e = 2.4e-7f * (2.0f * X + rsum + P.lmax) / (rs * c23);
+  const float h = 0.15f * e;  // the usual size of that rounding, not its bound
+  if (xi < kJkrXiNeg + h || (xi > kJkrXiWalk - h && xi < kJkrXiPos + h)) return CREC_HARD;
+  if (!learn) return 0u;
+  const float m = 0.02f + e;
+  if (xi < kJkrXiNeg - m) return 0u;
+  if (xi > m && xi < kJkrXiPos - m) return 0u;
   const float f1 = logf(rs);
-  if (f1 < P.jdom_lo[1] || f1 > P.jdom_hi[1]) return false;
-  if (sqrtf(fmaxf(xi - m + kJkrKappa, 0.0f)) > P.jdom_hi[0]) return false;
-  return true;
+  if (f1 < P.jdom_lo[1] || f1 > P.jdom_hi[1]) return 0u;
+  if (sqrtf(fmaxf(xi - m + kJkrKappa, 0.0f)) > P.jdom_hi[0]) return 0u;
+  return CREC_NET;
 }
 
 // Whether a JKR pair is certainly in the ZERO region of jkr_certify (no
@@ -1299,19 +1314,8 @@ __device__ __forceinline__ uint32_t warp_exclusive(uint32_t v, uint32_t& total) 
   return x - v;
 }
 
-// v slots of the array behind a device counter for each lane of the warp,
-// contiguous in lane order, with one atomic per warp: returns this lane's
-// first slot. Every lane of the warp takes part.
-__device__ __forceinline__ uint32_t warp_reserve(uint32_t* ctr, uint32_t v) {
-  uint32_t total;
-  const uint32_t ex = warp_exclusive(v, total);
-  uint32_t base = 0;
-  if ((threadIdx.x & 31) == 0 && total) base = atomicAdd(ctr, total);
-  return __shfl_sync(0xFFFFFFFFu, base, 0) + ex;
-}
-
 // The contact pass's counters (records, evaluating records, network queue,
-// deferred pairs, wall candidates) start every force pass at zero.
+// deferred pairs, wall candidates, hard pairs) start every force pass at zero.
 constexpr int CTOT_WORDS = 8;
 
 // Pass 1 (FP32 and integer work only): the candidates of each particle, i.e.
@@ -1319,113 +1323,179 @@ constexpr int CTOT_WORDS = 8;
 // visits from this end (visit counts from both ends recorded); marks the ones
 // that evaluate their pair (the lower slot of a pair seen from both ends, or
 // the only end that sees it). The pretest is symmetric, so a pair seen from
-// both ends is a candidate at both. Each warp then reserves, with one atomic
-// per counter, the result slots of its particles' records (coff) and their
-// places in the compact list of evaluating records (and the network queue):
-// where a record's result lands changes nothing in its value, and each
-// particle's results stay contiguous and in list order. The block size is a
-// multiple of 32 and every lane of a warp runs the same number of iterations.
+// both ends is a candidate at both. Each warp then reserves the result slots of
+// its particles' records (coff) and their places in the compact list of
+// evaluating records (and the queues of the JKR solvers), one atomic
+// instruction for all counters: where a record's result lands changes nothing
+// in its value, and each particle's results stay contiguous and in list order.
+// The block size is a multiple of 32 and every lane of a warp runs the same
+// number of iterations.
+//
+// Bound by the latency of the gathers, so a row is walked in two phases of up
+// to 32 entries: first four entries at a time, their indices in one 16-byte
+// load and their positions in flight together, into a mask of the entries that
+// pass; then the candidates, whose visit counts need no gather where the whole
+// neighbourhood lies in one reference cell (PF_ONECELL). One entry at a time
+// with the visit counts in between, the pass took 155 us on 1,048,576 spheres
+// (hopper, rows of 11) and 329 us on 2,097,152 adhesive ones; this form takes 122 and 176 us.
 template <bool PHYS, bool HIST>
 __global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
   Ctrl* C = P.ctrl;
   if (C->halt) return;
   const Bank B = P.bank[C->bank];
-  const bool adh = (P.nmodel == 3 || P.nmodel == 4);
   const bool learn_any = P.jkr_solver == 1 && P.nmodel == 3 && P.mlp != nullptr;
-  // Certified-zero JKR pairs add exactly +-0 to F and T when the tangential
-  // force then vanishes too (Coulomb with |F_n| = 0; physical-mode springs
-  // reset out of contact): with the certified solvers they are not
-  // candidates at all. Parity-mode springs (G* = 0, NaN for Mindlin at
-  // negative overlap) and debug recording keep every pair.
-  const bool zdrop_any = P.jkr_solver != 0 && P.nmodel == 3 && P.pretest && !P.debug && (P.tmodel == 0 || PHYS);
+  const bool hint_any = P.jfb != nullptr;  // a certified JKR solver
+  // JKR pairs certified to have no force add exactly +-0 to F and T (the
+  // tangential force then vanishes too, see StepParams::drop_zero): they are
+  // not candidates at all, whichever solver takes the others. The reference's
+  // own Newton, which returns zero for them after up to 20 steps, had spent
+  // nine tenths of its time on them (262,144 spheres at solid fraction 0.35:
+  // the step 2.68 -> 0.22 ms).
+  const bool zdrop_any = P.drop_zero && P.nmodel == 3;
   // the same for sJKR, whose zero region is explicit (no iteration to certify)
-  const bool sdrop = P.nmodel == 4 && P.pretest && !P.debug && (P.tmodel == 0 || PHYS);
+  const bool sdrop = P.drop_zero && P.nmodel == 4;
   const size_t plane = (size_t)P.n * P.cap;
+  const float margin = pretest_margin(P, C);
+  const int lane = threadIdx.x & 31;
   // slots in the rebuild-time order (tiles of 256 sorted by list length), so
   // a warp's lanes walk lists of similar length
   for (int i0 = blockIdx.x * blockDim.x; i0 < P.n; i0 += gridDim.x * blockDim.x) {
     const int i = i0 + (int)threadIdx.x;
     const int k = i < P.n ? (int)P.aorder[i] : -1;
-    uint32_t nrec = 0, ncmp = 0, nnet = 0, nw = 0, ts = 0, te = 0, gi = 0;
+    uint32_t nrec = 0, ncmp = 0, nnet = 0, nhard = 0, nw = 0, ts = 0, te = 0, gi = 0;
+    uint32_t evals = 0u;  // records (the first 32) that evaluate their pair
     float4 xif = make_float4(0.f, 0.f, 0.f, 0.f);
     float Xi = 0.f;
     const uint32_t flk = k >= 0 ? B.flags[k] : PF_DEAD;
     if (!(flk & PF_DEAD)) {
-      const unsigned long long ci = PHYS ? 0ull : (unsigned long long)__double_as_longlong(B.wc[k].w);
-      // visits of a neighbour in the same reference cell (most pairs at a 1 m
-      // cell): a constant, without the 27-cell walk of ref_visits
-      const int same = (PHYS || !ref_inside(P, ci)) ? 0 : P.same_cell_visits;
-      const Law lw = law_of(P, B, k);  // pairs never cross groups (the lists exclude them)
-      const bool adhesive = lw.gamma_pp > 0.0;
-      const bool learn = learn_any && adhesive, zdrop = zdrop_any && adhesive;
+      const bool onecell = PHYS || (flk & PF_ONECELL);
+      const int same = PHYS ? 1 : P.same_cell_visits;
+      const unsigned long long ci = onecell ? 0ull : (unsigned long long)__double_as_longlong(B.wc[k].w);
+      const int same_c = !PHYS && !onecell && ref_inside(P, ci) ? same : 0;
       xif = B.xf[k];
-      Xi = fmaxf(fmaxf(fabsf(xif.x), fabsf(xif.y)), fabsf(xif.z));
+      const bool image = !(flk & PF_NOIMAGE);
       const uint32_t cnt = B.ncnt[k];
       const uint32_t* row = B.nbr + (size_t)k * P.cap;
       CRec* out = P.crec + (size_t)k * P.cap;
-      unsigned long long hm = HIST ? B.hmask[k] : 0ull;
-      const unsigned long long hm0 = hm;
-      // the next two entries and their FP32 positions are loaded while this
-      // one is tested (rows and positions are read-only during the pass)
-      uint32_t jn = cnt > 0 ? __ldg(row) : 0u, jn2 = cnt > 1 ? __ldg(row + 1) : 0u;
-      float4 xn = cnt > 0 ? __ldg(B.xf + jn) : make_float4(0.f, 0.f, 0.f, 0.f);
-      float4 xn2 = cnt > 1 ? __ldg(B.xf + jn2) : make_float4(0.f, 0.f, 0.f, 0.f);
-      for (uint32_t m = 0; m < cnt; ++m) {
-        const uint32_t j = jn;
-        const float4 xjf = xn;
-        jn = jn2;
-        xn = xn2;
-        if (m + 2 < cnt) {
-          jn2 = __ldg(row + m + 2);
-          xn2 = __ldg(B.xf + jn2);
+      for (uint32_t c0 = 0; c0 < cnt; c0 += 32) {
+        const uint32_t ce = min(cnt - c0, 32u);
+        const uint32_t valid = 0xFFFFFFFFu >> (32u - ce);
+        uint32_t near = 0u;
+        if (P.pretest) {
+          for (uint32_t m = 0; m < ce; m += 4) {
+            uint4 j;
+            if ((P.cap & 3) == 0) {  // rows start on 16 bytes; entries past the end are not followed
+              j = __ldg(reinterpret_cast<const uint4*>(row + c0 + m));
+              if (m + 1 >= ce) j.y = j.x;
+              if (m + 2 >= ce) j.z = j.x;
+              if (m + 3 >= ce) j.w = j.x;
+            } else {
+              j.x = __ldg(row + c0 + m);
+              j.y = m + 1 < ce ? __ldg(row + c0 + m + 1) : j.x;
+              j.z = m + 2 < ce ? __ldg(row + c0 + m + 2) : j.x;
+              j.w = m + 3 < ce ? __ldg(row + c0 + m + 3) : j.x;
+            }
+            const float4 x0 = __ldg(B.xf + j.x), x1 = __ldg(B.xf + j.y), x2 = __ldg(B.xf + j.z), x3 = __ldg(B.xf + j.w);
+            const uint32_t q = (pretest_near(P, xif, x0, image, margin) ? 1u : 0u) |
+                               (pretest_near(P, xif, x1, image, margin) ? 2u : 0u) |
+                               (pretest_near(P, xif, x2, image, margin) ? 4u : 0u) |
+                               (pretest_near(P, xif, x3, image, margin) ? 8u : 0u);
+            near |= q << m;
+          }
+          near &= valid;
+        } else {
+          near = valid;
         }
-        const size_t hi = (size_t)k * P.cap + m;
-        int vij = 0, vji = 0;
-        if (!(P.pretest && pretest_far(P, xif, Xi, xjf, adh)) && !(zdrop && jkr_far_zero(P, lw.jkr_Cf, xif, Xi, xjf)) &&
-            !(sdrop && sjkr_far_zero(P, lw, xif, Xi, xjf))) {
-          if (PHYS) {
-            vij = vji = 1;
-          } else {
+        uint32_t kept = 0u;
+        for (uint32_t left = near; left; left &= left - 1u) {
+          const uint32_t b = (uint32_t)__ffs((int)left) - 1u, m = c0 + b;
+          const uint32_t j = __ldg(row + m);
+          uint32_t hint = 0u;
+          if (P.nmodel >= 3) {  // pairs never cross groups (the lists exclude them)
+            const Law lw = law_of(P, B, k);
+            const float4 xjf = __ldg(B.xf + j);
+            Xi = fmaxf(fmaxf(fabsf(xif.x), fabsf(xif.y)), fabsf(xif.z));
+            const bool adhesive = lw.gamma_pp > 0.0;
+            if (zdrop_any && adhesive && jkr_far_zero(P, lw.jkr_Cf, xif, Xi, xjf)) continue;
+            if (sdrop && sjkr_far_zero(P, lw, xif, Xi, xjf)) continue;
+            // (the higher slot of a pair seen from both ends does not evaluate it)
+            if (hint_any && adhesive && !(onecell && (uint32_t)k > j)) hint = jkr_hint(P, lw.jkr_Cf, xif, xjf, learn_any);
+          }
+          int vij = same, vji = same;
+          if (!onecell) {
             const unsigned long long cj = (unsigned long long)__double_as_longlong(B.wc[j].w);
             if (cj == ci) {
-              vij = vji = same;
+              vij = vji = same_c;
             } else {
               vij = ref_visits(P, ci, cj);
               vji = ref_visits(P, cj, ci);
             }
           }
-        }
-        if (vij > 0) {
+          if (vij == 0) continue;
+          kept |= 1u << b;
           const bool evaluates = !(vji > 0 && (uint32_t)k > j);
-          const uint32_t net = (learn && evaluates && jkr_net_hint(P, lw.jkr_Cf, xif, xjf)) ? CREC_NET : 0u;
-          out[nrec] = CRec{j, m | ((uint32_t)vij << 16) | ((uint32_t)vji << 24) | net};
+          if (evaluates) {
+            if (hint & CREC_HARD) ++nhard;
+            else ++ncmp;
+            if (hint & CREC_NET) ++nnet;
+            if (nrec < 32) evals |= 1u << nrec;
+          } else {
+            hint = 0u;
+          }
+          out[nrec] = CRec{j, m | ((uint32_t)vij << 16) | ((uint32_t)vji << 24) | hint};
           ++nrec;
-          if (evaluates) ++ncmp;
-          if (net) ++nnet;
-        } else {
-          // a spring out of reach resets; one already +0 (its bit clear) stays
-          if (HIST && (m >= 64 || ((hm >> m) & 1ull))) {
+        }
+        if (HIST) {
+          // a spring out of reach resets; one already +0 (its bit clear; entries past 64 have none) stays
+          uint32_t* hm = reinterpret_cast<uint32_t*>(B.hmask + k) + (c0 >> 5);
+          const uint32_t live = c0 < 64 ? *hm : 0xFFFFFFFFu;
+          const uint32_t reset = valid & ~kept & live;
+          for (uint32_t left = reset; left; left &= left - 1u) {
+            const size_t hi = (size_t)k * P.cap + c0 + (uint32_t)__ffs((int)left) - 1u;
             B.hist[hi] = 0.0;
             B.hist[plane + hi] = 0.0;
             B.hist[2 * plane + hi] = 0.0;
-            if (m < 64) hm &= ~(1ull << m);
           }
-          if (P.debug) P.dbgMult[hi] = 0;
+          if (c0 < 64 && reset) *hm = live & ~reset;
         }
+        if (P.debug)
+          for (uint32_t left = valid & ~kept; left; left &= left - 1u)
+            P.dbgMult[(size_t)k * P.cap + c0 + (uint32_t)__ffs((int)left) - 1u] = 0;
       }
-      if (HIST && hm != hm0) B.hmask[k] = hm;
       // wall candidates: the triangles of its triangle-grid cell that pass
       // the FP32 pretest, counted here and listed once the arena is reserved
       if (P.ntri > 0 && !(P.wall_far_ok && (flk & PF_WALLFAR)) && tri_cell_range(P, xif, ts, te)) {
+        Xi = fmaxf(fmaxf(fabsf(xif.x), fabsf(xif.y)), fabsf(xif.z));
         gi = P.ngroups > 1 ? B.grp[k] : 0u;
         for (uint32_t t = ts; t < te; ++t) nw += wall_pretest(P.tri[P.titems[t]], gi, xif, Xi) ? 1u : 0u;
       }
     }
     __syncwarp();
-    const uint32_t rb = warp_reserve(P.ctot, nrec);
-    uint32_t q = warp_reserve(P.ctot + 1, ncmp);
-    uint32_t qn = learn_any ? warp_reserve(P.ctot + 2, nnet) : 0u;
-    const uint32_t wb = P.ntri > 0 ? warp_reserve(P.ctot + 4, nw) : 0u;
+    // exclusive prefixes over the warp; records and evaluating records share a
+    // word where 32 rows cannot overflow its halves
+    uint32_t tr = 0, tc = 0, tn = 0, tw = 0, th = 0, rb, q, qn = 0, wb = 0, qh = 0;
+    if (P.cap < 2048) {
+      uint32_t t;
+      const uint32_t ex = warp_exclusive(nrec | (ncmp << 16), t);
+      rb = ex & 0xFFFFu;
+      q = ex >> 16;
+      tr = t & 0xFFFFu;
+      tc = t >> 16;
+    } else {
+      rb = warp_exclusive(nrec, tr);
+      q = warp_exclusive(ncmp, tc);
+    }
+    if (learn_any) qn = warp_exclusive(nnet, tn);
+    if (hint_any) qh = warp_exclusive(nhard, th);
+    if (__any_sync(0xFFFFFFFFu, nw != 0)) wb = warp_exclusive(nw, tw);
+    const uint32_t add = lane == 0 ? tr : lane == 1 ? tc : lane == 2 ? tn : lane == 4 ? tw : lane == 5 ? th : 0u;
+    uint32_t at = 0;
+    if (add) at = atomicAdd(P.ctot + lane, add);
+    rb += __shfl_sync(0xFFFFFFFFu, at, 0);
+    q += __shfl_sync(0xFFFFFFFFu, at, 1);
+    if (learn_any) qn += __shfl_sync(0xFFFFFFFFu, at, 2);
+    if (hint_any) qh += __shfl_sync(0xFFFFFFFFu, at, 5);
+    wb += __shfl_sync(0xFFFFFFFFu, at, 4);
     if (k < 0) continue;
     P.ccnt[k] = nrec;
     P.coff[k] = rb;
@@ -1444,17 +1514,26 @@ __global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
       P.wcnt[k] = nw;
       P.woff[k] = wb;
     }
-    if (ncmp == 0) continue;
-    // the evaluating records into the compact list (the queued ones into the
-    // network queue too), read back from the row this thread just wrote
+    if (ncmp + nhard == 0) continue;
+    // the evaluating records into the compact list
     const size_t base = (size_t)k * P.cap;
+    if (nrec <= 32 && !hint_any) {
+      for (uint32_t left = evals; left; left &= left - 1u)
+        P.clist[q++] = (uint32_t)(base + (uint32_t)__ffs((int)left) - 1u);
+      continue;
+    }
+    // read back from the row this thread just wrote: long rows, and the
+    // queues of the certified JKR solvers
     const CRec* out = P.crec + base;
     for (uint32_t c = 0; c < nrec; ++c) {
       const CRec r = out[c];
-      if (!(crec_vji(r.mv) > 0 && (uint32_t)k > r.j)) {
-        if (r.mv & CREC_NET) P.jq[qn++] = make_uint2(q, (uint32_t)(base + c));
-        P.clist[q++] = (uint32_t)(base + c);
+      if (crec_vji(r.mv) > 0 && (uint32_t)k > r.j) continue;
+      if (r.mv & CREC_HARD) {
+        P.jhard[qh++] = (uint32_t)(base + c);
+        continue;
       }
+      if (r.mv & CREC_NET) P.jq[qn++] = make_uint2(q, (uint32_t)(base + c));
+      P.clist[q++] = (uint32_t)(base + c);
     }
   }
 }
@@ -1469,12 +1548,8 @@ __global__ void __launch_bounds__(128) k_jkr_mlp(StepParams P) {
   if (C->halt) return;
   const uint32_t qn = P.ctot[2];
   if ((uint32_t)blockIdx.x * blockDim.x >= qn) return;
-  __shared__ MlpInfer M;
-  {
-    const uint4* src = reinterpret_cast<const uint4*>(P.mlp);
-    uint4* dst = reinterpret_cast<uint4*>(&M);
-    for (int i = threadIdx.x; i < (int)(sizeof(MlpInfer) / 16); i += blockDim.x) dst[i] = src[i];
-  }
+  __shared__ MlpShared M;
+  mlp_stage(M, P.mlp);
   __syncthreads();
   const Bank B = P.bank[C->bank];
   const int lane = threadIdx.x & 31;
@@ -1558,18 +1633,17 @@ __device__ __forceinline__ void put_result(const StepParams& P, uint32_t rec, T3
   }
 }
 
-template <bool PHYS, bool HIST, typename R>
-__device__ __forceinline__ bool contact_eval(const StepParams& P, const Bank& B, uint32_t t, bool first_pass,
-                                             bool& excess, uint32_t* tally) {
+template <bool PHYS, bool HIST, typename R, bool JKR>
+__device__ __forceinline__ bool contact_eval(const StepParams& P, const Bank& B, uint32_t s, float guess,
+                                             bool can_defer, bool newton, bool& excess, uint32_t* tally) {
   const size_t plane = (size_t)P.n * P.cap;
   const bool adh = (P.nmodel == 3 || P.nmodel == 4);
-  const uint32_t s = P.clist[t];
   const uint32_t k = s / (uint32_t)P.cap, c = s - k * (uint32_t)P.cap;
   const CRec r = P.crec[s];
   const uint32_t j = r.j, m = r.mv & 0xFFFFu;
   const int vij = (r.mv >> 16) & 0xFF, vji = crec_vji(r.mv);
-  const float guess = (first_pass && (r.mv & CREC_NET)) ? P.jguess[t] : -1.0f;
-  if (tally && (r.mv & CREC_NET)) tally[3] += 1;
+  if (!(r.mv & CREC_NET)) guess = -1.0f;
+  else if (tally) tally[3] += 1;
   const D4 xi4 = B.xr[k], xj4 = B.xr[j];
   const V d = mic(P, xyz(xi4) - xyz(xj4));
   const double d2 = dot(d, d);
@@ -1583,29 +1657,27 @@ __device__ __forceinline__ bool contact_eval(const StepParams& P, const Bank& B,
     const D4 vi4 = B.vm[k], wi4 = B.wc[k], vj4 = B.vm[j], wj4 = B.wc[j];
     const Law lw = law_of(P, B, (int)k);
     bool deferred = false;
-    const bool can_defer = first_pass && P.jfb != nullptr;
     if constexpr (PHYS && sizeof(R) == sizeof(double)) {
-      pair_contact_fused<HIST>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4), xyz(wi4), xyz(wj4),
-                               hk, plane, fc, nrm, excess, guess, tally, can_defer ? &deferred : nullptr,
-                               !first_pass);
+      pair_contact_fused<HIST, JKR>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4), xyz(wi4), xyz(wj4),
+                               hk, plane, fc, nrm, excess, guess, tally, can_defer ? &deferred : nullptr, newton);
       tc = (-xi4.w) * nrm;
       tc2 = (-xj4.w) * nrm;
     } else {
-      bool done = pair_contact<R, PHYS, HIST>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4),
+      bool done = pair_contact<R, PHYS, HIST, JKR>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4),
                                               xyz(wi4), xyz(wj4), hk, plane, fc, tc, nrm, excess, guess, tally,
-                                              can_defer ? &deferred : nullptr, !first_pass);
+                                              can_defer ? &deferred : nullptr, newton);
       if (!done) {  // FP32 cannot decide the pair
         V fd, td, nd;
         if constexpr (PHYS) {
-          pair_contact_fused<HIST>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4), xyz(wi4),
-                                   xyz(wj4), hk, plane, fd, nd, excess, guess, nullptr, nullptr, !first_pass);
+          pair_contact_fused<HIST, JKR>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4), xyz(wi4),
+                                   xyz(wj4), hk, plane, fd, nd, excess, guess, nullptr, nullptr, newton);
           fc = cvt<R>(fd);
           tc = cvt<R>((-xi4.w) * nd);
           tc2 = cvt<R>((-xj4.w) * nd);
         } else {
-          pair_contact<double, PHYS, HIST>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4),
+          pair_contact<double, PHYS, HIST, JKR>(P, lw, d, d2, rsum, xi4.w, xj4.w, vi4.w, vj4.w, xyz(vi4), xyz(vj4),
                                            xyz(wi4), xyz(wj4), hk, plane, fd, td, nd, excess, guess, nullptr,
-                                           nullptr, !first_pass);
+                                           nullptr, newton);
           fc = cvt<R>(fd);
           tc = cvt<R>(td);
           nrm = cvt<R>(nd);
@@ -1646,12 +1718,13 @@ __device__ __forceinline__ bool contact_eval(const StepParams& P, const Bank& B,
 // A wall candidate of the filter: the FP64 sphere-triangle contact
 // (src/simulation.rs:464-523); its force and torque are kept for
 // k_accumulate, which adds them after the pair contacts in mesh order.
+template <bool JKR>
 __device__ __forceinline__ void wall_eval(const StepParams& P, const Bank& B, uint32_t w, bool& excess) {
   const uint2 e = P.warena[w];
   const int k = (int)e.x;
   const D4 xi = B.xr[k], vi = B.vm[k], wi = B.wc[k];
   V fc, tc;
-  const bool ok = wall_contact(P, law_of(P, B, k), P.tri[e.y], xyz(xi), xyz(vi), xyz(wi), xi.w, vi.w, fc, tc, excess);
+  const bool ok = wall_contact<JKR>(P, law_of(P, B, k), P.tri[e.y], xyz(xi), xyz(vi), xyz(wi), xi.w, vi.w, fc, tc, excess);
   if (ok) {
     double2* o = reinterpret_cast<double2*>(P.wres + 6 * (size_t)w);
     o[0] = make_double2(fc.x, fc.y);
@@ -1661,9 +1734,20 @@ __device__ __forceinline__ void wall_eval(const StepParams& P, const Bank& B, ui
   P.wok[w] = ok ? 1 : 0;
 }
 
+// The JKR tallies of a warp's threads into the control block. Every lane of the
+// warp takes part.
+__device__ __forceinline__ void add_tally(Ctrl* C, const uint32_t tally[6]) {
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    const uint32_t v = __reduce_add_sync(0xFFFFFFFFu, tally[q]);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(&C->jkr_count[q], (unsigned long long)v);
+  }
+}
+
 // Pass 3: one thread per evaluating record, then one per wall candidate (the
 // few wall contacts spread over the whole grid with the pairs).
-template <bool PHYS, bool HIST, typename R>
+template <bool PHYS, bool HIST, typename R, bool JKR>
 __global__ void __launch_bounds__(256) k_contact_force(StepParams P) {
   Ctrl* C = P.ctrl;
   if (C->halt) return;
@@ -1673,10 +1757,18 @@ __global__ void __launch_bounds__(256) k_contact_force(StepParams P) {
   bool excess = false;
   uint32_t tally[6] = {0u, 0u, 0u, 0u, 0u, 0u};
   const int lane = threadIdx.x & 31;
+  const bool learn = P.jkr_solver == 1 && P.nmodel == 3 && P.mlp != nullptr;
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < items; t += gridDim.x * blockDim.x) {
     bool deferred = false;
-    if (t < total) deferred = contact_eval<PHYS, HIST, R>(P, B, t, true, excess, tally);
-    else wall_eval(P, B, t - total, excess);
+    uint32_t s = 0;
+    if (t < total) {
+      s = P.clist[t];
+      deferred = contact_eval<PHYS, HIST, R, JKR>(P, B, s, JKR && learn ? P.jguess[t] : -1.0f, JKR && P.jfb != nullptr,
+                                                  false, excess, JKR ? tally : nullptr);
+    } else {
+      wall_eval<JKR>(P, B, t - total, excess);
+    }
+    if (!JKR) continue;
     // append the deferred pairs with one atomic per warp
     const unsigned act = __activemask();
     const unsigned bal = __ballot_sync(act, deferred);
@@ -1685,23 +1777,42 @@ __global__ void __launch_bounds__(256) k_contact_force(StepParams P) {
       uint32_t base = 0;
       if (lane == leader) base = atomicAdd(P.ctot + 3, (uint32_t)__popc(bal));
       base = __shfl_sync(act, base, leader);
-      if (deferred) P.jfb[base + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = t;
+      if (deferred) P.jfb[base + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = s;
     }
   }
   if (excess) C->overlap_flag = 1;
-  if (P.jkr_solver != 0 && P.nmodel == 3) {
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      const uint32_t v = __reduce_add_sync(0xFFFFFFFFu, tally[q]);
-      if ((threadIdx.x & 31) == 0 && v) atomicAdd(&C->jkr_count[q], (unsigned long long)v);
-    }
-  }
+  if (JKR && P.jkr_solver != 0) add_tally(C, tally);
 }
 
-// The deferred pairs of k_contact_force, one thread each, with the
-// reference's Newton iteration for their JKR force.
+// The pairs that the filter found next to the JKR fold, one thread each: the
+// exact certificates decide, and most run the reference's Newton iteration, up
+// to 20 steps of ~55 dependent FP64 instructions: ~57 us for a single warp,
+// which the whole force pass waited for after the pair kernel. This kernel runs
+// beside the network and the pair kernel, which it does not depend on. In the
+// mixed form a pair takes the FP32 law first, as the others do, and FP64 for the
+// Newton.
 template <bool PHYS, bool HIST, typename R>
+__global__ void __launch_bounds__(128) k_contact_hard(StepParams P) {
+  Ctrl* C = P.ctrl;
+  if (C->halt) return;
+  const Bank B = P.bank[C->bank];
+  const uint32_t total = P.ctot[5];
+  bool excess = false;
+  uint32_t tally[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const uint32_t s = P.jhard[i];
+    constexpr bool f32 = sizeof(R) == sizeof(float);
+    const bool deferred = contact_eval<PHYS, HIST, R, true>(P, B, s, -1.0f, f32, false, excess, tally);
+    if (f32 && deferred) contact_eval<PHYS, HIST, double, true>(P, B, s, -1.0f, false, true, excess, nullptr);
+  }
+  if (excess) C->overlap_flag = 1;
+  add_tally(C, tally);
+}
+
+// The deferred pairs of k_contact_force (few: the filter's hint sends most of
+// their kind to k_contact_hard), one thread each, with the reference's Newton
+// iteration for their JKR force.
+template <bool PHYS, bool HIST>
 __global__ void __launch_bounds__(128) k_contact_deferred(StepParams P) {
   Ctrl* C = P.ctrl;
   if (C->halt) return;
@@ -1709,7 +1820,7 @@ __global__ void __launch_bounds__(128) k_contact_deferred(StepParams P) {
   const uint32_t total = P.ctot[3];
   bool excess = false;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
-    contact_eval<PHYS, HIST, R>(P, B, P.jfb[i], false, excess, nullptr);
+    contact_eval<PHYS, HIST, double, true>(P, B, P.jfb[i], -1.0f, false, true, excess, nullptr);
   if (excess) C->overlap_flag = 1;
 }
 
@@ -1761,6 +1872,32 @@ __device__ bool wall_far(const StepParams& P, float4 xf) {
   return true;
 }
 
+// PF_NOIMAGE and PF_ONECELL of a particle at xf (its position at a list
+// rebuild) with reference-cell code c: whether a partner within reach can be a
+// periodic image, or lie in another reference cell, before the next rebuild.
+// Until then each of the two moves less than half the skin, so a partner that
+// is within the cutoff then lies within cutoff + skin / 2 of the particle's
+// position now, and the particle's own cell changes only across that distance
+// too; home_margin covers the rounding of the mirror and of the pretest. A
+// partner may lie up to `out` beyond a periodic face at the rebuild (and no
+// farther than half the skin later).
+__device__ uint32_t home_flags(const StepParams& P, float4 xf, long long c, float out) {
+  const float p[3] = {xf.x, xf.y, xf.z};
+  const float reach = (xf.w + P.rmaxf) * P.cut_a + (float)P.skin + P.home_margin;
+  uint32_t f = PF_NOIMAGE | PF_ONECELL;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float lo = (float)P.bmin[a], hi = (float)P.bmax[a];
+    if (P.periodic[a] && !(p[a] - lo > reach + out && hi - p[a] > reach + out)) f = 0u;
+    const float q = (p[a] - lo) * (float)P.inv_href, r = reach * (float)P.inv_href;
+    const float g = floorf(q);
+    if (!(g >= 0.0f && g < (float)P.rdims[a] && q - g > r && (g + 1.0f) - q > r &&
+          (int)g == code_axis((unsigned long long)c, a)))
+      f &= ~PF_ONECELL;
+  }
+  return f;
+}
+
 // The visiting order of k_accumulate, at a list rebuild: within each tile of
 // 256 slots a counting sort by (triangles listed in the triangle-grid cell,
 // Verlet-list length), dead slots after the live ones. Reads the bank the
@@ -1785,7 +1922,8 @@ __global__ void __launch_bounds__(ACC_TILE) k_accum_order(StepParams P) {
         const float4 xf = B.xf[k0];
         if (P.ntri > 0 && tri_cell_nonempty(P, xf)) key += 64;
         const bool far = P.ntri > 0 && P.wall_far_ok && wall_far(P, xf);
-        B.flags[k0] = far ? (fl | PF_WALLFAR) : (fl & ~PF_WALLFAR);
+        const uint32_t home = home_flags(P, xf, __double_as_longlong(B.wc[k0].w), __uint_as_float(P.ctrl->xout));
+        B.flags[k0] = (fl & ~(PF_WALLFAR | PF_NOIMAGE | PF_ONECELL)) | (far ? PF_WALLFAR : 0u) | home;
       }
     }
     for (uint32_t i = threadIdx.x; i < ACC_BINS; i += blockDim.x) bins[i] = 0;
@@ -2053,12 +2191,12 @@ int launch_rebuild_condition(const StepParams& P, cudaGraphConditionalHandle h, 
   return 1;
 }
 
-template <typename R>
+template <typename R, bool JKR>
 static void launch_force_t(const StepParams& P, int g, cudaStream_t s) {
   const bool hist = P.mode == 1 && P.tmodel != 0;
-  if (P.mode == 0) k_force<false, false, R><<<g, 128, 0, s>>>(P);
-  else if (hist) k_force<true, true, R><<<g, 128, 0, s>>>(P);
-  else k_force<true, false, R><<<g, 128, 0, s>>>(P);
+  if (P.mode == 0) k_force<false, false, R, JKR><<<g, 128, 0, s>>>(P);
+  else if (hist) k_force<true, true, R, JKR><<<g, 128, 0, s>>>(P);
+  else k_force<true, false, R, JKR><<<g, 128, 0, s>>>(P);
 }
 
 // Grid for a grid-stride kernel of block `bs` over n items, at most `cap` blocks.
@@ -2069,8 +2207,8 @@ static int shaped_grid(uint64_t n, int bs, int cap) {
   return (int)g;
 }
 
-template <typename R>
-static int launch_contact_path(const StepParams& P, cudaStream_t s) {
+template <typename R, bool JKR>
+static int launch_contact_path(const StepParams& P, cudaStream_t s, const SideStream& side) {
   const int bf = P.bs_filter > 0 ? P.bs_filter : 128, bc = P.bs_force > 0 ? P.bs_force : 128,
             ba = P.bs_accum > 0 ? P.bs_accum : 128, cap = P.grid_cap > 0 ? P.grid_cap : P.nsm * 64;
   const int g = shaped_grid((uint64_t)P.n, bf, cap);
@@ -2081,20 +2219,30 @@ static int launch_contact_path(const StepParams& P, cudaStream_t s) {
   else k_contact_filter<true, false><<<g, bf, 0, s>>>(P);
   const bool learn = P.jkr_solver == 1 && P.nmodel == 3 && P.mlp != nullptr;
   int launched = 3;
+  if (P.jfb != nullptr) {
+    cudaEventRecord(side.fork, s);
+    cudaStreamWaitEvent(side.stream, side.fork, 0);
+    if (P.mode == 0) k_contact_hard<false, false, R><<<P.nsm * 8, 128, 0, side.stream>>>(P);
+    else if (hist) k_contact_hard<true, true, R><<<P.nsm * 8, 128, 0, side.stream>>>(P);
+    else k_contact_hard<true, false, R><<<P.nsm * 8, 128, 0, side.stream>>>(P);
+    cudaEventRecord(side.join, side.stream);
+    ++launched;
+  }
   if (learn) {
     k_jkr_mlp<<<P.nsm * 4, 128, 0, s>>>(P);
     ++launched;
   }
   const int gc = shaped_grid((uint64_t)P.n * 4, bc, cap);
-  if (P.mode == 0) k_contact_force<false, false, R><<<gc, bc, 0, s>>>(P);
-  else if (hist) k_contact_force<true, true, R><<<gc, bc, 0, s>>>(P);
-  else k_contact_force<true, false, R><<<gc, bc, 0, s>>>(P);
+  if (P.mode == 0) k_contact_force<false, false, R, JKR><<<gc, bc, 0, s>>>(P);
+  else if (hist) k_contact_force<true, true, R, JKR><<<gc, bc, 0, s>>>(P);
+  else k_contact_force<true, false, R, JKR><<<gc, bc, 0, s>>>(P);
   if (P.jfb != nullptr) {
     // the deferred pairs lie in the band next to the JKR fold, where only
     // FP64 resolves the contact radius: FP64 in the mixed form too
-    if (P.mode == 0) k_contact_deferred<false, false, double><<<P.nsm * 8, 128, 0, s>>>(P);
-    else if (hist) k_contact_deferred<true, true, double><<<P.nsm * 8, 128, 0, s>>>(P);
-    else k_contact_deferred<true, false, double><<<P.nsm * 8, 128, 0, s>>>(P);
+    if (P.mode == 0) k_contact_deferred<false, false><<<P.nsm, 128, 0, s>>>(P);
+    else if (hist) k_contact_deferred<true, true><<<P.nsm, 128, 0, s>>>(P);
+    else k_contact_deferred<true, false><<<P.nsm, 128, 0, s>>>(P);
+    cudaStreamWaitEvent(s, side.join, 0);
     ++launched;
   }
   if (P.prec == 1) k_accumulate<true><<<shaped_grid((uint64_t)P.n, ba, cap), ba, 0, s>>>(P);
@@ -2102,12 +2250,21 @@ static int launch_contact_path(const StepParams& P, cudaStream_t s) {
   return launched;
 }
 
-int launch_force(const StepParams& P, cudaStream_t s) {
+int launch_force(const StepParams& P, cudaStream_t s, const SideStream& side) {
   if (P.n == 0) return 0;
-  if (P.force_path == 0) return P.prec == 1 ? launch_contact_path<float>(P, s) : launch_contact_path<double>(P, s);
+  if (P.force_path == 0) {
+    if (P.nmodel == 3)
+      return P.prec == 1 ? launch_contact_path<float, true>(P, s, side) : launch_contact_path<double, true>(P, s, side);
+    return P.prec == 1 ? launch_contact_path<float, false>(P, s, side) : launch_contact_path<double, false>(P, s, side);
+  }
   const int g = grid_for(P.n, 128);
-  if (P.prec == 1) launch_force_t<float>(P, g, s);
-  else launch_force_t<double>(P, g, s);
+  if (P.nmodel == 3) {
+    if (P.prec == 1) launch_force_t<float, true>(P, g, s);
+    else launch_force_t<double, true>(P, g, s);
+  } else {
+    if (P.prec == 1) launch_force_t<float, false>(P, g, s);
+    else launch_force_t<double, false>(P, g, s);
+  }
   return 1;
 }
 

@@ -19,9 +19,13 @@ struct alignas(32) D4 {
   double x, y, z, w;
 };
 
-// PF_WALLFAR (set at each list rebuild, with wall_far_ok): no triangle within
-// reach of the slot until the next rebuild, so the filter skips its walls
-enum : uint32_t { PF_FIXED = 1u, PF_DEAD = 2u, PF_WALLFAR = 4u };
+// Set at each list rebuild and true until the next one:
+//   PF_WALLFAR (with wall_far_ok): no triangle within reach of the slot, so the
+//              filter skips its walls
+//   PF_NOIMAGE no pair of the slot is a periodic image
+//   PF_ONECELL every partner within reach lies in the slot's own reference
+//              cell (parity mode; implies PF_NOIMAGE)
+enum : uint32_t { PF_FIXED = 1u, PF_DEAD = 2u, PF_WALLFAR = 4u, PF_NOIMAGE = 8u, PF_ONECELL = 16u };
 
 enum : unsigned { ST_OVERLAP = 1u, ST_NAN = 2u, ST_NLIST_GROW = 4u, ST_WALL_GROW = 8u };
 
@@ -39,6 +43,8 @@ struct Ctrl {
   unsigned long long overlap_steps;
   int pending;                    // the last completed step still owes its second half kick
   unsigned int wall_need;         // wall candidates a halted filter wanted room for
+  unsigned int xmax;              // bits of the largest |coordinate| of the FP32 mirror since the upload
+  unsigned int xout;              // list rebuild: bits of the farthest distance of a particle outside the periodic faces
   unsigned long long target;      // device step loop: run while steps_done < target
   unsigned long long iters;       // device step loop iterations (bounded by target + 4)
   // learned JKR tallies (pair evaluations): network/certified-solver results
@@ -115,9 +121,10 @@ struct TriRec {
 
 // A contact candidate kept by the filter: neighbour slot, row position and
 // the reference's visit counts from both ends (m | vis_ij << 16 | vis_ji << 24,
-// visit counts <= 27), bit 31 set when the pair is queued for the JKR network.
-constexpr uint32_t CREC_NET = 0x80000000u;
-__host__ __device__ __forceinline__ int crec_vji(uint32_t mv) { return (int)((mv >> 24) & 0x7Fu); }
+// visit counts <= 27), bit 31 set when the pair is queued for the JKR network,
+// bit 30 when it goes to the list of pairs that need the reference's Newton.
+constexpr uint32_t CREC_NET = 0x80000000u, CREC_HARD = 0x40000000u;
+__host__ __device__ __forceinline__ int crec_vji(uint32_t mv) { return (int)((mv >> 24) & 0x3Fu); }
 struct CRec {
   uint32_t j;
   uint32_t mv;
@@ -146,8 +153,10 @@ struct StepParams {
   uint32_t wcap;    // wall candidate capacity
   uint32_t* coff;   // first result slot of particle k (its ccnt results are contiguous)
   uint32_t* clist;  // compact list of evaluating record slots
-  uint32_t* ctot;   // [0] records, [1] evaluating records, [2] network queue, [3] deferred pairs, [4] wall candidates
-  uint32_t* jfb;    // evaluating indices deferred to the reference-Newton pass (null: no deferral)
+  // [0] records, [1] evaluating records, [2] network queue, [3] deferred pairs, [4] wall candidates, [5] hard pairs
+  uint32_t* ctot;
+  uint32_t* jfb;    // record slots deferred to the reference-Newton pass (null: no deferral)
+  uint32_t* jhard;  // record slots that the filter sends to that Newton at once (null with jfb)
   double* cres;     // per record: force (3) and torque (3) on the row's particle
   float* cresf;     // the same buffer as FP32 records (the mixed form: its pair forces are FP32 values)
   int nmodel, tmodel, mode, prec;
@@ -179,6 +188,15 @@ struct StepParams {
   uint32_t fncells;
   double skin;
   float list_scale;  // 1 + relative margin of the FP32 list test
+  // distance within which a pair can exert a force: min(r_sum cut_a, r_sum +
+  // cut_b); the lists hold it plus the skin
+  float cut_a, cut_b;
+  float cutmaxf;     // the largest such distance: 2 r_max cut_a
+  // adhesive pairs whose normal force is certainly zero are left out: their
+  // tangential force vanishes too (Coulomb with |F_n| = 0; physical springs
+  // reset out of contact), while parity-mode springs (G* = 0, NaN for Mindlin
+  // at a negative overlap) and debug recording keep every pair of the cutoff
+  int drop_zero;
   int pretest;       // FP32 pair pretest enabled (off when a periodic length < 4 cutoffs)
   float lmax;        // largest periodic length (enters the pretest rounding bound)
   // triangles
@@ -190,6 +208,7 @@ struct StepParams {
   const uint32_t* tstart;
   const uint32_t* titems;
   const WallMotion* motions;
+  float home_margin;     // margin of PF_NOIMAGE and PF_ONECELL
   int wall_far_ok;       // the triangle-grid cell exceeds half the skin: PF_WALLFAR is set and read
   float wall_far_gap;    // half the skin with margin: the distance a slot keeps from a periodic face
   // JKR solver for particle pairs: 0 the reference's Newton, 1 certificates +

@@ -64,7 +64,13 @@ int launch_first_half(const StepParams& P, cudaStream_t s);  // each returns ker
 int launch_second_half(const StepParams& P, cudaStream_t s);
 int launch_rebuild_condition(const StepParams& P, cudaGraphConditionalHandle h, cudaStream_t s);
 int launch_end_step_loop(const StepParams& P, cudaGraphConditionalHandle loop, cudaStream_t s);
-int launch_force(const StepParams& P, cudaStream_t s);
+// A second stream for work that runs beside the force pass, with the events
+// that fork it from the pass's stream and join it again.
+struct SideStream {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+};
+int launch_force(const StepParams& P, cudaStream_t s, const SideStream& side);
 int launch_accum_order(const StepParams& P, cudaStream_t s);  // inside the rebuild chain, before the bank flip
 int launch_end_step(const StepParams& P, cudaStream_t s);
 // Kinetic energy (translational + rotational) of the live slots, FP64.

@@ -60,6 +60,17 @@ struct alignas(16) MlpInfer {
   float xmean[4], xinv[4], ymean, ystd;
 };
 
+// The same in shared memory, its weight rows padded: a fragment load reads 8
+// rows x 4 words, and rows of 64 (or 16) 16-bit weights put all 8 rows on the
+// same banks (8-way conflicts, two thirds of the network kernel's time: 57,000
+// rows took 28.8 us, 14.6 with rows of 72 and 24).
+struct alignas(16) MlpShared {
+  static constexpr int LD1 = 24, LD = MLP_H + 8;
+  uint16_t w1[MLP_H * LD1], w2[MLP_H * LD], w3[MLP_H * LD], w4[8 * LD];
+  float b1[MLP_H], b2[MLP_H], b3[MLP_H], b4;
+  float xmean[4], xinv[4], ymean, ystd;
+};
+
 // ---------------------------------------------------------- certificates
 constexpr float kJkrKappa = 0.472470394f;  // 16^(-1/6) - 16^(-2/3)
 constexpr float kJkrXiNeg = -0.4525f;      // delta <= 0: xi >= this (roots merge at -kappa)
@@ -140,6 +151,24 @@ __device__ __forceinline__ void mma_bf16(float c[4], const uint32_t a[4], uint32
 
 __device__ __forceinline__ uint32_t ld_pair(const uint16_t* p) { return *reinterpret_cast<const uint32_t*>(p); }
 
+// The weights from global into shared memory, by the whole block (a barrier
+// must follow), 16 bytes at a time (8 weights; rows stay 16-byte aligned).
+__device__ __forceinline__ void mlp_stage(MlpShared& S, const MlpInfer* M) {
+  const int n = blockDim.x;
+  auto rows = [&](uint16_t* dst, const uint16_t* src, int count, int width, int ld) {
+    const int per = width / 8;
+    for (int i = threadIdx.x; i < count * per; i += n)
+      *reinterpret_cast<uint4*>(dst + (i / per) * ld + (i % per) * 8) = *reinterpret_cast<const uint4*>(src + i * 8);
+  };
+  rows(S.w1, M->w1, MLP_H, 16, MlpShared::LD1);
+  rows(S.w2, M->w2, MLP_H, MLP_H, MlpShared::LD);
+  rows(S.w3, M->w3, MLP_H, MLP_H, MlpShared::LD);
+  rows(S.w4, M->w4, 8, MLP_H, MlpShared::LD);
+  float* dst = S.b1;  // the biases and scalings follow each other in both
+  const float* src = M->b1;
+  for (int i = threadIdx.x; i < 3 * MLP_H + 1 + 10; i += n) dst[i] = src[i];
+}
+
 // One hidden layer on a 16-row tile: 4 k-tiles of A fragments in (64 inputs),
 // 8 n-tiles of C fragments out (64 outputs), bias added. B fragments come
 // straight from the row-major [out][in] weights: B[k][n] = W[n][k].
@@ -152,7 +181,7 @@ __device__ __forceinline__ void mlp_layer64(const uint16_t* w, const float* b, c
     acc[nt][1] = bh;
     acc[nt][2] = bl;
     acc[nt][3] = bh;
-    const uint16_t* wr = w + (nt * 8 + g) * MLP_H + tig * 2;
+    const uint16_t* wr = w + (nt * 8 + g) * MlpShared::LD + tig * 2;
 #pragma unroll
     for (int kt = 0; kt < 4; ++kt) mma_bf16(acc[nt], ain[kt], ld_pair(wr + kt * 16), ld_pair(wr + kt * 16 + 8));
   }
@@ -173,8 +202,8 @@ __device__ __forceinline__ void mlp_repack(const float acc[8][4], uint32_t aout[
 
 // Warp-wide forward pass for 32 rows (lane L owns row L): normalised features
 // in, normalised prediction out. All 32 lanes must call it together (the
-// mma.sync instructions are warp-collective). M may point to shared memory.
-__device__ __forceinline__ float mlp_forward_warp(const MlpInfer* M, const float f[4]) {
+// mma.sync instructions are warp-collective).
+__device__ __forceinline__ float mlp_forward_warp(const MlpShared* M, const float f[4]) {
   const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
   float out_tile[2] = {0.f, 0.f};
 #pragma unroll 1
@@ -201,7 +230,7 @@ __device__ __forceinline__ float mlp_forward_warp(const MlpInfer* M, const float
       acc[nt][1] = bh;
       acc[nt][2] = bl;
       acc[nt][3] = bh;
-      const uint16_t* wr = M->w1 + (nt * 8 + g) * 16 + tig * 2;
+      const uint16_t* wr = M->w1 + (nt * 8 + g) * MlpShared::LD1 + tig * 2;
       mma_bf16(acc[nt], a1, ld_pair(wr), ld_pair(wr + 8));
     }
     uint32_t a[4][4];
@@ -211,7 +240,7 @@ __device__ __forceinline__ float mlp_forward_warp(const MlpInfer* M, const float
     mlp_layer64(M->w3, M->b3, a, acc, g, tig);
     mlp_repack(acc, a);
     float o[4] = {M->b4, 0.f, M->b4, 0.f};
-    const uint16_t* wr = M->w4 + g * MLP_H + tig * 2;
+    const uint16_t* wr = M->w4 + g * MlpShared::LD + tig * 2;
 #pragma unroll
     for (int kt = 0; kt < 4; ++kt) mma_bf16(o, a[kt], ld_pair(wr + kt * 16), ld_pair(wr + kt * 16 + 8));
     // output column 0 of row r (0..15) sits in lane 4 (r mod 8): o[0] for r < 8, o[2] above
