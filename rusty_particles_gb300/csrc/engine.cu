@@ -334,8 +334,8 @@ int Engine::alloc_slots(size_t n) {
   TRY(dalloc(&woff_, na)); TRY(dalloc(&wcnt_, na));
   TRY(alloc_walls(std::max(wcap_, na / 2 + 65536)));
   TRY(dalloc(&ccnt_, na)); TRY(dalloc(&coff_, na));
-  TRY(dalloc(&ctot_, 8));
-  CK(cudaMemset(ctot_, 0, 8 * sizeof(uint32_t)));
+  TRY(dalloc(&ctot_, 16));
+  CK(cudaMemset(ctot_, 0, 16 * sizeof(uint32_t)));
   n_alloc_ = na;
   // lists must be re-allocated for the new slot count
   for (int b = 0; b < 2; ++b) {
@@ -1018,6 +1018,10 @@ int Engine::finish_step_accounting() {
 // bank's rows for the history carry-over) or the arena, and finish that step.
 int Engine::recover_halt() {
   while (ctrl_h_->halt) {
+    if (ctrl_h_->halt & HALT_STUCK) {
+      set_error("the device step loop's blocks did not meet in time");
+      return RP_E_DEVICE_FLAG;
+    }
     if (ctrl_h_->halt & HALT_LISTS) {
       int newcap = grown_capacity(ctrl_h_->max_count);
       TRY(alloc_lists(newcap, true));
@@ -1055,7 +1059,9 @@ void Engine::destroy_graph() {
 // step). k_end_step sets the loop condition from the device counters, so a
 // stepping call of any length is one graph launch and the host never has to
 // decide whether a step needs a rebuild.
-int Engine::build_graph() {
+// Small beds (steps_in_one_launch) run many steps in each iteration: the body
+// is k_steps, the IF node with the rebuild chain, and the loop condition.
+int Engine::build_graph(bool small) {
   destroy_graph();
   if (!cap_stream_) {
     CK(cudaStreamCreateWithFlags(&cap_stream_, cudaStreamNonBlocking));
@@ -1077,8 +1083,21 @@ int Engine::build_graph() {
   cudaGraphConditionalHandle hif;
   CK(cudaGraphConditionalHandleCreate(&hif, body, 0, cudaGraphCondAssignDefault));
   CK(cudaStreamBeginCaptureToGraph(cap_stream_, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-  int sk = launch_first_half(P_, cap_stream_);
-  sk += launch_rebuild_condition(P_, hif, cap_stream_);
+  int sk = 0;
+  if (small) {
+    CK(cudaMemsetAsync(ctot_, 0, 16 * sizeof(uint32_t), cap_stream_));
+    const int k = launch_steps_small(P_, cap_stream_);
+    if (k == 0) {
+      cudaGraph_t t0 = nullptr;
+      cudaStreamEndCapture(cap_stream_, &t0);
+      set_error("cooperative launch not available");
+      return RP_E_CUDA;
+    }
+    sk = k + launch_steps_next(P_, hif, hloop, 0, cap_stream_);
+  } else {
+    sk = launch_first_half(P_, cap_stream_);
+    sk += launch_rebuild_condition(P_, hif, cap_stream_);
+  }
   cudaStreamCaptureStatus st;
   cudaGraph_t cg = nullptr;
   const cudaGraphNode_t* deps = nullptr;
@@ -1097,9 +1116,14 @@ int Engine::build_graph() {
   chain_kernels_ = launch_rebuild(P_, rb_, cap_stream2_);
   cudaGraph_t t2 = nullptr;
   CK(cudaStreamEndCapture(cap_stream2_, &t2));
-  sk += launch_force(P_, cap_stream_, side_);
-  sk += launch_end_step_loop(P_, hloop, cap_stream_);
+  if (small) {
+    sk += launch_steps_next(P_, hif, hloop, 1, cap_stream_);
+  } else {
+    sk += launch_force(P_, cap_stream_, side_);
+    sk += launch_end_step_loop(P_, hloop, cap_stream_);
+  }
   step_kernels_ = sk;
+  small_loop_ = small;
   cudaGraph_t t1 = nullptr;
   CK(cudaStreamEndCapture(cap_stream_, &t1));
   CK(cudaGraphInstantiate(&graph_exec_, g, 0));
@@ -1114,7 +1138,15 @@ int Engine::launch_steps_graph(uint64_t n) {
     // capacity): recover_halt reallocates the lists, so it is rebuilt before
     // every launch that follows a change.
     if (graph_dirty_ || !graph_exec_) {
-      int r = build_graph();
+      int r = RP_E_CUDA;
+      if (small_ok_ && steps_in_one_launch(P_)) {
+        r = build_graph(true);
+        if (r != RP_OK) {
+          small_ok_ = false;
+          cudaGetLastError();
+        }
+      }
+      if (r != RP_OK) r = build_graph(false);
       if (r != RP_OK) {
         // conditional graph nodes unavailable: host-issued steps instead
         destroy_graph();
@@ -1135,7 +1167,7 @@ int Engine::launch_steps_graph(uint64_t n) {
     cudaEventElapsedTime(&ms, ev0_, ev1_);
     ms_total_ += ms;
     TRY(recover_halt());
-    launches_ += (uint64_t)step_kernels_ * (ctrl_h_->steps_done - before) +
+    launches_ += (uint64_t)step_kernels_ * (small_loop_ ? ctrl_h_->iters : ctrl_h_->steps_done - before) +
                  (uint64_t)chain_kernels_ * (ctrl_h_->rebuilds - rb_before);
     TRY(finish_step_accounting());
     const uint64_t done = last_.steps_done - before;

@@ -148,7 +148,8 @@ class Engine {
   uint8_t* dbgMult_ = nullptr;
   // contact-parallel force buffers
   CRec* crec_ = nullptr;
-  uint32_t *ccnt_ = nullptr, *coff_ = nullptr, *clist_ = nullptr;
+  uint32_t *ccnt_ = nullptr, *coff_ = nullptr;
+  uint4* clist_ = nullptr;
   uint32_t* aorder_ = nullptr;  // k_accumulate visiting order (set at every list rebuild)
   uint2* warena_ = nullptr;     // wall candidates of the force pass
   double* wres_ = nullptr;      // their results
@@ -165,11 +166,11 @@ class Engine {
   float jkr_norm_[10] = {};
   float jkr_dom_[8] = {};
   MlpInfer* mlp_d_ = nullptr;
-  uint2* jq_ = nullptr;
+  uint32_t* jq_ = nullptr;
   float* jguess_ = nullptr;
   size_t jq_alloc_ = 0;
   uint32_t* jfb_ = nullptr;    // pairs deferred to the reference-Newton pass
-  uint32_t* jhard_ = nullptr;  // pairs that the filter sends to it at once
+  uint4* jhard_ = nullptr;  // pairs that the filter sends to it at once
   SideStream side_;
   size_t jfb_alloc_ = 0;
   int ensure_jkr_buffers();
@@ -208,7 +209,9 @@ class Engine {
   void free_lists();
   int launch_steps(uint64_t n);
   int launch_steps_graph(uint64_t n);
-  int build_graph();
+  int build_graph(bool small);
+  bool small_loop_ = false;  // the graph's body runs many steps an iteration (k_steps)
+  bool small_ok_ = true;     // cooperative launches can be captured
   void destroy_graph();
   int recover_halt();
   int alloc_walls(size_t cap);

@@ -768,6 +768,15 @@ __device__ __forceinline__ void second_half_kick(V& v, V& vres, V& w, V& wres, V
   w = tw;
 }
 
+// A thread's items of a pass: at, at + all, at + 2 all, ... (the lanes of a warp
+// next to each other).
+struct Span {
+  int at, all;
+};
+__device__ __forceinline__ Span grid_span() {
+  return Span{(int)(blockIdx.x * blockDim.x + threadIdx.x), (int)(gridDim.x * blockDim.x)};
+}
+
 // ------------------------------------------------------------- first half
 // The force kernel only writes a and tau: neighbours read v and omega while
 // it runs, so the second half kick of step n-1 is applied here, at the start
@@ -788,12 +797,10 @@ __device__ __forceinline__ void second_half_kick(V& v, V& vres, V& w, V& wres, V
 // step's second half kick pending, the two half kicks are one kick of a dt.
 // It takes ~45 of the ~85 FP64-pipe instructions per particle and 128 of the
 // 484 bytes (the residuals' read and three writes) off this kernel.
+// (Called by a whole grid, each thread for its items of the span; returns
+// whether one of the thread's particles asks for a rebuild.)
 template <bool KAHAN>
-__global__ void __launch_bounds__(256) k_first_half(StepParams P) {
-  Ctrl* C = P.ctrl;
-  if (C->halt) return;
-  const bool FUSE = C->pending != 0;
-  const Bank B = P.bank[C->bank];
+__device__ __forceinline__ bool first_half_pass(const StepParams& P, Ctrl* C, const Bank& B, bool FUSE, Span sp) {
   const double dt = P.dt;
   const bool anyp = P.periodic[0] | P.periodic[1] | P.periodic[2];
   const float half_skin = (float)(0.5 * P.skin);
@@ -803,7 +810,7 @@ __global__ void __launch_bounds__(256) k_first_half(StepParams P) {
   const float inv_hf = (float)P.inv_href;
   const unsigned xmax = C->xmax;
   bool want_rebuild = false;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < P.n; k += gridDim.x * blockDim.x) {
+  for (int k = sp.at; k < P.n; k += sp.all) {
     uint32_t fl = B.flags[k];
     if (fl & PF_DEAD) continue;
     D4 xr = B.xr[k], vm = B.vm[k], wc = B.wc[k];
@@ -907,7 +914,14 @@ __global__ void __launch_bounds__(256) k_first_half(StepParams P) {
     float d2 = ddx * ddx + ddy * ddy + ddz * ddz;
     if (!(d2 <= half_skin * half_skin)) want_rebuild = true;  // NaN (no build yet) also rebuilds
   }
-  if (want_rebuild) C->rebuild = 1;
+  return want_rebuild;
+}
+
+template <bool KAHAN>
+__global__ void __launch_bounds__(KAHAN ? 128 : 256, KAHAN ? 5 : 4) k_first_half(StepParams P) {
+  Ctrl* C = P.ctrl;
+  if (C->halt) return;
+  if (first_half_pass<KAHAN>(P, C, P.bank[C->bank], C->pending != 0, grid_span())) C->rebuild = 1;
 }
 
 // Completes the last step of a stepping call (the pending second half);
@@ -961,16 +975,17 @@ __device__ __forceinline__ bool tri_cell_range(const StepParams& P, float4 xf, u
 }
 
 // FP32 pretest of a sphere (centre xf, radius rf = xf.w, largest |coordinate|
-// xmag, group gi) against a triangle: false when it cannot touch it.
-__device__ __forceinline__ bool wall_pretest(const TriRec& tr, uint32_t gi, float4 xf, float xmag) {
-  if (tr.group != GROUP_ALL && tr.group != gi) return false;
-  const float rf = xf.w;
+// xmag, group gi) against a triangle: false when it cannot touch it. First its
+// plane (hd: the distance, mrg: its rounding margin), then its edges.
+__device__ __forceinline__ bool wall_plane(const TriRec& tr, uint32_t gi, float4 xf, float xmag, float& hd, float& mrg) {
   // FP32 rounding of n, n.v0 and x moves n.x - n.v0 by at most
   // ~3e-7 (|x| + |n.v0|) + 1.1e-7 |x - v0|; the margin is larger
   const float4 pl = tr.plane;
-  const float hd = fabsf(pl.x * xf.x + pl.y * xf.y + pl.z * xf.z - pl.w);
-  const float mrg = 1e-6f * (1.0f + xmag + fabsf(pl.w) + rf) + 2e-7f * (xmag + tr.bound.x);
-  if (hd > rf + mrg) return false;
+  hd = fabsf(pl.x * xf.x + pl.y * xf.y + pl.z * xf.z - pl.w);
+  mrg = 1e-6f * (1.0f + xmag + fabsf(pl.w) + xf.w) + 2e-7f * (xmag + tr.bound.x);
+  return (tr.group == GROUP_ALL || tr.group == gi) && !(hd > xf.w + mrg);
+}
+__device__ __forceinline__ bool wall_edges(const TriRec& tr, float4 xf, float hd, float mrg) {
   // the distance to the triangle is at least sqrt(hd^2 + s^2), s the
   // largest outward in-plane distance to an edge line (each with the
   // plane test's rounding margin; |m.v| <= sqrt(3) bound)
@@ -980,7 +995,27 @@ __device__ __forceinline__ bool wall_pretest(const TriRec& tr, uint32_t gi, floa
                         g2.x * xf.x + g2.y * xf.y + g2.z * xf.z - g2.w);
   const float me = mrg + 4e-7f * tr.bound.x;
   const float hl = fmaxf(hd - mrg, 0.0f), sl = fmaxf(s - me, 0.0f);
-  return !(hl * hl + sl * sl > rf * rf * (1.0f + 1e-6f));
+  return !(hl * hl + sl * sl > xf.w * xf.w * (1.0f + 1e-6f));
+}
+__device__ __forceinline__ bool wall_pretest(const TriRec& tr, uint32_t gi, float4 xf, float xmag) {
+  float hd, mrg;
+  return wall_plane(tr, gi, xf, xmag, hd, mrg) && wall_edges(tr, xf, hd, mrg);
+}
+// The entries t .. t + 3 of a triangle-grid cell (those below te) that pass, as
+// bits; the four triangles' planes are loaded together.
+__device__ __forceinline__ uint32_t wall_pretest4(const StepParams& P, uint32_t t, uint32_t te, uint32_t gi, float4 xf,
+                                                  float xmag) {
+  uint32_t id[4], pass = 0u;
+  float hd[4], mrg[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) id[q] = P.titems[min(t + q, te - 1u)];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (wall_plane(P.tri[id[q]], gi, xf, xmag, hd[q], mrg[q]) && t + q < te) pass |= 1u << q;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if ((pass >> q & 1u) && !wall_edges(P.tri[id[q]], xf, hd[q], mrg[q])) pass &= ~(1u << q);
+  return pass;
 }
 
 // The FP64 contact of a sphere with a triangle that passed the pretest:
@@ -1338,11 +1373,14 @@ constexpr int CTOT_WORDS = 8;
 // neighbourhood lies in one reference cell (PF_ONECELL). One entry at a time
 // with the visit counts in between, the pass took 155 us on 1,048,576 spheres
 // (hopper, rows of 11) and 329 us on 2,097,152 adhesive ones; this form takes 122 and 176 us.
-template <bool PHYS, bool HIST>
-__global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
-  Ctrl* C = P.ctrl;
-  if (C->halt) return;
-  const Bank B = P.bank[C->bank];
+// COHERENT: the positions were written by the same kernel launch, so they are
+// not read through the read-only path; slots are taken in order.
+template <bool COHERENT>
+__device__ __forceinline__ float4 load_xf(const float4* p) {
+  return COHERENT ? *p : __ldg(p);
+}
+template <bool PHYS, bool HIST, bool COHERENT>
+__device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const Bank& B, uint32_t* ctot, Span sp) {
   const bool learn_any = P.jkr_solver == 1 && P.nmodel == 3 && P.mlp != nullptr;
   const bool hint_any = P.jfb != nullptr;  // a certified JKR solver
   // JKR pairs certified to have no force add exactly +-0 to F and T (the
@@ -1359,11 +1397,12 @@ __global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
   const int lane = threadIdx.x & 31;
   // slots in the rebuild-time order (tiles of 256 sorted by list length), so
   // a warp's lanes walk lists of similar length
-  for (int i0 = blockIdx.x * blockDim.x; i0 < P.n; i0 += gridDim.x * blockDim.x) {
-    const int i = i0 + (int)threadIdx.x;
-    const int k = i < P.n ? (int)P.aorder[i] : -1;
+  for (int i0 = sp.at - lane; i0 < P.n; i0 += sp.all) {
+    const int i = i0 + lane;
+    const int k = i < P.n ? (COHERENT ? i : (int)P.aorder[i]) : -1;
     uint32_t nrec = 0, ncmp = 0, nnet = 0, nhard = 0, nw = 0, ts = 0, te = 0, gi = 0;
     uint32_t evals = 0u;  // records (the first 32) that evaluate their pair
+    uint32_t wmask = 0u;  // entries of its triangle-grid cell (the first 32) that pass
     float4 xif = make_float4(0.f, 0.f, 0.f, 0.f);
     float Xi = 0.f;
     const uint32_t flk = k >= 0 ? B.flags[k] : PF_DEAD;
@@ -1377,6 +1416,15 @@ __global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
       const uint32_t cnt = B.ncnt[k];
       const uint32_t* row = B.nbr + (size_t)k * P.cap;
       CRec* out = P.crec + (size_t)k * P.cap;
+      const bool wide = (P.cap & 3) == 0;  // rows on 16 bytes
+      // where latency is all that counts, the first eight entries come with the
+      // particle itself (a dilute bed of a million would read rows it does not have)
+      uint4 head0 = make_uint4(0u, 0u, 0u, 0u), head1 = head0;
+      if (COHERENT && wide) {
+        head0 = __ldg(reinterpret_cast<const uint4*>(row));
+        if (P.cap > 4) head1 = __ldg(reinterpret_cast<const uint4*>(row) + 1);
+      }
+      const bool walled = P.ntri > 0 && !(P.wall_far_ok && (flk & PF_WALLFAR)) && tri_cell_range(P, xif, ts, te);
       for (uint32_t c0 = 0; c0 < cnt; c0 += 32) {
         const uint32_t ce = min(cnt - c0, 32u);
         const uint32_t valid = 0xFFFFFFFFu >> (32u - ce);
@@ -1384,8 +1432,9 @@ __global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
         if (P.pretest) {
           for (uint32_t m = 0; m < ce; m += 4) {
             uint4 j;
-            if ((P.cap & 3) == 0) {  // rows start on 16 bytes; entries past the end are not followed
-              j = __ldg(reinterpret_cast<const uint4*>(row + c0 + m));
+            if (wide) {  // entries past the end are not followed
+              if (COHERENT && c0 + m < 8) j = c0 + m == 0 ? head0 : head1;
+              else j = __ldg(reinterpret_cast<const uint4*>(row + c0 + m));
               if (m + 1 >= ce) j.y = j.x;
               if (m + 2 >= ce) j.z = j.x;
               if (m + 3 >= ce) j.w = j.x;
@@ -1395,7 +1444,8 @@ __global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
               j.z = m + 2 < ce ? __ldg(row + c0 + m + 2) : j.x;
               j.w = m + 3 < ce ? __ldg(row + c0 + m + 3) : j.x;
             }
-            const float4 x0 = __ldg(B.xf + j.x), x1 = __ldg(B.xf + j.y), x2 = __ldg(B.xf + j.z), x3 = __ldg(B.xf + j.w);
+            const float4 x0 = load_xf<COHERENT>(B.xf + j.x), x1 = load_xf<COHERENT>(B.xf + j.y),
+                         x2 = load_xf<COHERENT>(B.xf + j.z), x3 = load_xf<COHERENT>(B.xf + j.w);
             const uint32_t q = (pretest_near(P, xif, x0, image, margin) ? 1u : 0u) |
                                (pretest_near(P, xif, x1, image, margin) ? 2u : 0u) |
                                (pretest_near(P, xif, x2, image, margin) ? 4u : 0u) |
@@ -1413,7 +1463,7 @@ __global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
           uint32_t hint = 0u;
           if (P.nmodel >= 3) {  // pairs never cross groups (the lists exclude them)
             const Law lw = law_of(P, B, k);
-            const float4 xjf = __ldg(B.xf + j);
+            const float4 xjf = load_xf<COHERENT>(B.xf + j);
             Xi = fmaxf(fmaxf(fabsf(xif.x), fabsf(xif.y)), fabsf(xif.z));
             const bool adhesive = lw.gamma_pp > 0.0;
             if (zdrop_any && adhesive && jkr_far_zero(P, lw.jkr_Cf, xif, Xi, xjf)) continue;
@@ -1464,10 +1514,14 @@ __global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
       }
       // wall candidates: the triangles of its triangle-grid cell that pass
       // the FP32 pretest, counted here and listed once the arena is reserved
-      if (P.ntri > 0 && !(P.wall_far_ok && (flk & PF_WALLFAR)) && tri_cell_range(P, xif, ts, te)) {
+      if (walled) {
         Xi = fmaxf(fmaxf(fabsf(xif.x), fabsf(xif.y)), fabsf(xif.z));
         gi = P.ngroups > 1 ? B.grp[k] : 0u;
-        for (uint32_t t = ts; t < te; ++t) nw += wall_pretest(P.tri[P.titems[t]], gi, xif, Xi) ? 1u : 0u;
+        for (uint32_t t = ts; t < te; t += 4) {
+          const uint32_t pass = wall_pretest4(P, t, te, gi, xif, Xi);
+          nw += (uint32_t)__popc(pass);
+          if (t - ts < 32u) wmask |= pass << (t - ts);
+        }
       }
     }
     __syncwarp();
@@ -1490,7 +1544,7 @@ __global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
     if (__any_sync(0xFFFFFFFFu, nw != 0)) wb = warp_exclusive(nw, tw);
     const uint32_t add = lane == 0 ? tr : lane == 1 ? tc : lane == 2 ? tn : lane == 4 ? tw : lane == 5 ? th : 0u;
     uint32_t at = 0;
-    if (add) at = atomicAdd(P.ctot + lane, add);
+    if (add) at = atomicAdd(ctot + lane, add);
     rb += __shfl_sync(0xFFFFFFFFu, at, 0);
     q += __shfl_sync(0xFFFFFFFFu, at, 1);
     if (learn_any) qn += __shfl_sync(0xFFFFFFFFu, at, 2);
@@ -1503,7 +1557,9 @@ __global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
       if (nw > 0 && wb + nw <= P.wcap) {  // in mesh order, as the reference visits them
         uint2* dst = P.warena + wb;
         uint32_t c = 0;
-        for (uint32_t t = ts; t < te && c < nw; ++t) {
+        for (uint32_t left = wmask; left; left &= left - 1u)
+          dst[c++] = make_uint2((uint32_t)k, P.titems[ts + (uint32_t)__ffs((int)left) - 1u]);
+        for (uint32_t t = ts + 32u; t < te && c < nw; ++t) {
           const uint32_t id = P.titems[t];
           if (wall_pretest(P.tri[id], gi, xif, Xi)) dst[c++] = make_uint2((uint32_t)k, id);
         }
@@ -1515,27 +1571,37 @@ __global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
       P.woff[k] = wb;
     }
     if (ncmp + nhard == 0) continue;
-    // the evaluating records into the compact list
-    const size_t base = (size_t)k * P.cap;
+    // the evaluating records into the compact list, read back from the row that
+    // this thread just wrote
+    const CRec* out = P.crec + (size_t)k * P.cap;
     if (nrec <= 32 && !hint_any) {
-      for (uint32_t left = evals; left; left &= left - 1u)
-        P.clist[q++] = (uint32_t)(base + (uint32_t)__ffs((int)left) - 1u);
+      for (uint32_t left = evals; left; left &= left - 1u) {
+        const uint32_t c = (uint32_t)__ffs((int)left) - 1u;
+        const CRec r = out[c];
+        P.clist[q++] = make_uint4((uint32_t)k, r.j, r.mv, rb + c);
+      }
       continue;
     }
-    // read back from the row this thread just wrote: long rows, and the
-    // queues of the certified JKR solvers
-    const CRec* out = P.crec + base;
+    // long rows, and the queues of the certified JKR solvers
     for (uint32_t c = 0; c < nrec; ++c) {
       const CRec r = out[c];
       if (crec_vji(r.mv) > 0 && (uint32_t)k > r.j) continue;
+      const uint4 it = make_uint4((uint32_t)k, r.j, r.mv, rb + c);
       if (r.mv & CREC_HARD) {
-        P.jhard[qh++] = (uint32_t)(base + c);
+        P.jhard[qh++] = it;
         continue;
       }
-      if (r.mv & CREC_NET) P.jq[qn++] = make_uint2(q, (uint32_t)(base + c));
-      P.clist[q++] = (uint32_t)(base + c);
+      if (r.mv & CREC_NET) P.jq[qn++] = q;
+      P.clist[q++] = it;
     }
   }
+}
+
+template <bool PHYS, bool HIST>
+__global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
+  Ctrl* C = P.ctrl;
+  if (C->halt) return;
+  filter_pass<PHYS, HIST, false>(P, C, P.bank[C->bank], P.ctot, grid_span());
 }
 
 // Pass 2b: the JKR network over the queue, 32 pairs per warp on the tensor
@@ -1562,11 +1628,9 @@ __global__ void __launch_bounds__(128) k_jkr_mlp(StepParams P) {
     bool ok = false;
     uint32_t q = 0;
     if (valid) {
-      const uint2 it = P.jq[idx];
-      q = it.x;
-      const uint32_t s = it.y;
-      const uint32_t k = s / (uint32_t)P.cap;
-      const uint32_t j = P.crec[s].j;
+      q = P.jq[idx];
+      const uint4 it = P.clist[q];
+      const uint32_t k = it.x, j = it.y;
       const D4 xi4 = B.xr[k], xj4 = B.xr[j];
       const V d = mic(P, xyz(xi4) - xyz(xj4));
       const double d2 = dot(d, d);
@@ -1633,18 +1697,45 @@ __device__ __forceinline__ void put_result(const StepParams& P, uint32_t rec, T3
   }
 }
 
+// The record of row j whose partner is k (its place among the row's records),
+// NO_RECORD when the row has none; four records at a time where rows allow it,
+// the first four without waiting for the row's count.
+constexpr uint32_t NO_RECORD = 0xFFFFFFFFu;
+__device__ __forceinline__ uint32_t back_record(const StepParams& P, uint32_t j, uint32_t k) {
+  const CRec* row = P.crec + (size_t)j * P.cap;
+  if ((P.cap & 3) == 0) {
+    const uint4* two = reinterpret_cast<const uint4*>(row);
+    uint4 a = two[0], b = two[1];
+    const uint32_t n = P.ccnt[j];
+    for (uint32_t c = 0; c < n;) {
+      const uint32_t at = a.x == k ? 0u : a.z == k ? 1u : b.x == k ? 2u : b.z == k ? 3u : 4u;
+      if (at < 4u && c + at < n) return c + at;
+      c += 4;
+      if (c < n) { a = two[c / 2]; b = two[c / 2 + 1]; }
+    }
+  } else {
+    const uint32_t n = P.ccnt[j];
+    for (uint32_t c = 0; c < n; ++c)
+      if (row[c].j == k) return c;
+  }
+  return NO_RECORD;
+}
+
 template <bool PHYS, bool HIST, typename R, bool JKR>
-__device__ __forceinline__ bool contact_eval(const StepParams& P, const Bank& B, uint32_t s, float guess,
+__device__ __forceinline__ bool contact_eval(const StepParams& P, const Bank& B, uint4 it, float guess,
                                              bool can_defer, bool newton, bool& excess, uint32_t* tally) {
   const size_t plane = (size_t)P.n * P.cap;
   const bool adh = (P.nmodel == 3 || P.nmodel == 4);
-  const uint32_t k = s / (uint32_t)P.cap, c = s - k * (uint32_t)P.cap;
-  const CRec r = P.crec[s];
-  const uint32_t j = r.j, m = r.mv & 0xFFFFu;
-  const int vij = (r.mv >> 16) & 0xFF, vji = crec_vji(r.mv);
-  if (!(r.mv & CREC_NET)) guess = -1.0f;
+  const uint32_t k = it.x, j = it.y, m = it.z & 0xFFFFu;
+  const int vij = (it.z >> 16) & 0xFF, vji = crec_vji(it.z);
+  if (!(it.z & CREC_NET)) guess = -1.0f;
   else if (tally) tally[3] += 1;
+  // everything the pair needs is asked for at once: the chain of a pair is
+  // latency (list, both ends and the other's records), then FP64
   const D4 xi4 = B.xr[k], xj4 = B.xr[j];
+  const D4 vi4 = B.vm[k], wi4 = B.wc[k], vj4 = B.vm[j], wj4 = B.wc[j];
+  const uint32_t offj = P.coff[j];
+  const uint32_t back = vji > 0 ? back_record(P, j, k) : NO_RECORD;
   const V d = mic(P, xyz(xi4) - xyz(xj4));
   const double d2 = dot(d, d);
   const double rsum = xi4.w + xj4.w;
@@ -1654,7 +1745,6 @@ __device__ __forceinline__ bool contact_eval(const StepParams& P, const Bank& B,
   double* hk = HIST ? B.hist + hik : nullptr;
   T3<R> fc = t3(R(0), R(0), R(0)), tc = fc, tc2 = fc, nrm = fc;  // tc2: the torque on the other end
   if (in) {
-    const D4 vi4 = B.vm[k], wi4 = B.wc[k], vj4 = B.vm[j], wj4 = B.wc[j];
     const Law lw = law_of(P, B, (int)k);
     bool deferred = false;
     if constexpr (PHYS && sizeof(R) == sizeof(double)) {
@@ -1693,23 +1783,19 @@ __device__ __forceinline__ bool contact_eval(const StepParams& P, const Bank& B,
     hk[2 * plane] = 0.0;
   }
   if (P.debug) P.dbgMult[hik] = (uint8_t)(in ? vij : 0);
-  put_result(P, P.coff[k] + c, fc, tc, vij);
-  if (vji > 0) {
-    const uint32_t nj = P.ccnt[j];
-    const CRec* rj = P.crec + (size_t)j * P.cap;
-    for (uint32_t c2 = 0; c2 < nj; ++c2) {
-      if (rj[c2].j != k) continue;
-      put_result(P, P.coff[j] + c2, -fc, tc2, vji);
-      const size_t h2 = (size_t)j * P.cap + (rj[c2].mv & 0xFFFFu);
+  put_result(P, it.w, fc, tc, vij);
+  if (back != NO_RECORD) {
+    put_result(P, offj + back, -fc, tc2, vji);
+    if (HIST || P.debug) {
+      const uint32_t m2 = P.crec[(size_t)j * P.cap + back].mv & 0xFFFFu;
+      const size_t h2 = (size_t)j * P.cap + m2;
       if (HIST) {
         B.hist[h2] = -hk[0];
         B.hist[plane + h2] = -hk[plane];
         B.hist[2 * plane + h2] = -hk[2 * plane];
-        const uint32_t m2 = rj[c2].mv & 0xFFFFu;
         if (m2 < 64) atomicOr(B.hmask + j, 1ull << m2);
       }
       if (P.debug) P.dbgMult[h2] = (uint8_t)(in ? vji : 0);
-      break;
     }
   }
   return false;
@@ -1748,25 +1834,22 @@ __device__ __forceinline__ void add_tally(Ctrl* C, const uint32_t tally[6]) {
 // Pass 3: one thread per evaluating record, then one per wall candidate (the
 // few wall contacts spread over the whole grid with the pairs).
 template <bool PHYS, bool HIST, typename R, bool JKR>
-__global__ void __launch_bounds__(256) k_contact_force(StepParams P) {
-  Ctrl* C = P.ctrl;
-  if (C->halt) return;
-  const Bank B = P.bank[C->bank];
-  const uint32_t total = P.ctot[1];
-  const uint32_t items = total + (P.ntri > 0 ? min(P.ctot[4], P.wcap) : 0u);
+__device__ __forceinline__ void contact_pass(const StepParams& P, Ctrl* C, const Bank& B, uint32_t* ctot, Span sp) {
+  const uint32_t total = ctot[1];
+  // the walls start on a warp of their own (a mixed one runs both laws)
+  const uint32_t walls = (total + 31u) & ~31u;
+  const uint32_t items = P.ntri > 0 ? walls + min(ctot[4], P.wcap) : total;
   bool excess = false;
   uint32_t tally[6] = {0u, 0u, 0u, 0u, 0u, 0u};
   const int lane = threadIdx.x & 31;
   const bool learn = P.jkr_solver == 1 && P.nmodel == 3 && P.mlp != nullptr;
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < items; t += gridDim.x * blockDim.x) {
+  for (uint32_t t = (uint32_t)sp.at; t < items; t += (uint32_t)sp.all) {
     bool deferred = false;
-    uint32_t s = 0;
     if (t < total) {
-      s = P.clist[t];
-      deferred = contact_eval<PHYS, HIST, R, JKR>(P, B, s, JKR && learn ? P.jguess[t] : -1.0f, JKR && P.jfb != nullptr,
+      deferred = contact_eval<PHYS, HIST, R, JKR>(P, B, P.clist[t], JKR && learn ? P.jguess[t] : -1.0f, JKR && P.jfb != nullptr,
                                                   false, excess, JKR ? tally : nullptr);
-    } else {
-      wall_eval<JKR>(P, B, t - total, excess);
+    } else if (t >= walls) {
+      wall_eval<JKR>(P, B, t - walls, excess);
     }
     if (!JKR) continue;
     // append the deferred pairs with one atomic per warp
@@ -1775,13 +1858,20 @@ __global__ void __launch_bounds__(256) k_contact_force(StepParams P) {
     if (bal) {
       const int leader = __ffs(bal) - 1;
       uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(P.ctot + 3, (uint32_t)__popc(bal));
+      if (lane == leader) base = atomicAdd(ctot + 3, (uint32_t)__popc(bal));
       base = __shfl_sync(act, base, leader);
-      if (deferred) P.jfb[base + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = s;
+      if (deferred) P.jfb[base + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = t;
     }
   }
   if (excess) C->overlap_flag = 1;
   if (JKR && P.jkr_solver != 0) add_tally(C, tally);
+}
+
+template <bool PHYS, bool HIST, typename R, bool JKR>
+__global__ void __launch_bounds__(256) k_contact_force(StepParams P) {
+  Ctrl* C = P.ctrl;
+  if (C->halt) return;
+  contact_pass<PHYS, HIST, R, JKR>(P, C, P.bank[C->bank], P.ctot, grid_span());
 }
 
 // The pairs that the filter found next to the JKR fold, one thread each: the
@@ -1800,10 +1890,10 @@ __global__ void __launch_bounds__(128) k_contact_hard(StepParams P) {
   bool excess = false;
   uint32_t tally[6] = {0u, 0u, 0u, 0u, 0u, 0u};
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-    const uint32_t s = P.jhard[i];
+    const uint4 it = P.jhard[i];
     constexpr bool f32 = sizeof(R) == sizeof(float);
-    const bool deferred = contact_eval<PHYS, HIST, R, true>(P, B, s, -1.0f, f32, false, excess, tally);
-    if (f32 && deferred) contact_eval<PHYS, HIST, double, true>(P, B, s, -1.0f, false, true, excess, nullptr);
+    const bool deferred = contact_eval<PHYS, HIST, R, true>(P, B, it, -1.0f, f32, false, excess, tally);
+    if (f32 && deferred) contact_eval<PHYS, HIST, double, true>(P, B, it, -1.0f, false, true, excess, nullptr);
   }
   if (excess) C->overlap_flag = 1;
   add_tally(C, tally);
@@ -1820,7 +1910,7 @@ __global__ void __launch_bounds__(128) k_contact_deferred(StepParams P) {
   const uint32_t total = P.ctot[3];
   bool excess = false;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
-    contact_eval<PHYS, HIST, double, true>(P, B, P.jfb[i], -1.0f, false, true, excess, nullptr);
+    contact_eval<PHYS, HIST, double, true>(P, B, P.clist[P.jfb[i]], -1.0f, false, true, excess, nullptr);
   if (excess) C->overlap_flag = 1;
 }
 
@@ -2000,12 +2090,57 @@ __device__ __forceinline__ void finish_particle(const StepParams& P, const Bank&
   B.tq[k] = D4{plus_zero(T.x), plus_zero(T.y), plus_zero(T.z), 0.0};
 }
 
-// Threads take the slots in the order aorder gives (tiles of 256 sorted by
-// list length, particles in triangle cells last). The contact results are
-// FP64 records (the FP64 form) or FP32 records (the mixed form, whose pair
-// forces are FP32 values); either way the sums are FP64, in list order.
+// One particle's contact results: FP64 records (the FP64 form) or FP32 records
+// (the mixed form, whose pair forces are FP32 values), in list order, then its
+// wall results in mesh order.
 template <bool F32REC>
-__global__ void __launch_bounds__(256) k_accumulate(StepParams P) {
+__device__ __forceinline__ void sum_particle(const StepParams& P, const Bank& B, Ctrl* C, int k) {
+  V F = vmk(0.0, 0.0, 0.0), T = vmk(0.0, 0.0, 0.0);
+  const uint32_t n = P.ccnt[k];
+  if (F32REC) {
+    // the mixed form's FP32 pair forces summed in FP32 (in list order, from
+    // zero; the rounding adds at most (n - 1) 2^-24 of the sum of the
+    // magnitudes), then widened exactly
+    const float2* res = reinterpret_cast<const float2*>(P.cresf + 6 * (size_t)P.coff[k]);
+    float fx = 0.0f, fy = 0.0f, fz = 0.0f, tx = 0.0f, ty = 0.0f, tz = 0.0f;
+    for (uint32_t c = 0; c < n; ++c) {
+      const float2 r0 = res[3 * c], r1 = res[3 * c + 1], r2 = res[3 * c + 2];
+      fx = fx + r0.x; fy = fy + r0.y; fz = fz + r1.x;
+      tx = tx + r1.y; ty = ty + r2.x; tz = tz + r2.y;
+    }
+    F = vmk(f2d_exact(fx), f2d_exact(fy), f2d_exact(fz));
+    T = vmk(f2d_exact(tx), f2d_exact(ty), f2d_exact(tz));
+  } else {
+    // the next record's loads are in flight while this one is added
+    const double2* res = reinterpret_cast<const double2*>(P.cres + 6 * (size_t)P.coff[k]);
+    double2 a0, a1, a2;
+    if (n > 0) { a0 = res[0]; a1 = res[1]; a2 = res[2]; }
+    for (uint32_t c = 0; c < n; ++c) {
+      const double2 r0 = a0, r1 = a1, r2 = a2;
+      if (c + 1 < n) { a0 = res[3 * c + 3]; a1 = res[3 * c + 4]; a2 = res[3 * c + 5]; }
+      F = F + vmk(r0.x, r0.y, r1.x);
+      T = T + vmk(r1.y, r2.x, r2.y);
+    }
+  }
+  // the wall contacts (FP64 in both forms) after the pair contacts, in mesh order
+  if (P.ntri > 0) {
+    const uint32_t wn = P.wcnt[k], wo = P.woff[k];
+    for (uint32_t c = 0; c < wn; ++c) {
+      const double2* r = reinterpret_cast<const double2*>(P.wres + 6 * (size_t)(wo + c));
+      const bool ok = P.wok[wo + c] != 0;
+      const double2 r0 = r[0], r1 = r[1], r2 = r[2];
+      if (!ok) continue;
+      F = F + vmk(r0.x, r0.y, r1.x);
+      T = T + vmk(r1.y, r2.x, r2.y);
+    }
+  }
+  finish_particle(P, B, C, k, F, T);
+}
+
+// Threads take the slots in the order aorder gives (tiles of 256 sorted by
+// list length, particles in triangle cells last).
+template <bool F32REC>
+__global__ void __launch_bounds__(256, 5) k_accumulate(StepParams P) {
   Ctrl* C = P.ctrl;
   if (C->halt) return;
   const Bank B = P.bank[C->bank];
@@ -2044,42 +2179,338 @@ __global__ void __launch_bounds__(256) k_accumulate(StepParams P) {
     k = dealt[threadIdx.x];
     __syncthreads();
     if (k < 0) continue;
-    V F = vmk(0.0, 0.0, 0.0), T = vmk(0.0, 0.0, 0.0);
-    const uint32_t n = P.ccnt[k];
-    if (F32REC) {
-      // the mixed form's FP32 pair forces summed in FP32 (in list order, from
-      // zero; the rounding adds at most (n - 1) 2^-24 of the sum of the
-      // magnitudes), then widened exactly
-      const float2* res = reinterpret_cast<const float2*>(P.cresf + 6 * (size_t)P.coff[k]);
-      float fx = 0.0f, fy = 0.0f, fz = 0.0f, tx = 0.0f, ty = 0.0f, tz = 0.0f;
-      for (uint32_t c = 0; c < n; ++c) {
-        const float2 r0 = res[3 * c], r1 = res[3 * c + 1], r2 = res[3 * c + 2];
-        fx = fx + r0.x; fy = fy + r0.y; fz = fz + r1.x;
-        tx = tx + r1.y; ty = ty + r2.x; tz = tz + r2.y;
-      }
-      F = vmk(f2d_exact(fx), f2d_exact(fy), f2d_exact(fz));
-      T = vmk(f2d_exact(tx), f2d_exact(ty), f2d_exact(tz));
-    } else {
-      const double2* res = reinterpret_cast<const double2*>(P.cres + 6 * (size_t)P.coff[k]);
-      for (uint32_t c = 0; c < n; ++c) {
-        const double2 r0 = res[3 * c], r1 = res[3 * c + 1], r2 = res[3 * c + 2];
-        F = F + vmk(r0.x, r0.y, r1.x);
-        T = T + vmk(r1.y, r2.x, r2.y);
-      }
-    }
-    // the wall contacts (FP64 in both forms) after the pair contacts, in mesh order
-    if (P.ntri > 0) {
-      const uint32_t wn = P.wcnt[k], wo = P.woff[k];
-      for (uint32_t c = 0; c < wn; ++c) {
-        if (!P.wok[wo + c]) continue;
-        const double2* r = reinterpret_cast<const double2*>(P.wres + 6 * (size_t)(wo + c));
-        const double2 r0 = r[0], r1 = r[1], r2 = r[2];
-        F = F + vmk(r0.x, r0.y, r1.x);
-        T = T + vmk(r1.y, r2.x, r2.y);
-      }
-    }
-    finish_particle(P, B, C, k, F, T);
+    sum_particle<F32REC>(P, B, C, k);
   }
+}
+
+// ------------------------------------------------------ many steps, one launch
+// A small bed's step is a chain of dependent latencies, not work: eight graph
+// nodes of 1,000 spheres take 53 us a step, with one warp in each FP64 unit at
+// most. k_steps runs the step's passes in one cooperative launch, three grid
+// barriers apart, step after step, until the target is reached, the lists must
+// be rebuilt (the graph runs the chain and launches it again; Ctrl::resume says
+// that the first half of the current step has been done) or a buffer is full.
+// The sums of a step and the first half of the next are one quad's, so no
+// barrier lies between them: 1,000 spheres take 26 us a step.
+// The launch fits the device at once (cooperative); every wait is bounded, and
+// one that runs out halts the simulation with an error.
+constexpr unsigned SMALL_SPINS = 1u << 20;      // ~1 s
+constexpr unsigned SMALL_STEPS = 4096;          // steps a launch
+constexpr int SMALL_BLOCK = 512;                // threads a block at most, one block a multiprocessor
+// Particles taken by four lanes each: below one quad warp for every other FP64
+// unit (608 x 8 particles) the integrator is a quarter as long, at 16,000 the
+// extra loads cost what it saves (us a step with quads / without: 1,000 spheres
+// 26.2 / 30.3, 8,000 32.7 / 32.2, 16,000 49.1 / 43.7, one item order for both).
+constexpr int QUAD_MAX = 8192;
+// Particles: up to here a launch of many steps is the faster loop on every bed
+// measured (us a step, this / eight graph nodes: Hertz + Coulomb FP64 box 1,000
+// 26 / 48, 24,000 32.5 / 55, 100,000 78 / 98, 250,000 171 / 179, 400,000 264 /
+// 256; mixed bed 250,000 167 / 183, 800,000 482 / 462; linear springs 250,000
+// 303 / 314, 800,000 891 / 873). Above, a kernel for each pass holds fewer
+// registers and more warps.
+constexpr int SMALL_MAX = 262144;
+
+__device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// All blocks of the launch; `gen` counts the barriers passed. False when the
+// others did not arrive in time.
+__device__ __forceinline__ bool grid_barrier(Ctrl* C, unsigned& gen) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ++gen;
+    const unsigned want = gen * gridDim.x;
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&C->bar), "r"(1u) : "memory");
+    bool here = load_acquire(&C->bar) >= want;
+    for (unsigned n = 0; !here && n < SMALL_SPINS; ++n) here = load_acquire(&C->bar) >= want;
+    if (!here) {
+      atomicOr(&C->halt, HALT_STUCK);
+      atomicOr(&C->status, (unsigned)ST_STUCK);
+    }
+    ok = here;
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+// first_half_pass and sum_particle with four lanes a particle: lane c < 3 holds
+// component c of every vector, lane 3 the fourth words (mass, radius, cell code,
+// 1/m, 1/I). A warp instruction takes the FP64 unit of a partition 66 clocks
+// whatever its lanes do, so with less than a warp for each unit the integrator's
+// ~90 FP64 instructions become ~28 and a record's sum two instead of six. The
+// operations of each component and their order are those of the scalar passes.
+__device__ __forceinline__ double quad_word(double v, int word) { return __shfl_sync(0xFFFFFFFFu, v, word, 4); }
+__device__ __forceinline__ float quad_word(float v, int word) { return __shfl_sync(0xFFFFFFFFu, v, word, 4); }
+__device__ __forceinline__ unsigned quad_mask() { return 7u << (threadIdx.x & 28); }  // the three components' lanes
+__device__ __forceinline__ bool nonzero_bits(double x) { return (__double_as_longlong(x) << 1) != 0; }
+__device__ __forceinline__ void kahan_add(double& s, double& r, double d) {
+  const double y = d - r;
+  const double t = s + y;
+  r = (t - s) - y;
+  s = t;
+}
+template <typename A>
+__device__ __forceinline__ A pick(int c, const A* v) {  // v[c] without an indexed parameter read; 0 for lane 3
+  return c == 0 ? v[0] : c == 1 ? v[1] : c == 2 ? v[2] : A(0);
+}
+
+// The first half of the warp's particles k (one a quad; on: it exists), whole
+// warps only; returns whether the particle asks for a rebuild.
+template <bool KAHAN>
+__device__ __forceinline__ bool first_half_quad(const StepParams& P, Ctrl* C, const Bank& B, bool fuse, int k, bool on) {
+  constexpr unsigned ALL = 0xFFFFFFFFu;
+  const int c = threadIdx.x & 3;
+  const bool part = c < 3;
+  const size_t at = 4 * (size_t)k + c;
+  uint32_t fl = on ? B.flags[k] : PF_DEAD;
+  on = !(fl & PF_DEAD);
+  const bool moving = on && !(fl & PF_FIXED);
+  double x = 0.0, v = 0.0, w = 0.0, a = 0.0, tau = 0.0, vres = 0.0, wres = 0.0, xres = 0.0;
+  float xo = 0.0f, ref = 0.0f;
+  if (on) {
+    x = reinterpret_cast<const double*>(B.xr)[at];
+    v = reinterpret_cast<const double*>(B.vm)[at];
+    w = reinterpret_cast<const double*>(B.wc)[at];
+    xo = reinterpret_cast<const float*>(B.xf)[at];
+    ref = reinterpret_cast<const float*>(B.xref)[at];
+    if (moving) {
+      a = reinterpret_cast<const double*>(B.acc)[at];
+      tau = reinterpret_cast<const double*>(B.tq)[at];
+      wres = reinterpret_cast<const double*>(B.wres)[at];
+      if (KAHAN) {
+        vres = reinterpret_cast<const double*>(B.vres)[at];
+        xres = reinterpret_cast<const double*>(B.xres)[at];
+      }
+    }
+  }
+  const double dt = P.dt, hdt = 0.5 * dt, inv_inertia = quad_word(wres, 3);
+  const unsigned spinning = __ballot_sync(ALL, moving && (nonzero_bits(tau) || (KAHAN && nonzero_bits(wres))));
+  const bool own_spin = (spinning & quad_mask()) != 0;
+  const double kdt = (!KAHAN && fuse) ? dt : hdt;
+  const double dv = a * kdt;
+  const double dw = KAHAN ? (tau * inv_inertia) * kdt : tau * (inv_inertia * kdt);
+  if (KAHAN && fuse && moving && part) {
+    kahan_add(v, vres, dv);
+    if (own_spin) kahan_add(w, wres, dw);
+  }
+  // wrap and removal, each lane its axis
+  const bool per = pick(c, P.periodic) != 0;
+  const double lo = pick(c, P.bmin), hi = pick(c, P.bmax);
+  const bool inner = !part || (xo > pick(c, P.inner_lo) && xo < pick(c, P.inner_hi));
+  bool keep = true;
+  if (part && !inner) {
+    if (per) {
+      const double size = pick(c, P.bsize);
+      if (x < lo) x = x + size;
+      else if (x >= hi) x = x - size;
+    } else {
+      keep = c == 1 ? x >= lo - 1.0 : (x >= lo - 1.0 && x <= hi + 1.0);
+    }
+  }
+  const unsigned leaving = __ballot_sync(ALL, on && !keep);  // every lane takes part
+  const bool gone = on && (leaving & quad_mask()) != 0;
+  if (gone) {
+    if (part) {
+      reinterpret_cast<double*>(B.xr)[at] = __longlong_as_double(0x7ff8000000000000ll);
+      reinterpret_cast<float*>(B.xf)[at] = __int_as_float(0x7fc00000);
+    } else {
+      B.flags[k] = fl | PF_DEAD;
+      atomicAdd(&C->removed, 1ull);
+    }
+    on = false;
+  }
+  const bool move = moving && !gone && part;
+  if (move) {
+    if (KAHAN) {
+      kahan_add(v, vres, dv);
+      kahan_add(x, xres, v * dt);
+      reinterpret_cast<double*>(B.vres)[at] = vres;
+      reinterpret_cast<double*>(B.xres)[at] = xres;
+      if (own_spin) {
+        kahan_add(w, wres, dw);
+        reinterpret_cast<double*>(B.wres)[at] = wres;
+      }
+    } else {
+      v = v + dv;
+      x = x + v * dt;
+      if (own_spin) w = w + dw;
+    }
+    reinterpret_cast<double*>(B.vm)[at] = v;
+    if (own_spin) reinterpret_cast<double*>(B.wc)[at] = w;
+  }
+  const float xf = (float)x;
+  if (on && part) {
+    reinterpret_cast<double*>(B.xr)[at] = x;
+    reinterpret_cast<float*>(B.xf)[at] = xf;
+  }
+  if (P.mode == 0) {
+    int32_t q = 0;
+    if (on && part) q = ref_axis_fast(x, xf, lo, (float)lo, P.href, P.inv_href, (float)P.inv_href);
+    const int32_t c0 = __shfl_sync(ALL, q, 0, 4), c1 = __shfl_sync(ALL, q, 1, 4), c2 = __shfl_sync(ALL, q, 2, 4);
+    if (on && !part) {
+      const unsigned long long code = pack_code(c0, c1, c2);
+      if (code != (unsigned long long)__double_as_longlong(w))
+        reinterpret_cast<double*>(B.wc)[at] = __longlong_as_double((long long)code);
+    }
+  }
+  const float mag = fabsf(xf);
+  const unsigned top = __reduce_max_sync(ALL, on && part && mag >= 0.0f ? __float_as_uint(mag) : 0u);
+  if ((threadIdx.x & 31) == 0 && top > C->xmax) atomicMax(&C->xmax, top);
+  float d = xf - ref;
+  if (per) {
+    const float size = pick(c, P.bsizef);
+    d -= size * rintf(d / size);
+  }
+  d = d * d;
+  const float d2 = quad_word(d, 0) + quad_word(d, 1) + quad_word(d, 2);
+  const float half_skin = (float)(0.5 * P.skin);
+  return on && !(d2 <= half_skin * half_skin);
+}
+
+// The sums, a and tau of particle k (one a quad, whole warps).
+template <bool F32REC>
+__device__ __forceinline__ void sum_quad(const StepParams& P, const Bank& B, Ctrl* C, int k, bool on) {
+  const int c = threadIdx.x & 3;
+  on = on && !(B.flags[on ? k : 0] & PF_DEAD);
+  if (!on || c == 3) return;
+  double F = 0.0, T = 0.0;
+  const uint32_t n = P.ccnt[k], off = P.coff[k];
+  const double inv_mass = B.vres[k].w;
+  if (F32REC) {
+    const float* res = P.cresf + 6 * (size_t)off + c;
+    float f = 0.0f, t = 0.0f, f1 = 0.0f, t1 = 0.0f;
+    if (n > 0) { f1 = res[0]; t1 = res[3]; }
+    for (uint32_t q = 0; q < n; ++q) {
+      const float f0 = f1, t0 = t1;
+      if (q + 1 < n) { f1 = res[6 * q + 6]; t1 = res[6 * q + 9]; }
+      f = f + f0;
+      t = t + t0;
+    }
+    F = f2d_exact(f);
+    T = f2d_exact(t);
+  } else {
+    const double* res = P.cres + 6 * (size_t)off + c;
+    double f1 = 0.0, t1 = 0.0;
+    if (n > 0) { f1 = res[0]; t1 = res[3]; }
+    for (uint32_t q = 0; q < n; ++q) {
+      const double f0 = f1, t0 = t1;
+      if (q + 1 < n) { f1 = res[6 * q + 6]; t1 = res[6 * q + 9]; }
+      F = F + f0;
+      T = T + t0;
+    }
+  }
+  if (P.ntri > 0) {
+    const uint32_t wn = P.wcnt[k], wo = P.woff[k];
+    for (uint32_t q = 0; q < wn; ++q) {
+      const bool ok = P.wok[wo + q] != 0;
+      const double f0 = P.wres[6 * (size_t)(wo + q) + c], t0 = P.wres[6 * (size_t)(wo + q) + 3 + c];
+      if (!ok) continue;
+      F = F + f0;
+      T = T + t0;
+    }
+  }
+  if (P.debug) {
+    P.dbgF[3 * (size_t)k + c] = F;
+    P.dbgT[3 * (size_t)k + c] = T;
+  }
+  if (!(finite_bits(F) & finite_bits(T))) atomicOr(&C->status, (unsigned)ST_NAN);
+  reinterpret_cast<double*>(B.acc)[4 * (size_t)k + c] = pick(c, P.gravity) + F * inv_mass;
+  reinterpret_cast<double*>(B.tq)[4 * (size_t)k + c] = plus_zero(T);
+}
+
+template <bool PHYS, bool HIST, typename R>
+__global__ void __launch_bounds__(SMALL_BLOCK, 1) k_steps(StepParams P) {
+  Ctrl* C = P.ctrl;
+  volatile Ctrl* W = C;
+  // (a resumed launch filters before its first barrier: a full wall buffer that
+  // another block reports meanwhile must not keep this one from the barrier)
+  if (W->halt & (HALT_LISTS | HALT_STUCK)) return;
+  constexpr bool FP64 = sizeof(R) == sizeof(double);
+  const Bank B = P.bank[C->bank];
+  const unsigned long long target = C->target;
+  unsigned long long done = C->steps_done;
+  bool fuse = C->pending != 0, resume = C->resume != 0;
+  const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+  const bool quads = P.n <= QUAD_MAX;
+  // consecutive warps of items go to consecutive blocks, so few items occupy
+  // one FP64 unit each of as many multiprocessors as there are
+  const int lane = threadIdx.x & 31;
+  const Span sp{(int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + lane, (int)(gridDim.x * blockDim.x)};
+  const int quad0 = (sp.at - lane) >> 2, quad_all = sp.all >> 2;  // of the warp
+  unsigned gen = 0;
+  for (unsigned s = 0; s < SMALL_STEPS && done < target; ++s) {
+    uint32_t* ctot = P.ctot + (s & 1u) * CTOT_WORDS;
+    if (!resume) {
+      bool rebuild = false;
+      if (quads) {
+        for (int b = quad0; b < P.n; b += quad_all) {
+          const int k = b + (lane >> 2);
+          rebuild |= first_half_quad<FP64>(P, C, B, fuse, k, k < P.n);
+        }
+      } else {
+        rebuild = first_half_pass<FP64>(P, C, B, fuse, sp);
+      }
+      if (rebuild) W->rebuild = 1;
+      if (!grid_barrier(C, gen)) return;
+      if (W->rebuild) {
+        if (first) W->resume = 1;
+        return;
+      }
+    }
+    resume = false;
+    filter_pass<PHYS, HIST, true>(P, C, B, ctot, sp);
+    if (!grid_barrier(C, gen)) return;
+    if (W->halt) {  // the wall candidates outgrew their buffer: the host finishes this step
+      if (first) W->resume = 0;
+      return;
+    }
+    contact_pass<PHYS, HIST, R, false>(P, C, B, ctot, sp);
+    // the next step's counters, last read two barriers ago
+    if (blockIdx.x == 0 && threadIdx.x < CTOT_WORDS) P.ctot[((s + 1u) & 1u) * CTOT_WORDS + threadIdx.x] = 0u;
+    if (!grid_barrier(C, gen)) return;
+    if (quads) {
+      for (int b = quad0; b < P.n; b += quad_all) {
+        const int k = b + (lane >> 2);
+        sum_quad<!FP64>(P, B, C, k, k < P.n);
+      }
+      __syncwarp();  // the quad's next first half reads what its lanes wrote
+    } else {
+      for (int k = sp.at; k < P.n; k += sp.all)
+        if (!(B.flags[k] & PF_DEAD)) sum_particle<!FP64>(P, B, C, k);
+    }
+    ++done;
+    fuse = true;
+    if (first) {
+      W->steps_done = done;
+      W->pending = 1;
+      W->resume = 0;
+      if (W->overlap_flag) {
+        W->overlap_steps = W->overlap_steps + 1;
+        W->overlap_flag = 0;
+        atomicOr(&C->status, (unsigned)ST_OVERLAP);
+      }
+    }
+  }
+}
+
+// After k_steps: whether the rebuild chain runs (IF node), then whether the
+// loop goes on. An iteration completes a step or rebuilds the lists for one, so
+// the loop ends after 2 target + 8 iterations whatever the counters say.
+__global__ void k_steps_next(StepParams P, cudaGraphConditionalHandle rebuild, cudaGraphConditionalHandle loop, int end) {
+  Ctrl* C = P.ctrl;
+  if (!end) {
+    C->bar = 0;
+    for (int q = 0; q < 2 * CTOT_WORDS; ++q) P.ctot[q] = 0;
+    cudaGraphSetConditional(rebuild, (C->rebuild && !C->halt) ? 1u : 0u);
+    return;
+  }
+  C->iters += 1;
+  const bool again = !C->halt && C->steps_done < C->target && C->iters < 2 * C->target + 8;
+  cudaGraphSetConditional(loop, again ? 1u : 0u);
 }
 
 __global__ void k_clear_pending(StepParams P) {
@@ -2094,6 +2525,7 @@ __global__ void k_end_step(StepParams P, cudaGraphConditionalHandle loop, int in
   if (!C->halt) {
     C->steps_done += 1;
     C->pending = 1;
+    C->resume = 0;
     if (C->overlap_flag) {
       C->overlap_steps += 1;
       C->status |= ST_OVERLAP;
@@ -2265,6 +2697,42 @@ int launch_force(const StepParams& P, cudaStream_t s, const SideStream& side) {
     if (P.prec == 1) launch_force_t<float, false>(P, g, s);
     else launch_force_t<double, false>(P, g, s);
   }
+  return 1;
+}
+
+// At most one block of k_steps a multiprocessor, of two threads a particle (a
+// quad: four) in warps by the hundred and twenty-eight.
+template <bool PHYS, bool HIST, typename R>
+static int launch_steps_t(const StepParams& P, cudaStream_t s) {
+  const int threads = P.n * (P.n <= QUAD_MAX ? 4 : 2);
+  const int grid = std::min(P.nsm, (threads + 127) / 128);
+  const int block = std::min(SMALL_BLOCK, ((threads + grid - 1) / grid + 127) / 128 * 128);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_steps<PHYS, HIST, R>, P) == cudaSuccess ? 1 : 0;
+}
+
+bool steps_in_one_launch(const StepParams& P) {
+  return P.n > 0 && P.n <= SMALL_MAX && P.force_path == 0 && P.nmodel != 3;
+}
+
+int launch_steps_small(const StepParams& P, cudaStream_t s) {
+  const bool hist = P.mode == 1 && P.tmodel != 0, mixed = P.prec == 1;
+  if (P.mode == 0) return mixed ? launch_steps_t<false, false, float>(P, s) : launch_steps_t<false, false, double>(P, s);
+  if (hist) return mixed ? launch_steps_t<true, true, float>(P, s) : launch_steps_t<true, true, double>(P, s);
+  return mixed ? launch_steps_t<true, false, float>(P, s) : launch_steps_t<true, false, double>(P, s);
+}
+
+int launch_steps_next(const StepParams& P, cudaGraphConditionalHandle rebuild, cudaGraphConditionalHandle loop, int end,
+                      cudaStream_t s) {
+  k_steps_next<<<1, 1, 0, s>>>(P, rebuild, loop, end);
   return 1;
 }
 

@@ -27,7 +27,7 @@ struct alignas(32) D4 {
 //              cell (parity mode; implies PF_NOIMAGE)
 enum : uint32_t { PF_FIXED = 1u, PF_DEAD = 2u, PF_WALLFAR = 4u, PF_NOIMAGE = 8u, PF_ONECELL = 16u };
 
-enum : unsigned { ST_OVERLAP = 1u, ST_NAN = 2u, ST_NLIST_GROW = 4u, ST_WALL_GROW = 8u };
+enum : unsigned { ST_OVERLAP = 1u, ST_NAN = 2u, ST_NLIST_GROW = 4u, ST_WALL_GROW = 8u, ST_STUCK = 16u };
 
 // Device control block: written by kernels, read by the host after a chunk.
 struct Ctrl {
@@ -43,6 +43,8 @@ struct Ctrl {
   unsigned long long overlap_steps;
   int pending;                    // the last completed step still owes its second half kick
   unsigned int wall_need;         // wall candidates a halted filter wanted room for
+  unsigned int bar;               // k_steps: blocks that have arrived at its grid barriers
+  int resume;                     // k_steps: the current step's first half is done (it stopped for a rebuild)
   unsigned int xmax;              // bits of the largest |coordinate| of the FP32 mirror since the upload
   unsigned int xout;              // list rebuild: bits of the farthest distance of a particle outside the periodic faces
   unsigned long long target;      // device step loop: run while steps_done < target
@@ -75,6 +77,8 @@ constexpr uint32_t GROUP_ALL = 0xFFFFFFFFu;
 // wall candidates outgrew their arena (contact filter)
 constexpr int HALT_LISTS = 1;
 constexpr int HALT_WALLS = 2;
+// a grid barrier of k_steps ran out of its bounded wait (an error, not recovered)
+constexpr int HALT_STUCK = 4;
 
 // A rigid surface velocity V + W x (p - C) of a set of triangles whose geometry
 // stays put (a surface of revolution turning about its own axis, a belt). The
@@ -152,11 +156,11 @@ struct StepParams {
   uint32_t* wcnt;   // wall candidates of slot k
   uint32_t wcap;    // wall candidate capacity
   uint32_t* coff;   // first result slot of particle k (its ccnt results are contiguous)
-  uint32_t* clist;  // compact list of evaluating record slots
+  uint4* clist;     // compact list of evaluating records: slot, partner, m and visits, result slot
   // [0] records, [1] evaluating records, [2] network queue, [3] deferred pairs, [4] wall candidates, [5] hard pairs
-  uint32_t* ctot;
-  uint32_t* jfb;    // record slots deferred to the reference-Newton pass (null: no deferral)
-  uint32_t* jhard;  // record slots that the filter sends to that Newton at once (null with jfb)
+  uint32_t* ctot;   // (k_steps alternates between two such sets)
+  uint32_t* jfb;    // entries of clist deferred to the reference-Newton pass (null: no deferral)
+  uint4* jhard;     // records (as clist) that the filter sends to that Newton at once (null with jfb)
   double* cres;     // per record: force (3) and torque (3) on the row's particle
   float* cresf;     // the same buffer as FP32 records (the mixed form: its pair forces are FP32 values)
   int nmodel, tmodel, mode, prec;
@@ -216,7 +220,7 @@ struct StepParams {
   int jkr_solver;
   float jdom_lo[4], jdom_hi[4];  // raw-feature range of the training set
   const MlpInfer* mlp;
-  uint2* jq;        // network queue: (evaluating index, record slot); length ctot[2]
+  uint32_t* jq;     // network queue: entries of clist; length ctot[2]
   float* jguess;    // per evaluating index: predicted a/R* (NaN = outside the training range)
   // diagnostics
   double* dbgF;

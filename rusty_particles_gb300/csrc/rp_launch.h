@@ -63,6 +63,13 @@ int launch_triangle_grid(const float* v, const float* nrm, const uint32_t* grp, 
 int launch_first_half(const StepParams& P, cudaStream_t s);  // each returns kernels launched
 int launch_second_half(const StepParams& P, cudaStream_t s);
 int launch_rebuild_condition(const StepParams& P, cudaGraphConditionalHandle h, cudaStream_t s);
+// Whether a stepping call runs its steps inside cooperative launches (k_steps),
+// and the nodes of that loop's body; launch_steps_small returns 0 when such a
+// launch is not possible.
+bool steps_in_one_launch(const StepParams& P);
+int launch_steps_small(const StepParams& P, cudaStream_t s);
+int launch_steps_next(const StepParams& P, cudaGraphConditionalHandle rebuild, cudaGraphConditionalHandle loop, int end,
+                      cudaStream_t s);
 int launch_end_step_loop(const StepParams& P, cudaGraphConditionalHandle loop, cudaStream_t s);
 // A second stream for work that runs beside the force pass, with the events
 // that fork it from the pass's stream and join it again.
