@@ -1029,6 +1029,8 @@ int Engine::recover_halt() {
     }
     if (ctrl_h_->halt & HALT_WALLS) {
       TRY(alloc_walls(std::max<size_t>(wcap_ * 2, (size_t)ctrl_h_->wall_need * 5 / 4 + 65536)));
+      const int none = 0;  // that filter has kicked the spins
+      CK(cudaMemcpyAsync(&ctrl_->spin_due, &none, sizeof(int), cudaMemcpyHostToDevice, stream_));
       tot_.status |= ST_WALL_GROW;
     }
     graph_dirty_ = true;
@@ -1095,7 +1097,7 @@ int Engine::build_graph(bool small) {
     }
     sk = k + launch_steps_next(P_, hif, hloop, 0, cap_stream_);
   } else {
-    sk = launch_first_half(P_, cap_stream_);
+    sk = launch_first_half(P_, cap_stream_, spin_in_filter(P_));
     sk += launch_rebuild_condition(P_, hif, cap_stream_);
   }
   cudaStreamCaptureStatus st;

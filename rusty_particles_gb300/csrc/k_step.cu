@@ -799,7 +799,8 @@ __device__ __forceinline__ Span grid_span() {
 // 484 bytes (the residuals' read and three writes) off this kernel.
 // (Called by a whole grid, each thread for its items of the span; returns
 // whether one of the thread's particles asks for a rebuild.)
-template <bool KAHAN>
+// SPIN = false leaves the spin's kicks to the contact filter (spin_kick).
+template <bool KAHAN, bool SPIN>
 __device__ __forceinline__ bool first_half_pass(const StepParams& P, Ctrl* C, const Bank& B, bool FUSE, Span sp) {
   const double dt = P.dt;
   const bool anyp = P.periodic[0] | P.periodic[1] | P.periodic[2];
@@ -813,8 +814,10 @@ __device__ __forceinline__ bool first_half_pass(const StepParams& P, Ctrl* C, co
   for (int k = sp.at; k < P.n; k += sp.all) {
     uint32_t fl = B.flags[k];
     if (fl & PF_DEAD) continue;
-    D4 xr = B.xr[k], vm = B.vm[k], wc = B.wc[k];
-    V x = xyz(xr), v = xyz(vm), w = xyz(wc);
+    D4 xr = B.xr[k], vm = B.vm[k], wc;
+    if (SPIN) wc = B.wc[k];
+    else wc.w = B.wc[k].w;
+    V x = xyz(xr), v = xyz(vm), w = SPIN ? xyz(wc) : x;
     const bool moving = !(fl & PF_FIXED);
     V vres = vmk(0.0, 0.0, 0.0), wres = vres, xres = vres, dv = vres, dw = vres;
     double inv_inertia = 0.0, inv_mass = 0.0;
@@ -823,14 +826,17 @@ __device__ __forceinline__ bool first_half_pass(const StepParams& P, Ctrl* C, co
       // the fused second half of the previous step and this step's first
       // half kick with the same a and tau: the increments are computed once
       const V a = xyz(B.acc[k]);
-      const V tau = xyz(B.tq[k]);
-      const D4 vr4 = B.vres[k];
-      inv_mass = vr4.w;
-      const D4 wr4 = B.wres[k];
-      inv_inertia = wr4.w;
+      V tau = vres;
+      if (SPIN) {
+        tau = xyz(B.tq[k]);
+        const D4 wr4 = B.wres[k];
+        inv_inertia = wr4.w;
+        if (KAHAN) wres = xyz(wr4);
+      }
       if (KAHAN) {
+        const D4 vr4 = B.vres[k];
+        inv_mass = vr4.w;
         vres = xyz(vr4);
-        wres = xyz(wr4);
         xres = xyz(B.xres[k]);
       }
       // the mixed form joins the pending second half kick and this step's
@@ -841,8 +847,10 @@ __device__ __forceinline__ bool first_half_pass(const StepParams& P, Ctrl* C, co
       // its value, adding zeros to it: two of the seven 32-byte stores fall
       // away and, where that holds for a whole warp, 30 of the ~90 FP64
       // instructions (decided by the warp: lanes going apart cost more)
-      own_spin = some_bits(tau) || (KAHAN && some_bits(wres));
-      spin = __any_sync(__activemask(), own_spin);
+      if (SPIN) {
+        own_spin = some_bits(tau) || (KAHAN && some_bits(wres));
+        spin = __any_sync(__activemask(), own_spin);
+      }
       if (spin) dw = KAHAN ? (tau * inv_inertia) * kdt : tau * (inv_inertia * kdt);
       if (KAHAN && FUSE) {
         kahan_add(v, vres, dv);
@@ -888,7 +896,7 @@ __device__ __forceinline__ bool first_half_pass(const StepParams& P, Ctrl* C, co
         if (spin) w = w + dw;
       }
       B.vm[k] = D4{v.x, v.y, v.z, vm.w};
-      wc.x = w.x; wc.y = w.y; wc.z = w.z;
+      if (SPIN) { wc.x = w.x; wc.y = w.y; wc.z = w.z; }
     }
     const double code = wc.w;
     const float4 xf = make_float4((float)x.x, (float)x.y, (float)x.z, (float)xr.w);
@@ -898,7 +906,11 @@ __device__ __forceinline__ bool first_half_pass(const StepParams& P, Ctrl* C, co
       const int32_t c2 = ref_axis_fast(x.z, xf.z, P.bmin[2], bminf[2], P.href, P.inv_href, inv_hf);
       wc.w = __longlong_as_double((long long)pack_code(c0, c1, c2));
     }
-    if (own_spin || __double_as_longlong(code) != __double_as_longlong(wc.w)) B.wc[k] = wc;
+    if (SPIN) {
+      if (own_spin || __double_as_longlong(code) != __double_as_longlong(wc.w)) B.wc[k] = wc;
+    } else if (__double_as_longlong(code) != __double_as_longlong(wc.w)) {
+      B.wc[k].w = wc.w;
+    }
     B.xr[k] = D4{x.x, x.y, x.z, xr.w};
     B.xf[k] = xf;
     // the largest |coordinate| sets the filter's rounding margin (the bits of
@@ -917,12 +929,38 @@ __device__ __forceinline__ bool first_half_pass(const StepParams& P, Ctrl* C, co
   return want_rebuild;
 }
 
-template <bool KAHAN>
+template <bool KAHAN, bool SPIN>
 __global__ void __launch_bounds__(KAHAN ? 128 : 256, KAHAN ? 5 : 4) k_first_half(StepParams P) {
   Ctrl* C = P.ctrl;
   if (C->halt) return;
-  if (first_half_pass<KAHAN>(P, C, P.bank[C->bank], C->pending != 0, grid_span())) C->rebuild = 1;
+  if (first_half_pass<KAHAN, SPIN>(P, C, P.bank[C->bank], C->pending != 0, grid_span())) C->rebuild = 1;
+  if (!SPIN && blockIdx.x == 0 && threadIdx.x == 0) C->spin_due = 1;
 }
+
+// The spin's part of the first half for slot k (with the previous step's second
+// half kick when `fuse`): the operations of first_half_pass. Nothing before the
+// pair kernel reads a spin, so in the device loop the contact filter does this:
+// the integrator is bound by the FP64 pipe and the filter by gathers, with that
+// pipe idle. Only x, y, z are written; other threads read the cell code in w.
+// FP64 form only (us a step with / without: hopper 1 M 687 / 716, gas 1 M 270 /
+// 305, boxes 1.6 M 907 / 945): the mixed form's spin is 9 FP64 instructions, not
+// 30, and the filter's extra traffic costs more (drum 4.2 M 1499 / 1450).
+__device__ __forceinline__ void spin_kick(const StepParams& P, const Bank& B, int k, bool fuse) {
+  const D4 wr4 = B.wres[k];
+  const V tau = xyz(B.tq[k]);
+  V wres = xyz(wr4);
+  if (!(some_bits(tau) || some_bits(wres))) return;
+  double* at = &B.wc[k].x;
+  const double2 w0 = *reinterpret_cast<const double2*>(at);
+  V w = vmk(w0.x, w0.y, at[2]);
+  const V dw = (tau * wr4.w) * (0.5 * P.dt);
+  if (fuse) kahan_add(w, wres, dw);
+  kahan_add(w, wres, dw);
+  B.wres[k] = D4{wres.x, wres.y, wres.z, wr4.w};
+  *reinterpret_cast<double2*>(at) = make_double2(w.x, w.y);
+  at[2] = w.z;
+}
+bool spin_in_filter(const StepParams& P) { return P.prec == 0 && P.force_path == 0; }
 
 // Completes the last step of a stepping call (the pending second half);
 // k_clear_pending then marks the state complete. KAHAN as in k_first_half.
@@ -1395,6 +1433,7 @@ __device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const 
   const size_t plane = (size_t)P.n * P.cap;
   const float margin = pretest_margin(P, C);
   const int lane = threadIdx.x & 31;
+  const bool kick = !COHERENT && C->spin_due != 0, fuse = C->pending != 0;
   // slots in the rebuild-time order (tiles of 256 sorted by list length), so
   // a warp's lanes walk lists of similar length
   for (int i0 = sp.at - lane; i0 < P.n; i0 += sp.all) {
@@ -1416,6 +1455,7 @@ __device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const 
       const uint32_t cnt = B.ncnt[k];
       const uint32_t* row = B.nbr + (size_t)k * P.cap;
       CRec* out = P.crec + (size_t)k * P.cap;
+      if (kick && !(flk & PF_FIXED)) spin_kick(P, B, k, fuse);
       const bool wide = (P.cap & 3) == 0;  // rows on 16 bytes
       // where latency is all that counts, the first eight entries come with the
       // particle itself (a dilute bed of a million would read rows it does not have)
@@ -1600,7 +1640,9 @@ __device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const 
 template <bool PHYS, bool HIST>
 __global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
   Ctrl* C = P.ctrl;
-  if (C->halt) return;
+  // a full wall buffer that another block reports must not keep this one from
+  // its spin kicks (the device loop ends with the step that halts)
+  if (C->spin_due ? (C->halt & HALT_LISTS) : C->halt) return;
   filter_pass<PHYS, HIST, false>(P, C, P.bank[C->bank], P.ctot, grid_span());
 }
 
@@ -2452,7 +2494,7 @@ __global__ void __launch_bounds__(SMALL_BLOCK, 1) k_steps(StepParams P) {
           rebuild |= first_half_quad<FP64>(P, C, B, fuse, k, k < P.n);
         }
       } else {
-        rebuild = first_half_pass<FP64>(P, C, B, fuse, sp);
+        rebuild = first_half_pass<FP64, true>(P, C, B, fuse, sp);
       }
       if (rebuild) W->rebuild = 1;
       if (!grid_barrier(C, gen)) return;
@@ -2526,6 +2568,7 @@ __global__ void k_end_step(StepParams P, cudaGraphConditionalHandle loop, int in
     C->steps_done += 1;
     C->pending = 1;
     C->resume = 0;
+    C->spin_due = 0;
     if (C->overlap_flag) {
       C->overlap_steps += 1;
       C->status |= ST_OVERLAP;
@@ -2601,12 +2644,13 @@ void launch_bed_stats(const StepParams& P, double* out, unsigned long long* pair
   k_bed_stats<<<grid_for(P.n, 256), 256, 0, s>>>(P, out, pairs);
 }
 
-int launch_first_half(const StepParams& P, cudaStream_t s) {
+int launch_first_half(const StepParams& P, cudaStream_t s, bool spin_later) {
   if (P.n == 0) return 0;
   // the Kahan form holds 90 registers: blocks of 128 keep 20 warps resident
   // per multiprocessor where blocks of 256 keep 16
-  if (P.prec == 1) k_first_half<false><<<grid_for(P.n, 256), 256, 0, s>>>(P);
-  else k_first_half<true><<<grid_for(P.n, 128), 128, 0, s>>>(P);
+  if (P.prec == 1) k_first_half<false, true><<<grid_for(P.n, 256), 256, 0, s>>>(P);
+  else if (spin_later) k_first_half<true, false><<<grid_for(P.n, 128), 128, 0, s>>>(P);
+  else k_first_half<true, true><<<grid_for(P.n, 128), 128, 0, s>>>(P);
   return 1;
 }
 

@@ -43,6 +43,7 @@ struct Ctrl {
   unsigned long long overlap_steps;
   int pending;                    // the last completed step still owes its second half kick
   unsigned int wall_need;         // wall candidates a halted filter wanted room for
+  int spin_due;                   // the step's first half left the spin kicks to the contact filter
   unsigned int bar;               // k_steps: blocks that have arrived at its grid barriers
   int resume;                     // k_steps: the current step's first half is done (it stopped for a rebuild)
   unsigned int xmax;              // bits of the largest |coordinate| of the FP32 mirror since the upload

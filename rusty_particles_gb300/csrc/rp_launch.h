@@ -60,7 +60,10 @@ int launch_triangle_grid(const float* v, const float* nrm, const uint32_t* grp, 
                          uint32_t* part, uint32_t* counts, uint32_t* tstart, cudaStream_t s, const uint32_t** items);
 
 // k_step.cu
-int launch_first_half(const StepParams& P, cudaStream_t s);  // each returns kernels launched
+// Each returns kernels launched. spin_later: the step's contact filter kicks the
+// spins (Ctrl::spin_due); only where no later step's kernels follow a halt.
+int launch_first_half(const StepParams& P, cudaStream_t s, bool spin_later = false);
+bool spin_in_filter(const StepParams& P);  // whether that pays
 int launch_second_half(const StepParams& P, cudaStream_t s);
 int launch_rebuild_condition(const StepParams& P, cudaGraphConditionalHandle h, cudaStream_t s);
 // Whether a stepping call runs its steps inside cooperative launches (k_steps),
