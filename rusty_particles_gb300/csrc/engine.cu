@@ -66,6 +66,11 @@ Law Engine::make_law(const Material& m) const {
   L.mu = m.mu;
   L.jkr_C = (8.0 * kPiH) * L.gamma_pp / L.es_pp;
   L.jkr_Cf = (float)L.jkr_C;
+  L.es_ppf = (float)L.es_pp;
+  L.gs_ppf = (float)L.gs_pp;
+  L.gamma_ppf = (float)L.gamma_pp;
+  L.beta_absf = (float)L.beta_abs;
+  L.muf = (float)L.mu;
   return L;
 }
 
@@ -552,6 +557,10 @@ int Engine::build_params() {
   double skin = skin_user > 0.0 ? skin_user : 0.1 * 2.0 * rmax;
   if (!(skin > 0.0)) skin = 1e-6;
   P.skin = skin;
+  P.hdt = 0.5 * dt;
+  P.half_skinf = (float)(0.5 * skin);
+  P.inv_hreff = (float)P.inv_href;
+  for (int k = 0; k < 3; ++k) P.bminf[k] = (float)bmin[k];
   P.list_scale = 1.0f + 1e-5f;
   {
     double cutmax = 2.0 * rmax * adh;

@@ -170,6 +170,26 @@ __device__ __forceinline__ V cross_fma(V a, V b) {
 }
 __device__ __forceinline__ V mad(double s, V a, V b) { return V{fma(s, a.x, b.x), fma(s, a.y, b.y), fma(s, a.z, b.z)}; }
 
+// double -> float, rounded to nearest even, on the integer pipe where the value
+// and its rounding are normal floats (zeros and the rest take the hardware
+// conversion, an FP64-pipe instruction). It pays in the integrator, which that
+// pipe bounds (drum 4.2 M mixed 1.3 %), not in the mixed pair kernel, whose 14
+// conversions a contact cost more as integer instructions (1.2 % on the same
+// bed: it waits for its gathers as well).
+__device__ __forceinline__ float d2f_exact(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x), e = hi & 0x7FFFFFFFu;
+  if (e - 0x38100000u >= 0x47E00000u - 0x38100000u) return (float)x;
+  const uint32_t f = ((e - 0x38000000u) << 3) | (lo >> 29);
+  const uint32_t up = ((lo & 0x1FFFFFFFu) + 0x0FFFFFFFu + (f & 1u)) >> 29;
+  return __uint_as_float((f + up) | (hi & 0x80000000u));
+}
+// The law's constants in the pair law's precision (the FP32 ones come rounded).
+template <typename R> __device__ __forceinline__ R law_es(const Law& L) { return sizeof(R) == 4 ? (R)L.es_ppf : (R)L.es_pp; }
+template <typename R> __device__ __forceinline__ R law_gamma(const Law& L) { return sizeof(R) == 4 ? (R)L.gamma_ppf : (R)L.gamma_pp; }
+template <typename R> __device__ __forceinline__ R law_beta(const Law& L) { return sizeof(R) == 4 ? (R)L.beta_absf : (R)L.beta_abs; }
+template <typename R> __device__ __forceinline__ R law_mu(const Law& L) { return sizeof(R) == 4 ? (R)L.muf : (R)L.mu; }
+template <typename R> __device__ __forceinline__ R law_gs(const Law& L) { return sizeof(R) == 4 ? (R)L.gs_ppf : (R)L.gs_pp; }
+
 // ------------------------------------------------------------- force laws
 // src/physics.rs:49-70
 template <typename R>
@@ -185,7 +205,7 @@ __device__ __forceinline__ R hertz_mag(R overlap, R vn, R es, R rs, R ms, R beta
   R s = sqrt_rn(rs * overlap);
   R fe = R(4.0 / 3.0) * es * s * overlap;
   R kt = R(2) * es * s;
-  R cn = R(2) * sqrt_rn(ms * kt) * beta_abs;
+  R cn = sqrt_rn(ms * kt) * (R(2) * beta_abs);  // == (2 sqrt) beta: doubling is exact
   R fd = -cn * vn;
   return relu(fe + fd);
 }
@@ -516,7 +536,8 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
     vt = cvt<R>(rvd - vnd * nd);
   }
   const R rs = div_rn(rir * rjr, rir + rjr);
-  const R ms = div_rn((R)mi * (R)mj, (R)mi + (R)mj);
+  const R mir = (R)mi, mjr = (R)mj;
+  const R ms = div_rn(mir * mjr, mir + mjr);
   R fmag;
   int jkind = JKR_FALLBACK;
   if (JKR && P.jkr_solver != 0 && !newton && L.gamma_pp > 0.0) {
@@ -536,7 +557,7 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
   }
   if (jkind != JKR_FALLBACK) {
   } else if (JKR && !F32) {
-    fmag = jkr_mag<R>(overlap, (R)L.es_pp, rs, (R)L.gamma_pp);
+    fmag = jkr_mag<R>(overlap, law_es<R>(L), rs, law_gamma<R>(L));
   } else if (JKR) {
     // The contact radius has a square-root fold next to the pull-off: there
     // the FP32 iteration cannot resolve the root (an FP32 residual moves it by
@@ -547,13 +568,13 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
       if (jkr_certify(x, c, jkr_c23(c), overlap > R(0)) == JKR_FALLBACK) return false;
     }
     bool near = false;
-    fmag = jkr_mag<R>(overlap, (R)L.es_pp, rs, (R)L.gamma_pp, &near);
+    fmag = jkr_mag<R>(overlap, law_es<R>(L), rs, law_gamma<R>(L), &near);
     if (near) return false;
   } else {
-    fmag = normal_mag_vn<R>(P.nmodel, overlap, n, vn, (R)L.es_pp, rs, ms, (R)L.beta_abs, (R)L.gamma_pp);
+    fmag = normal_mag_vn<R>(P.nmodel, overlap, n, vn, law_es<R>(L), rs, ms, law_beta<R>(L), law_gamma<R>(L));
   }
   if (F32 && !JKR && P.nmodel == 4 && L.gamma_pp > 0.0) {
-    const R gamma = (R)L.gamma_pp, es = (R)L.es_pp;
+    const R gamma = law_gamma<R>(L), es = law_es<R>(L);
     const R f_pull = R(1.5) * R(kPi) * gamma * rs;
     const R delta_c = -sqrt(R(3) * (R(kPi) * R(kPi)) * (gamma * gamma) * rs / (es * es));
     if (fabs(vn) <= R(1e-6) * (len(rv) + R(1e-30))) return false;
@@ -569,9 +590,9 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
     if (F32) {
       const R vt2 = dot(vt, vt);
       if (fabs(vt2 - R(1e-8)) <= R(1e-5) * (vt2 + R(1e-8))) return false;
-      ft = coulomb_force_vt<R>(fnm, vt, (R)L.mu);
+      ft = coulomb_force_vt<R>(fnm, vt, law_mu<R>(L));
     } else {
-      ft = coulomb_force<R>(fnm, rv, n, (R)L.mu);
+      ft = coulomb_force<R>(fnm, rv, n, law_mu<R>(L));
     }
   } else if (!PHYS) {
     // G* = 0 in parity mode (src/material.rs:39-50): the spring force is
@@ -592,11 +613,11 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
   } else {
     T3<R> xi_s = t3(R(0), R(0), R(0));
     if (overlap > R(0)) {
-      R kt = P.tmodel == 2 ? R(8) * (R)L.gs_pp * sqrt(rs * overlap) : (R)L.gs_pp * rs;
+      R kt = P.tmodel == 2 ? R(8) * law_gs<R>(L) * sqrt(rs * overlap) : law_gs<R>(L) * rs;
       if (HIST) xi_s = t3((R)hist[0], (R)hist[plane], (R)hist[2 * plane]);
       xi_s = xi_s - dot(xi_s, n) * n;
-      ft = F32 ? spring_coulomb_vt<R>(fnm, vt, xi_s, kt, (R)L.mu, (R)P.dt)
-               : spring_coulomb<R>(fnm, rv, n, xi_s, kt, (R)L.mu, (R)P.dt);
+      ft = F32 ? spring_coulomb_vt<R>(fnm, vt, xi_s, kt, law_mu<R>(L), (R)P.dt)
+               : spring_coulomb<R>(fnm, rv, n, xi_s, kt, law_mu<R>(L), (R)P.dt);
     } else {
       ft = t3(R(0), R(0), R(0));
     }
@@ -753,8 +774,8 @@ __device__ __forceinline__ void kahan_add(V& s, V& r, V d) {
 // (tau/I as tau * (1/I), 1/I stored per particle in Bank::wres[k].w when the
 // state is uploaded; v and x are unchanged).
 __device__ __forceinline__ void second_half_kick(V& v, V& vres, V& w, V& wres, V a, V tau, double inv_inertia,
-                                                 double dt) {
-  const double hdt = 0.5 * dt;  // (0.5 a) dt == a (0.5 dt), both one rounding of a dt / 2
+                                                 double hdt) {
+  // (0.5 a) dt == a (0.5 dt), both one rounding of a dt / 2
   V dv = a * hdt;
   V yv = dv - vres;
   V tv = v + yv;
@@ -804,11 +825,11 @@ template <bool KAHAN, bool SPIN>
 __device__ __forceinline__ bool first_half_pass(const StepParams& P, Ctrl* C, const Bank& B, bool FUSE, Span sp) {
   const double dt = P.dt;
   const bool anyp = P.periodic[0] | P.periodic[1] | P.periodic[2];
-  const float half_skin = (float)(0.5 * P.skin);
-  // (0.5 a) dt and a (0.5 dt) are the same correctly rounded product
-  const double hdt = 0.5 * dt;
-  const float bminf[3] = {(float)P.bmin[0], (float)P.bmin[1], (float)P.bmin[2]};
-  const float inv_hf = (float)P.inv_href;
+  // (0.5 a) dt and a (0.5 dt) are the same correctly rounded product; the
+  // launch's constants come converted (each conversion or product here would be
+  // an FP64-pipe instruction of every warp: 7 of the mixed form's 40)
+  const double hdt = P.hdt;
+  const float half_skin = P.half_skinf, inv_hf = P.inv_hreff;
   const unsigned xmax = C->xmax;
   bool want_rebuild = false;
   for (int k = sp.at; k < P.n; k += sp.all) {
@@ -899,11 +920,11 @@ __device__ __forceinline__ bool first_half_pass(const StepParams& P, Ctrl* C, co
       if (SPIN) { wc.x = w.x; wc.y = w.y; wc.z = w.z; }
     }
     const double code = wc.w;
-    const float4 xf = make_float4((float)x.x, (float)x.y, (float)x.z, (float)xr.w);
+    const float4 xf = make_float4(d2f_exact(x.x), d2f_exact(x.y), d2f_exact(x.z), xo.w);
     if (P.mode == 0) {
-      const int32_t c0 = ref_axis_fast(x.x, xf.x, P.bmin[0], bminf[0], P.href, P.inv_href, inv_hf);
-      const int32_t c1 = ref_axis_fast(x.y, xf.y, P.bmin[1], bminf[1], P.href, P.inv_href, inv_hf);
-      const int32_t c2 = ref_axis_fast(x.z, xf.z, P.bmin[2], bminf[2], P.href, P.inv_href, inv_hf);
+      const int32_t c0 = ref_axis_fast(x.x, xf.x, P.bmin[0], P.bminf[0], P.href, P.inv_href, inv_hf);
+      const int32_t c1 = ref_axis_fast(x.y, xf.y, P.bmin[1], P.bminf[1], P.href, P.inv_href, inv_hf);
+      const int32_t c2 = ref_axis_fast(x.z, xf.z, P.bmin[2], P.bminf[2], P.href, P.inv_href, inv_hf);
       wc.w = __longlong_as_double((long long)pack_code(c0, c1, c2));
     }
     if (SPIN) {
@@ -953,7 +974,7 @@ __device__ __forceinline__ void spin_kick(const StepParams& P, const Bank& B, in
   double* at = &B.wc[k].x;
   const double2 w0 = *reinterpret_cast<const double2*>(at);
   V w = vmk(w0.x, w0.y, at[2]);
-  const V dw = (tau * wr4.w) * (0.5 * P.dt);
+  const V dw = (tau * wr4.w) * P.hdt;
   if (fuse) kahan_add(w, wres, dw);
   kahan_add(w, wres, dw);
   B.wres[k] = D4{wres.x, wres.y, wres.z, wr4.w};
@@ -976,11 +997,11 @@ __global__ void __launch_bounds__(256) k_second_half(StepParams P) {
     const D4 wr4 = B.wres[k], vr4 = B.vres[k];
     V v = xyz(vm), w = xyz(wc), vres = xyz(vr4), wres = xyz(wr4);
     if (KAHAN) {
-      second_half_kick(v, vres, w, wres, xyz(B.acc[k]), xyz(B.tq[k]), wr4.w, P.dt);
+      second_half_kick(v, vres, w, wres, xyz(B.acc[k]), xyz(B.tq[k]), wr4.w, P.hdt);
       B.vres[k] = D4{vres.x, vres.y, vres.z, vr4.w};
       B.wres[k] = D4{wres.x, wres.y, wres.z, wr4.w};
     } else {
-      const double hdt = 0.5 * P.dt;
+      const double hdt = P.hdt;
       v = v + xyz(B.acc[k]) * hdt;
       w = w + (xyz(B.tq[k]) * wr4.w) * hdt;
     }
@@ -2329,7 +2350,7 @@ __device__ __forceinline__ bool first_half_quad(const StepParams& P, Ctrl* C, co
       }
     }
   }
-  const double dt = P.dt, hdt = 0.5 * dt, inv_inertia = quad_word(wres, 3);
+  const double dt = P.dt, hdt = P.hdt, inv_inertia = quad_word(wres, 3);
   const unsigned spinning = __ballot_sync(ALL, moving && (nonzero_bits(tau) || (KAHAN && nonzero_bits(wres))));
   const bool own_spin = (spinning & quad_mask()) != 0;
   const double kdt = (!KAHAN && fuse) ? dt : hdt;
@@ -2391,7 +2412,7 @@ __device__ __forceinline__ bool first_half_quad(const StepParams& P, Ctrl* C, co
   }
   if (P.mode == 0) {
     int32_t q = 0;
-    if (on && part) q = ref_axis_fast(x, xf, lo, (float)lo, P.href, P.inv_href, (float)P.inv_href);
+    if (on && part) q = ref_axis_fast(x, xf, lo, pick(c, P.bminf), P.href, P.inv_href, P.inv_hreff);
     const int32_t c0 = __shfl_sync(ALL, q, 0, 4), c1 = __shfl_sync(ALL, q, 1, 4), c2 = __shfl_sync(ALL, q, 2, 4);
     if (on && !part) {
       const unsigned long long code = pack_code(c0, c1, c2);
@@ -2409,8 +2430,7 @@ __device__ __forceinline__ bool first_half_quad(const StepParams& P, Ctrl* C, co
   }
   d = d * d;
   const float d2 = quad_word(d, 0) + quad_word(d, 1) + quad_word(d, 2);
-  const float half_skin = (float)(0.5 * P.skin);
-  return on && !(d2 <= half_skin * half_skin);
+  return on && !(d2 <= P.half_skinf * P.half_skinf);
 }
 
 // The sums, a and tau of particle k (one a quad, whole warps).

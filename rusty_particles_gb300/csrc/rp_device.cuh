@@ -71,7 +71,8 @@ struct Law {
   double beta_abs;             // |ln e / sqrt(ln^2 e + pi^2)| of the particle restitution (host libm)
   double mu;                   // particle friction, used for pairs and walls (src/simulation.rs:489)
   double jkr_C;                // 8 pi gamma / E* of pairs, as src/physics.rs:165 forms it
-  float jkr_Cf, pad_;
+  float jkr_Cf;
+  float es_ppf, gs_ppf, gamma_ppf, beta_absf, muf;  // rounded for the FP32 pair law
 };
 constexpr uint32_t GROUP_ALL = 0xFFFFFFFFu;
 // Ctrl::halt bits: a neighbour list outgrew its capacity (list rebuild), the
@@ -192,6 +193,8 @@ struct StepParams {
   int fdims[3];
   uint32_t fncells;
   double skin;
+  double hdt;                            // dt / 2
+  float bminf[3], half_skinf, inv_hreff;  // bmin, skin / 2 and 1 / href, rounded
   float list_scale;  // 1 + relative margin of the FP32 list test
   // distance within which a pair can exert a force: min(r_sum cut_a, r_sum +
   // cut_b); the lists hold it plus the skin
