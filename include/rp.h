@@ -184,6 +184,10 @@ int rp_set_threads(int n);                               /* set_num_threads (src
 
 /* --- metrics and errors */
 int rp_get_stats(rp_sim* sim, rp_stats* out);
+/* rp_stats::overlap_warn_steps alone, without the device work of the other
+ * statistics (what a binding needs after every call to print the reference's
+ * overlap warning, src/simulation.rs:528-530). */
+int rp_overlap_warn_steps(rp_sim* sim, uint64_t* steps);
 /* Statistics of the bed in its current state, in FP64 on the device (no
  * reference counterpart; the reference's scripts compute them in Python):
  * out[0] kinetic energy, translational plus rotational with I = 2/5 m r^2;

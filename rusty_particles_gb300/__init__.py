@@ -398,9 +398,9 @@ class Simulation:
         """The reference prints a warning on every step with an overlap above
         20 % of a radius (src/simulation.rs:528-530); here once per call."""
         try:
-            s = RpStats()
-            if self._L.rp_get_stats(self._h, ctypes.byref(s)) == 0 and s.overlap_warn_steps > self._warned:
+            n = ctypes.c_uint64()
+            if self._L.rp_overlap_warn_steps(self._h, ctypes.byref(n)) == 0 and n.value > self._warned:
                 print(_OVERLAP_WARNING, file=sys.stderr)
-                self._warned = s.overlap_warn_steps
+                self._warned = n.value
         except Exception:
             pass

@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -139,7 +140,12 @@ void Engine::free_device() {
   jfb_alloc_ = 0;
   dfree(ctrl_);
   if (ctrl_h_) cudaFreeHost(ctrl_h_);
+  if (pin_buf_) cudaFreeHost(pin_buf_);
+  if (lim_h_) cudaFreeHost(lim_h_);
   ctrl_h_ = nullptr;
+  pin_buf_ = nullptr;
+  pin_n_ = 0;
+  lim_h_ = nullptr;
   if (ev0_) cudaEventDestroy(ev0_);
   if (ev1_) cudaEventDestroy(ev1_);
   for (cudaEvent_t e : fev_) cudaEventDestroy(e);
@@ -188,6 +194,7 @@ int Engine::ensure_gpu() {
   CK(cudaEventCreateWithFlags(&side_.join, cudaEventDisableTiming));
   TRY(dalloc(&ctrl_, 1));
   CK(cudaMallocHost((void**)&ctrl_h_, sizeof(Ctrl)));
+  CK(cudaMallocHost((void**)&lim_h_, 2 * sizeof(unsigned long long)));
   TRY(dalloc(&ke_, 1));
   {
     // kernels may dereference the caller's pageable arrays when the device
@@ -308,9 +315,9 @@ int Engine::set_group_material(uint32_t group, const Material& m) {
 
 size_t Engine::count() {
   if (!host_valid_ && gpu_ && dev_valid_) {
-    // live slots, without bringing the state to the host
-    if (cudaSetDevice(device_) != cudaSuccess || sync_ctrl() != RP_OK) return 0;
-    return (size_t)n_ - (size_t)ctrl_h_->removed;
+    // live slots, without bringing the state to the host (last_ is the control
+    // block as the last stepping call or upload left it)
+    return (size_t)n_ - (size_t)last_.removed;
   }
   if (!host_valid_) {
     if (download() != RP_OK) return 0;
@@ -1137,6 +1144,12 @@ int Engine::build_graph(bool small) {
   small_loop_ = small;
   cudaGraph_t t1 = nullptr;
   CK(cudaStreamEndCapture(cap_stream_, &t1));
+  // after the loop: the call's closing second half kick and the control block to the host
+  CK(cudaStreamBeginCaptureToGraph(cap_stream_, g, &wnode, nullptr, 1, cudaStreamCaptureModeRelaxed));
+  close_kernels_ = launch_second_half(P_, cap_stream_);
+  CK(cudaMemcpyAsync(ctrl_h_, ctrl_, sizeof(Ctrl), cudaMemcpyDeviceToHost, cap_stream_));
+  cudaGraph_t t3 = nullptr;
+  CK(cudaStreamEndCapture(cap_stream_, &t3));
   CK(cudaGraphInstantiate(&graph_exec_, g, 0));
   graph_dirty_ = false;
   return RP_OK;
@@ -1167,19 +1180,20 @@ int Engine::launch_steps_graph(uint64_t n) {
       }
     }
     const uint64_t before = last_.steps_done, rb_before = last_.rebuilds;
-    unsigned long long lim[2] = {before + remaining, 0ull};  // target, iters
-    CK(cudaMemcpyAsync(&ctrl_->target, &lim[0], sizeof(unsigned long long), cudaMemcpyHostToDevice, stream_));
-    CK(cudaMemcpyAsync(&ctrl_->iters, &lim[1], sizeof(unsigned long long), cudaMemcpyHostToDevice, stream_));
+    lim_h_[0] = before + remaining;  // target
+    lim_h_[1] = 0ull;                // iters
+    static_assert(offsetof(Ctrl, iters) == offsetof(Ctrl, target) + sizeof(unsigned long long), "one copy sets both");
+    CK(cudaMemcpyAsync(&ctrl_->target, lim_h_, 2 * sizeof(unsigned long long), cudaMemcpyHostToDevice, stream_));
     CK(cudaEventRecord(ev0_, stream_));
     CK(cudaGraphLaunch(graph_exec_, stream_));
     CK(cudaEventRecord(ev1_, stream_));
-    TRY(sync_ctrl());
+    CK(cudaStreamSynchronize(stream_));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev0_, ev1_);
     ms_total_ += ms;
     TRY(recover_halt());
     launches_ += (uint64_t)step_kernels_ * (small_loop_ ? ctrl_h_->iters : ctrl_h_->steps_done - before) +
-                 (uint64_t)chain_kernels_ * (ctrl_h_->rebuilds - rb_before);
+                 (uint64_t)chain_kernels_ * (ctrl_h_->rebuilds - rb_before) + (uint64_t)close_kernels_;
     TRY(finish_step_accounting());
     const uint64_t done = last_.steps_done - before;
     if (done == 0) {
@@ -1256,9 +1270,12 @@ int Engine::step(uint64_t n) {
   host_valid_ = false;
   int r = (use_graph_ && !profiling) ? launch_steps_graph(n) : launch_steps(n);
   if (r != RP_OK) return r;
-  launches_ += launch_second_half(P_, stream_);
-  CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(stream_));
+  if (last_.pending) {  // the host issued the last step (a graph ends with this itself)
+    launches_ += launch_second_half(P_, stream_);
+    CK(cudaGetLastError());
+    TRY(sync_ctrl());
+    last_.pending = ctrl_h_->pending;
+  }
   if (last_.removed > 0) TRY(compact_removed());
   return RP_OK;
 }
@@ -1467,9 +1484,8 @@ int Engine::fast_read_state(rp_state* st, bool& done) {
   done = false;
   if (!gpu_ || !dev_valid_ || n_ <= 0) return RP_OK;
   CK(cudaSetDevice(device_));
-  TRY(sync_ctrl());
-  if (ctrl_h_->halt != 0) return RP_OK;
-  const size_t n = (size_t)n_ - (size_t)ctrl_h_->removed;  // ids of the live particles
+  if (last_.halt != 0) return RP_OK;
+  const size_t n = (size_t)n_ - (size_t)last_.removed;  // ids of the live particles
   TRY(ensure_io((size_t)std::max(n_, n_upload_)));
   double* vec[8] = {st->position, st->velocity, st->angular_velocity, st->acceleration,
                     st->torque, st->position_residual, st->velocity_residual, st->angular_velocity_residual};
@@ -1495,6 +1511,31 @@ int Engine::fast_read_state(rp_state* st, bool& done) {
     done = true;
     return RP_OK;
   }
+  if (n <= kPinnedParticles) {
+    // a small bed: the gather writes pinned memory and the host copies from it
+    // (five arrays of 1,000 to 4,096 spheres: 37 to 59 us, by device copies into
+    // pageable memory 76 to 78; of 16,384: 158 against 87)
+    if (pin_n_ < n) {
+      if (pin_buf_) cudaFreeHost(pin_buf_);
+      pin_buf_ = nullptr;
+      pin_n_ = 0;
+      const size_t m = (n + 255) & ~size_t(255);
+      CK(cudaMallocHost((void**)&pin_buf_, sizeof(double) * (26 * m + m / 8 + 1)));
+      pin_n_ = m;
+    }
+    const StateIO pin = state_io(pin_buf_, n, vec, st->radius, st->mass, st->fixed);
+    launch_state_gather(P_, ids, pin, (int)n, stream_);
+    CK(cudaStreamSynchronize(stream_));
+    CK(cudaGetLastError());
+    for (int q = 0; q < 8; ++q)
+      if (vec[q]) std::memcpy(vec[q], pin.v[q], sizeof(double) * 3 * n);
+    if (st->radius) std::memcpy(st->radius, pin.radius, sizeof(double) * n);
+    if (st->mass) std::memcpy(st->mass, pin.mass, sizeof(double) * n);
+    if (st->fixed) std::memcpy(st->fixed, pin.fixed, n);
+    st->n_particles = n;
+    done = true;
+    return RP_OK;
+  }
   const StateIO io = state_io(io_buf_, n, vec, st->radius, st->mass, st->fixed);
   launch_state_gather(P_, ids, io, (int)n, stream_);
   for (int q = 0; q < 8; ++q)
@@ -1513,9 +1554,8 @@ int Engine::fast_write_state(const rp_state* st, bool& done) {
   done = false;
   if (!gpu_ || !dev_valid_ || n_ <= 0) return RP_OK;
   CK(cudaSetDevice(device_));
-  TRY(sync_ctrl());
-  if (ctrl_h_->halt != 0) return RP_OK;
-  const size_t n = (size_t)n_ - (size_t)ctrl_h_->removed;  // ids of the live particles
+  if (last_.halt != 0) return RP_OK;
+  const size_t n = (size_t)n_ - (size_t)last_.removed;  // ids of the live particles
   TRY(ensure_io((size_t)std::max(n_, n_upload_)));
   double* const vec[8] = {st->position, st->velocity, st->angular_velocity, st->acceleration,
                           st->torque, st->position_residual, st->velocity_residual, st->angular_velocity_residual};

@@ -65,6 +65,7 @@ class Engine {
   int enable_gpu(int device);
   int step(uint64_t n);
   size_t count();
+  uint64_t overlap_warn_steps() const { return tot_.overlap_steps; }
   int get_vec(size_t id, int which, double out[3]);
   int set_vec(size_t id, int which, const double in[3]);
   int read_state(rp_state* st);
@@ -210,6 +211,12 @@ class Engine {
   int launch_steps(uint64_t n);
   int launch_steps_graph(uint64_t n);
   int build_graph(bool small);
+  int close_kernels_ = 0;    // kernels the graph runs after its loop
+  unsigned long long* lim_h_ = nullptr;  // pinned: target and iters of the next graph launch
+  // pinned staging of small state reads, for the life of the device state
+  static constexpr size_t kPinnedParticles = 4096;  // at most 0.9 MB
+  double* pin_buf_ = nullptr;
+  size_t pin_n_ = 0;
   bool small_loop_ = false;  // the graph's body runs many steps an iteration (k_steps)
   bool small_ok_ = true;     // cooperative launches can be captured
   void destroy_graph();

@@ -951,7 +951,7 @@ __device__ __forceinline__ bool first_half_pass(const StepParams& P, Ctrl* C, co
 }
 
 template <bool KAHAN, bool SPIN>
-__global__ void __launch_bounds__(KAHAN ? 128 : 256, KAHAN ? 5 : 4) k_first_half(StepParams P) {
+__global__ void __launch_bounds__(KAHAN ? 128 : 256, KAHAN ? (SPIN ? 5 : 7) : 5) k_first_half(StepParams P) {
   Ctrl* C = P.ctrl;
   if (C->halt) return;
   if (first_half_pass<KAHAN, SPIN>(P, C, P.bank[C->bank], C->pending != 0, grid_span())) C->rebuild = 1;
@@ -984,11 +984,12 @@ __device__ __forceinline__ void spin_kick(const StepParams& P, const Bank& B, in
 bool spin_in_filter(const StepParams& P) { return P.prec == 0 && P.force_path == 0; }
 
 // Completes the last step of a stepping call (the pending second half);
-// k_clear_pending then marks the state complete. KAHAN as in k_first_half.
+// k_clear_pending then marks the state complete (a call that stopped short of
+// its target goes on first). KAHAN as in k_first_half.
 template <bool KAHAN>
 __global__ void __launch_bounds__(256) k_second_half(StepParams P) {
   Ctrl* C = P.ctrl;
-  if (C->halt || !C->pending) return;
+  if (C->halt || !C->pending || C->steps_done < C->target) return;
   const Bank B = P.bank[C->bank];
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < P.n; k += gridDim.x * blockDim.x) {
     uint32_t fl = B.flags[k];
@@ -2576,7 +2577,8 @@ __global__ void k_steps_next(StepParams P, cudaGraphConditionalHandle rebuild, c
 }
 
 __global__ void k_clear_pending(StepParams P) {
-  if (!P.ctrl->halt) P.ctrl->pending = 0;
+  Ctrl* C = P.ctrl;
+  if (!C->halt && C->steps_done >= C->target) C->pending = 0;
 }
 
 // End of a step: count it and, inside the device step loop, decide whether

@@ -576,6 +576,16 @@ int rp_get_stats(rp_sim* s, rp_stats* out) {
   return s->e->stats(out);
 }
 
+int rp_overlap_warn_steps(rp_sim* s, uint64_t* steps) {
+  SIM_OR_FAIL(s);
+  if (!steps) {
+    set_error("null output");
+    return RP_E_INVALID_ARG;
+  }
+  *steps = s->e->overlap_warn_steps();
+  return RP_OK;
+}
+
 int rp_set_profiling(rp_sim* s, int enable) {
   SIM_OR_FAIL(s);
   s->e->profiling = enable != 0;
