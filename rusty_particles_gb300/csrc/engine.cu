@@ -67,11 +67,23 @@ Law Engine::make_law(const Material& m) const {
   L.mu = m.mu;
   L.jkr_C = (8.0 * kPiH) * L.gamma_pp / L.es_pp;
   L.jkr_Cf = (float)L.jkr_C;
+  // the laws' products of constants, rounded as the laws round them
+  const double four_thirds = 4.0 / 3.0, pull = 1.5 * kPiH;
+  L.es43_pp = four_thirds * L.es_pp;
+  L.es43_pw = four_thirds * L.es_pw;
+  L.es2_pp = 2.0 * L.es_pp;
+  L.es2_pw = 2.0 * L.es_pw;
+  L.pull_pp = pull * L.gamma_pp;
+  L.pull_pw = pull * L.gamma_pw;
   L.es_ppf = (float)L.es_pp;
   L.gs_ppf = (float)L.gs_pp;
   L.gamma_ppf = (float)L.gamma_pp;
   L.beta_absf = (float)L.beta_abs;
   L.muf = (float)L.mu;
+  const float four_thirds_f = (float)(4.0 / 3.0), pull_f = 1.5f * (float)kPiH;
+  L.es43_ppf = four_thirds_f * L.es_ppf;
+  L.es2_ppf = 2.0f * L.es_ppf;
+  L.pull_ppf = pull_f * L.gamma_ppf;
   return L;
 }
 

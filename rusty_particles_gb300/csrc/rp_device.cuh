@@ -72,7 +72,9 @@ struct Law {
   double mu;                   // particle friction, used for pairs and walls (src/simulation.rs:489)
   double jkr_C;                // 8 pi gamma / E* of pairs, as src/physics.rs:165 forms it
   float jkr_Cf;
+  double es43_pp, es2_pp, pull_pp, es43_pw, es2_pw, pull_pw;  // (4/3) E*, 2 E*, 1.5 pi gamma (pair, wall)
   float es_ppf, gs_ppf, gamma_ppf, beta_absf, muf;  // rounded for the FP32 pair law
+  float es43_ppf, es2_ppf, pull_ppf;                // products of the rounded constants, in FP32
 };
 constexpr uint32_t GROUP_ALL = 0xFFFFFFFFu;
 // Ctrl::halt bits: a neighbour list outgrew its capacity (list rebuild), the
