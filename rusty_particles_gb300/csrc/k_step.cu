@@ -58,17 +58,21 @@ __device__ __forceinline__ float plus_zero(float x) { return (__float_as_int(x) 
 
 constexpr double kPi = 3.14159265358979323846;
 
-// float -> double, exactly, on the integer pipe: a normal float's exponent is
-// re-biased (+896) and its mantissa shifted into place; zeros keep their sign.
-// Subnormals, infinities and NaNs take the hardware conversion, which runs on
-// the FP64 pipe like every FP64 instruction.
+// float -> double, exactly, on the integer pipe: the exponent is re-biased
+// (+896) and the mantissa shifted into place; a subnormal's leading one becomes
+// the implicit one. A conversion instruction would run on the FP64 pipe, and
+// costs it an issue slot even where a predicate turns it off.
 __device__ __forceinline__ double f2d_exact(float f) {
   const uint32_t u = __float_as_uint(f);
-  const uint32_t e = (u >> 23) & 0xFFu;
-  if ((u << 1) == 0u) return __longlong_as_double((long long)((uint64_t)u << 32));
-  if (e == 0u || e == 0xFFu) return (double)f;
-  return __longlong_as_double((long long)(((uint64_t)(u & 0x80000000u) << 32) | ((uint64_t)(e + 896u) << 52) |
-                                          ((uint64_t)(u & 0x7FFFFFu) << 29)));
+  uint32_t m = u & 0x7FFFFFFFu, e = 896u << 20;
+  if (m < 0x00800000u) {  // zero or subnormal
+    const uint32_t up = __clz(m) - 8u;
+    m = m ? m << up : 0u;  // (bit 23 adds one to the exponent)
+    e = m ? (896u - up) << 20 : 0u;
+  } else if (m >= 0x7F800000u) {
+    e = (2047u - 255u) << 20;
+  }
+  return __hiloint2double((int)((u & 0x80000000u) | ((m >> 3) + e)), (int)(m << 29));
 }
 
 // -------------------------------------------- FP64 roots and quotients
@@ -1754,7 +1758,12 @@ __global__ void __launch_bounds__(128) k_jkr_mlp(StepParams P) {
 // count times an FP32 value rounds the same in FP32 as in FP64).
 template <typename R>
 __device__ __forceinline__ void put_result(const StepParams& P, uint32_t rec, T3<R> f, T3<R> t, int visits) {
-  if (visits != 1) {  // x * 1 = x: no multiply for the common single visit
+  // x * 1 = x: no multiply for the common single visit. The warp decides: as a
+  // branch of each lane the 7 FP64 instructions became predicated ones, and a
+  // predicated-off FP64 instruction takes the pipe as long as a full one (14 of
+  // ~125 a contact: hopper of 1,048,576 spheres 415 to 379 us in this kernel,
+  // 654 to 630 a step; its spring bed of 524,288 406 to 387).
+  if (__any_sync(__activemask(), visits != 1)) {
     const R s = (R)visits;
     f = f * s;
     t = t * s;
@@ -2000,6 +2009,7 @@ __global__ void __launch_bounds__(128) k_contact_deferred(StepParams P) {
 // changes a result.
 constexpr uint32_t ACC_BINS = 128;
 constexpr uint32_t ACC_TILE = 256;
+constexpr int ACC_DEAL = 256;           // slots a block deals to its threads at a time
 constexpr uint32_t ACC_SORT_BINS = 32;  // record counts up to 31 (more share the last bin)
 
 __device__ __forceinline__ bool tri_cell_nonempty(const StepParams& P, float4 xf) {
@@ -2186,10 +2196,14 @@ __device__ __forceinline__ void sum_particle(const StepParams& P, const Bank& B,
     F = vmk(f2d_exact(fx), f2d_exact(fy), f2d_exact(fz));
     T = vmk(f2d_exact(tx), f2d_exact(ty), f2d_exact(tz));
   } else {
-    // the next record's loads are in flight while this one is added
+    // the next record's loads are in flight while this one is added; one record
+    // a round, because an unrolled loop predicates its remainder, and a
+    // predicated-off FP64 instruction takes the pipe as long as a full one
+    // (million-sphere hopper: 1.25 to 0.98 million warp instructions, 92 to 76 us)
     const double2* res = reinterpret_cast<const double2*>(P.cres + 6 * (size_t)P.coff[k]);
     double2 a0, a1, a2;
     if (n > 0) { a0 = res[0]; a1 = res[1]; a2 = res[2]; }
+#pragma unroll 1
     for (uint32_t c = 0; c < n; ++c) {
       const double2 r0 = a0, r1 = a1, r2 = a2;
       if (c + 1 < n) { a0 = res[3 * c + 3]; a1 = res[3 * c + 4]; a2 = res[3 * c + 5]; }
@@ -2200,6 +2214,7 @@ __device__ __forceinline__ void sum_particle(const StepParams& P, const Bank& B,
   // the wall contacts (FP64 in both forms) after the pair contacts, in mesh order
   if (P.ntri > 0) {
     const uint32_t wn = P.wcnt[k], wo = P.woff[k];
+#pragma unroll 1
     for (uint32_t c = 0; c < wn; ++c) {
       const double2* r = reinterpret_cast<const double2*>(P.wres + 6 * (size_t)(wo + c));
       const bool ok = P.wok[wo + c] != 0;
@@ -2219,24 +2234,30 @@ __global__ void __launch_bounds__(256, 5) k_accumulate(StepParams P) {
   Ctrl* C = P.ctrl;
   if (C->halt) return;
   const Bank B = P.bank[C->bank];
-  // Each block takes a tile of blockDim.x slots (in aorder) and deals them
-  // to its threads by their record and wall counts (a counting sort in shared
-  // memory), so the lanes of a warp run sum loops of about the same length:
-  // a partly filled FP64 warp instruction costs the pipe as much as a full one.
+  // Each block takes a tile of ACC_DEAL slots (in aorder) and deals them to its
+  // threads by their record and wall counts (a counting sort in shared memory),
+  // so the lanes of a warp run sum loops of about the same length: a partly
+  // filled FP64 warp instruction costs the pipe as much as a full one. 256 slots
+  // for 128 threads: 128 left more lanes idle (hopper 656 against 654 us a step,
+  // 2.1 million adhesive spheres 1222 against 1215), 512 and 1024 read farther
+  // apart and end in a thinner last wave (661 and 666; 1218 and 1249).
   __shared__ uint32_t bins[ACC_SORT_BINS];
-  __shared__ int dealt[256];
-  for (int base = blockIdx.x * blockDim.x; base < P.n; base += gridDim.x * blockDim.x) {
-    const int i = base + (int)threadIdx.x;
-    int k = -1;
-    uint32_t key = 0;
-    if (i < P.n) {
-      k = (int)P.aorder[i];
-      if (B.flags[k] & PF_DEAD) k = -1;
-      else key = min(P.ccnt[k] + (P.ntri > 0 ? P.wcnt[k] : 0u), ACC_SORT_BINS - 1);
-    }
+  __shared__ int slot[ACC_DEAL], dealt[ACC_DEAL];
+  __shared__ uint32_t place[ACC_DEAL];  // key, rank among its equals
+  for (int base = blockIdx.x * ACC_DEAL; base < P.n; base += gridDim.x * ACC_DEAL) {
     for (uint32_t b = threadIdx.x; b < ACC_SORT_BINS; b += blockDim.x) bins[b] = 0;
     __syncthreads();
-    const uint32_t rank = atomicAdd(&bins[key], 1u);
+    for (int o = threadIdx.x; o < ACC_DEAL; o += blockDim.x) {
+      int k = -1;
+      uint32_t key = 0;
+      if (base + o < P.n) {
+        k = (int)P.aorder[base + o];
+        if (B.flags[k] & PF_DEAD) k = -1;
+        else key = min(P.ccnt[k] + (P.ntri > 0 ? P.wcnt[k] : 0u), ACC_SORT_BINS - 1);
+      }
+      slot[o] = k;
+      place[o] = key | atomicAdd(&bins[key], 1u) << 8;
+    }
     __syncthreads();
     if (threadIdx.x < 32) {  // exclusive scan of the bins, one per lane
       const uint32_t c0 = bins[threadIdx.x];
@@ -2249,12 +2270,12 @@ __global__ void __launch_bounds__(256, 5) k_accumulate(StepParams P) {
       bins[threadIdx.x] = incl - c0;
     }
     __syncthreads();
-    dealt[bins[key] + rank] = k;
+    for (int o = threadIdx.x; o < ACC_DEAL; o += blockDim.x) dealt[bins[place[o] & 0xFFu] + (place[o] >> 8)] = slot[o];
     __syncthreads();
-    k = dealt[threadIdx.x];
-    __syncthreads();
-    if (k < 0) continue;
-    sum_particle<F32REC>(P, B, C, k);
+    for (int o = threadIdx.x; o < ACC_DEAL; o += blockDim.x) {
+      const int k = dealt[o];
+      if (k >= 0) sum_particle<F32REC>(P, B, C, k);
+    }
   }
 }
 
@@ -2754,8 +2775,8 @@ static int launch_contact_path(const StepParams& P, cudaStream_t s, const SideSt
     cudaStreamWaitEvent(s, side.join, 0);
     ++launched;
   }
-  if (P.prec == 1) k_accumulate<true><<<shaped_grid((uint64_t)P.n, ba, cap), ba, 0, s>>>(P);
-  else k_accumulate<false><<<shaped_grid((uint64_t)P.n, ba, cap), ba, 0, s>>>(P);
+  if (P.prec == 1) k_accumulate<true><<<shaped_grid((uint64_t)P.n, ACC_DEAL, cap), ba, 0, s>>>(P);
+  else k_accumulate<false><<<shaped_grid((uint64_t)P.n, ACC_DEAL, cap), ba, 0, s>>>(P);
   return launched;
 }
 
