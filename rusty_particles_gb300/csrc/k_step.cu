@@ -187,19 +187,34 @@ __device__ __forceinline__ V cross_fma(V a, V b) {
 }
 __device__ __forceinline__ V mad(double s, V a, V b) { return V{fma(s, a.x, b.x), fma(s, a.y, b.y), fma(s, a.z, b.z)}; }
 
-// double -> float, rounded to nearest even, on the integer pipe where the value
-// and its rounding are normal floats (zeros and the rest take the hardware
-// conversion, an FP64-pipe instruction). It pays in the integrator, which that
-// pipe bounds (drum 4.2 M mixed 1.3 %), not in the mixed pair kernel, whose 14
-// conversions a contact cost more as integer instructions (1.2 % on the same
-// bed: it waits for its gathers as well).
+// double -> float, rounded to nearest even, on the integer pipe, for every input
+// (checked on the host against the conversion over 260 million doubles, all
+// exponents around the float range and ties among them). A conversion
+// instruction runs on the FP64 pipe, and takes it as long where a predicate
+// turns it off: leaving the rare inputs to one saved nothing. The mixed pair law
+// narrows 13 values a contact (58 FP64-pipe instructions with conversions),
+// the integrator 3 a particle: the pair kernel of a million-sphere hopper 196 to
+// 171 us, its mixed step 395 to 372, the FP64 step 629 to 623, a gas of a million
+// 259 to 254, a mixed drum of 4.2 million 1346 to 1253.
+__device__ __forceinline__ uint32_t d2f_odd(uint32_t hi, uint32_t lo) {
+  const uint32_t e = hi & 0x7FFFFFFFu;
+  if (e >= 0x47F00000u)  // 2^128 and above, infinity, NaN
+    return e > 0x7FF00000u || (e == 0x7FF00000u && lo != 0u) ? 0x7FFFFFFFu : 0x7F800000u;
+  const uint32_t down = 926u - (e >> 20);  // bits below the unit 2^-149
+  if (down > 54u) return 0u;
+  const unsigned long long m = ((unsigned long long)((e & 0x000FFFFFu) | 0x00100000u) << 32) | lo;
+  return (uint32_t)((m + ((1ull << (down - 1u)) - 1ull) + ((m >> down) & 1ull)) >> down);
+}
+template <typename R> __device__ __forceinline__ R narrow(double x) { return x; }
 __device__ __forceinline__ float d2f_exact(double x) {
   const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x), e = hi & 0x7FFFFFFFu;
-  if (e - 0x38100000u >= 0x47E00000u - 0x38100000u) return (float)x;
   const uint32_t f = ((e - 0x38000000u) << 3) | (lo >> 29);
-  const uint32_t up = ((lo & 0x1FFFFFFFu) + 0x0FFFFFFFu + (f & 1u)) >> 29;
-  return __uint_as_float((f + up) | (hi & 0x80000000u));
+  uint32_t r = f + (((lo & 0x1FFFFFFFu) + 0x0FFFFFFFu + (f & 1u)) >> 29);
+  if (e - 0x38100000u >= 0x47F00000u - 0x38100000u) r = d2f_odd(hi, lo);
+  return __uint_as_float(r | (hi & 0x80000000u));
 }
+template <> __device__ __forceinline__ float narrow<float>(double x) { return d2f_exact(x); }
+template <typename R> __device__ __forceinline__ T3<R> narrow(V a) { return T3<R>{narrow<R>(a.x), narrow<R>(a.y), narrow<R>(a.z)}; }
 // The law's constants in the pair law's precision (the FP32 ones come rounded),
 // with the products that every contact of a group would form again: (4/3) E*,
 // 2 E* and 1.5 pi gamma, each rounded as the laws' own left-to-right product.
@@ -417,7 +432,7 @@ __device__ __forceinline__ R normal_mag(const NormalLaw<R>& N, int model, R over
 template <typename R>
 __device__ __forceinline__ R reduced_mass(int model, double mi, double mj) {
   if (model > 1) return R(0);
-  const R a = (R)mi, b = (R)mj;
+  const R a = narrow<R>(mi), b = narrow<R>(mj);
   return div_rn(a * b, a + b);
 }
 
@@ -504,21 +519,21 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
       // contact radius next to its fold and the damping of a grazing contact
       // are sensitive to it.
       // (r0 is a normal float: widened by its bits; d2 / 2 by its exponent)
-      const uint32_t rb = __float_as_uint(rsqrtf((float)d2));
+      const uint32_t rb = __float_as_uint(rsqrtf(d2f_exact(d2)));
       const double r0 = rb ? __hiloint2double((int)((rb >> 3) + 0x38000000u), (int)(rb << 29)) : 0.0;
       const double half = __hiloint2double(__double2hiint(d2) - 0x00100000, __double2loint(d2));
       const double inv = r0 * (1.5 - half * (r0 * r0));
       ovd = rsum - d2 * inv;
       nd = d * inv;
-      n = cvt<R>(nd);
+      n = narrow<R>(nd);
     } else {
       ovd = rsum - sqrt(d2);
       nd = vmk(0.0, 1.0, 0.0);
       n = t3(R(0), R(1), R(0));
     }
-    overlap = (R)ovd;
+    overlap = narrow<R>(ovd);
   }
-  const R rir = (R)ri, rjr = (R)rj;
+  const R rir = narrow<R>(ri), rjr = narrow<R>(rj);
   if (is_excess(overlap, rir, rjr)) excess = true;
   const T3<R> ra = (-n) * rir;
   const T3<R> rb = n * rjr;
@@ -545,8 +560,8 @@ __device__ __forceinline__ bool pair_contact(const StepParams& P, const Law& L, 
     const V W = wi * ri + wj * rj;
     rvd = (vi - vj) - cross(W, nd);
     const double vnd = dot(rvd, nd);
-    vn = (R)vnd;
-    vt = cvt<R>(rvd - vnd * nd);
+    vn = narrow<R>(vnd);
+    vt = narrow<R>(rvd - vnd * nd);
   }
   const R rs = div_rn(rir * rjr, rir + rjr);
   const NormalLaw<R> N = pair_law<R>(L);
@@ -1857,7 +1872,7 @@ __device__ __forceinline__ bool contact_eval(const StepParams& P, const Bank& B,
           nrm = cvt<R>(nd);
         }
       }
-      if (done || !PHYS) tc2 = cross(nrm * (R)xj4.w, -fc);
+      if (done || !PHYS) tc2 = cross(nrm * narrow<R>(xj4.w), -fc);
     }
     if (deferred) return true;
     if (HIST && m < 64) atomicOr(B.hmask + k, 1ull << m);
