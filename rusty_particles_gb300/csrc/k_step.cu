@@ -2302,7 +2302,7 @@ __global__ void __launch_bounds__(256, 5) k_accumulate(StepParams P) {
 // be rebuilt (the graph runs the chain and launches it again; Ctrl::resume says
 // that the first half of the current step has been done) or a buffer is full.
 // The sums of a step and the first half of the next are one quad's, so no
-// barrier lies between them: 1,000 spheres take 26 us a step.
+// barrier lies between them: 1,000 spheres take 25 us a step.
 // The launch fits the device at once (cooperative); every wait is bounded, and
 // one that runs out halts the simulation with an error.
 constexpr unsigned SMALL_SPINS = 1u << 20;      // ~1 s
