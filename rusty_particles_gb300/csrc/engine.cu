@@ -275,7 +275,7 @@ int Engine::add_triangles(size_t n, const float* v, const float* nrm, uint32_t g
       for (int k = 0; k < 3; ++k) tri_n_.push_back(l > 0 ? (float)(c[k] / l) : 0.f);
     }
   }
-  dev_valid_ = false;
+  config_changed();
   return RP_OK;
 }
 
@@ -321,7 +321,7 @@ int Engine::set_group_material(uint32_t group, const Material& m) {
     gmat_[group] = m;
     gmat_set_[group] = 1;
   }
-  dev_valid_ = false;
+  config_changed();
   return RP_OK;
 }
 
@@ -2049,8 +2049,8 @@ int Engine::jkr_set_network(const float* params, const float* norm, const float*
   std::memcpy(jkr_norm_, norm, sizeof(jkr_norm_));
   std::memcpy(jkr_dom_, domain, sizeof(jkr_dom_));
   jkr_have_net_ = true;
+  config_changed();
   if (gpu_) dfree(mlp_d_);  // re-uploaded with the new weights
-  dev_valid_ = false;
   return RP_OK;
 }
 

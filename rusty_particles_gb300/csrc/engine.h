@@ -90,7 +90,12 @@ class Engine {
   int grown_capacity(unsigned max_count) const {
     return (std::max(cap_ + 8, (int)(max_count * 5 / 4 + 8)) + 3) & ~3;
   }
-  void config_changed() { dev_valid_ = false; }  // forces a fresh upload before the next step
+  // Forces a fresh upload before the next step, from the host's copy of the
+  // state: the device's is brought home first.
+  void config_changed() {
+    if (!host_valid_ && download() != RP_OK) return;
+    dev_valid_ = false;
+  }
   void set_capacity(int c) {
     if (!host_valid_) download();
     free_lists();
