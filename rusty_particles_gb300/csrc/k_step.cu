@@ -1211,7 +1211,7 @@ __device__ __forceinline__ bool pretest_near(const StepParams& P, float4 xi, flo
   const float d2 = fx * fx + fy * fy + fz * fz;
   const float rsum = xi.w + xj.w;
   const float t = fminf(rsum * P.cut_a, rsum + P.cut_b) + margin;
-  return !(d2 > t * t);  // NaN (a removed partner) stays: the exact test drops it
+  return d2 <= t * t;  // a removed partner's mirror is NaN: not near, from either end
 }
 
 // ---------------------------------------------------------------- forces
@@ -1552,6 +1552,9 @@ __device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const 
         for (uint32_t left = near; left; left &= left - 1u) {
           const uint32_t b = (uint32_t)__ffs((int)left) - 1u, m = c0 + b;
           const uint32_t j = __ldg(row + m);
+          // without the pretest a removed partner shows by its flag: its own
+          // row is not walked, so it evaluates nothing for this end
+          if (!P.pretest && (B.flags[j] & PF_DEAD)) continue;
           uint32_t hint = 0u;
           if (P.nmodel >= 3) {  // pairs never cross groups (the lists exclude them)
             const Law lw = law_of(P, B, k);

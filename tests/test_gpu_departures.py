@@ -1,0 +1,84 @@
+"""Spheres that leave while others hold them in their lists.
+
+A sphere that crosses an open face is dropped at once (src/simulation.rs:199-219),
+while the rows of the spheres next to it name it until the lists are rebuilt:
+nothing of it may reach them, whichever of the two has the higher slot.
+
+Positions to 1e-12 m; forces and torques to 1e-9 of a particle's sum of
+contact-force magnitudes (FP64), 1e-5 (mixed, whose pair law is in FP32).
+"""
+import numpy as np
+import pytest
+
+from tests import parity_util as pu
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def rp():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import rusty_particles_gb300 as m
+    return m
+
+
+def _state(x, r, v, w):
+    n = len(x)
+    return {"position": x, "radius": r, "mass": 2500.0 * 4.0 / 3.0 * np.pi * r ** 3, "velocity": v,
+            "angular_velocity": w, "acceleration": np.zeros((n, 3)), "torque": np.zeros((n, 3)),
+            "fixed": np.zeros(n, np.uint8)}
+
+
+def _clusters(seed, lo, hi):
+    """Triples of overlapping spheres straddling the removal bounds of the open faces, moving outward, each triple
+    turned another way, so that a leaving sphere is found before and after its neighbours in the slots."""
+    rng = np.random.default_rng(seed)
+    x, v = [], []
+    for axis, side in [(0, 0), (0, 1), (1, 0), (2, 0), (2, 1)]:
+        bound = lo[axis] - 1.0 if side == 0 else hi[axis] + 1.0
+        out = -1.0 if side == 0 else 1.0
+        for k in range(40):
+            c = np.zeros(3)
+            c[axis] = bound - out * rng.uniform(0.0002, 0.0008)
+            a, b = (axis + 1) % 3, (axis + 2) % 3
+            c[a], c[b] = lo[a] + 0.06 * (k % 8) - 0.02, lo[b] + 0.08 * (k // 8)
+            u = np.linalg.qr(rng.normal(size=(3, 3)))[0]
+            for d in (0.0 * u[0], 0.0185 * u[0], 0.0185 * u[1]):
+                x.append(c + d)
+                vel = rng.normal(0, 0.05, 3)
+                vel[axis] = out * 3.0
+                v.append(vel)
+    x = np.array(x)
+    keep = (x >= lo - 1.0).all(1) & (x[:, [0, 2]] <= hi[[0, 2]] + 1.0).all(1)
+    x, v = x[keep], np.array(v)[keep]
+    return _state(x, np.full(len(x), 0.01), v, rng.normal(0, 1.0, (len(x), 3)))
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("loop", [1, 0], ids=["device_loop", "host_loop"])
+@pytest.mark.parametrize("mode", [0, 1], ids=["parity", "physical"])
+def test_touching_spheres_leave_one_by_one(rp, oracle_mod, mode, loop, precision):
+    lo, hi = np.full(3, -0.2), np.full(3, 0.2)
+    st = _clusters(3, lo, hi)
+    o = pu.oracle_sim(oracle_mod, st, 1e-5, lo, hi, 1, 0, mode=mode)
+    g = pu.gpu_sim(rp, st, 1e-5, lo, hi, 1, 0, mode=mode, precision=precision)
+    g.set_skin(0.01)  # no rebuild after the first within a call
+    g._L.rp_set_device_loop(g._h, loop)
+    n0, tol = len(st["radius"]), 1e-5 if precision else 1e-9
+    # a call's results are those of its last step. Coulomb friction lets two
+    # roundings part, so the mixed form takes single steps, each from the same state
+    for steps in [1] * 24 if precision else (3, 1, 5, 2, 7, 6):
+        o.steps(steps)
+        g.steps(steps)
+        assert g.get_particle_count() == o.get_particle_count()
+        so, sg = o.state(), g.get_state()
+        FS, TS = o.last_force_scale()
+        assert np.all(np.abs(sg["position"] - so["x"]).max(1) <= (1e-9 if precision else 1e-12))
+        assert np.all(np.abs(sg["acceleration"] - so["a"]).max(1) <= tol * (FS / so["m"] + 10.0))
+        assert np.all(np.abs(sg["torque"] - so["tau"]).max(1) <= tol * TS + 1e-25)
+        if precision:
+            o.set_state({"x": sg["position"], "v": sg["velocity"], "a": sg["acceleration"],
+                         "w": sg["angular_velocity"], "tau": sg["torque"]})
+    assert 20 < o.get_particle_count() < n0 - 100
