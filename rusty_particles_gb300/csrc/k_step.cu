@@ -2077,7 +2077,9 @@ __device__ bool wall_far(const StepParams& P, float4 xf) {
 __device__ uint32_t home_flags(const StepParams& P, float4 xf, long long c, float out) {
   const float p[3] = {xf.x, xf.y, xf.z};
   const float reach = (xf.w + P.rmaxf) * P.cut_a + (float)P.skin + P.home_margin;
-  uint32_t f = PF_NOIMAGE | PF_ONECELL;
+  // without the pretest every row entry is a candidate, however far it has
+  // moved: the cells of both decide whether it counts
+  uint32_t f = P.pretest ? PF_NOIMAGE | PF_ONECELL : 0u;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const float lo = (float)P.bmin[a], hi = (float)P.bmax[a];

@@ -82,3 +82,44 @@ def test_touching_spheres_leave_one_by_one(rp, oracle_mod, mode, loop, precision
             o.set_state({"x": sg["position"], "v": sg["velocity"], "a": sg["acceleration"],
                          "w": sg["angular_velocity"], "tau": sg["torque"]})
     assert 20 < o.get_particle_count() < n0 - 100
+
+
+@pytest.mark.parametrize("loop", [1, 0], ids=["device_loop", "host_loop"])
+def test_partner_drops_out_of_the_grid_of_a_thin_bed(rp, oracle_mod, loop):
+    # a periodic length below four cutoffs: the FP32 pretest is off and every
+    # row entry a candidate. In each pair the lower sphere falls through the
+    # open floor, where the reference's grid no longer lists it
+    # (src/grid.rs:18-30), while the upper one keeps it in its row; clusters of
+    # touching spheres in between leave their forces in the same buffers.
+    rng = np.random.default_rng(8)
+    lo, hi = np.array([0.0, 0.0, -0.45]), np.array([0.06, 0.5, 0.45])
+    r, skin = 0.01, 4e-3
+    x, v = [], []
+    for k in range(24):
+        z = -0.32 + 0.0275 * k
+        up = np.array([0.03, 2 * r + skin + rng.uniform(2e-4, 4e-4), z])
+        low = np.array([0.03, rng.uniform(2e-4, 6e-4), z + rng.uniform(-2e-3, 2e-3)])
+        x += [up, low]
+        v += [np.zeros(3), np.array([0.0, -3.0, 0.0])]
+    for k in range(24):
+        c = np.array([0.03, 0.2, -0.32 + 0.0275 * k])
+        for d in ([0, 0, 0], [0.0, 0.0185, 0.0], [0.011, 0.009, 0.0]):
+            x.append(c + d)
+            v.append(rng.normal(0, 0.05, 3))
+    x, v = np.array(x), np.array(v)
+    st = _state(x, np.full(len(x), r), v, rng.normal(0, 1.0, (len(x), 3)))
+    per = (True, False, False)
+    o = pu.oracle_sim(oracle_mod, st, 1e-5, lo, hi, 1, 0, per)
+    g = pu.gpu_sim(rp, st, 1e-5, lo, hi, 1, 0, per)
+    g.set_skin(skin)
+    g._L.rp_set_device_loop(g._h, loop)
+    crossed = False  # while the rows of the first step still stand
+    for step in range(50):
+        o.step()
+        g.step()
+        so, sg = o.state(), g.get_state()
+        FS, _ = o.last_force_scale()
+        assert np.all(np.abs(sg["position"] - so["x"]).max(1) <= 1e-12), step
+        assert np.all(np.abs(sg["acceleration"] - so["a"]).max(1) <= 1e-9 * (FS / so["m"] + 10.0)), step
+        crossed |= bool((so["x"][1:48:2, 1] < 0).any()) and g.stats()["neighbor_rebuilds"] == 1
+    assert crossed and (so["x"][1:48:2, 1] < 0).all()
