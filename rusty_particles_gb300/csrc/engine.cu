@@ -402,7 +402,7 @@ int Engine::alloc_lists(int cap, bool keep_current) {
                            sizeof(uint32_t) * old_cap, n_, cudaMemcpyDeviceToDevice, stream_));
       if (need_hist && old_hist) {
         for (int p = 0; p < 3; ++p)
-          CK(cudaMemcpy2DAsync(nh + (size_t)p * n_ * cap, sizeof(double) * cap, old_hist + (size_t)p * n_ * old_cap,
+          CK(cudaMemcpy2DAsync(nh + (size_t)p * na * cap, sizeof(double) * cap, old_hist + (size_t)p * na * old_cap,
                                sizeof(double) * old_cap, sizeof(double) * old_cap, n_, cudaMemcpyDeviceToDevice,
                                stream_));
       }
@@ -473,6 +473,7 @@ int Engine::ensure_jkr_buffers() {
 
 void Engine::refresh_list_ptrs() {
   P_.cap = cap_;
+  P_.hplane = n_alloc_ * (size_t)cap_;
   P_.bank[0] = bank_[0];
   P_.bank[1] = bank_[1];
   P_.dbgMult = dbgMult_;

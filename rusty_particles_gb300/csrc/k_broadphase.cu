@@ -334,7 +334,7 @@ __global__ void k_build_nlist(StepParams P, const uint32_t* cstart, const uint32
   const int b = P.ctrl->bank;
   const Bank O = P.bank[b], B = P.bank[b ^ 1];
   const float skin = (float)P.skin;
-  const size_t plane_new = (size_t)P.n * P.cap;
+  const size_t plane = P.hplane;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < P.n; k += gridDim.x * blockDim.x) {
     uint32_t* row = B.nbr + (size_t)k * P.cap;
     if (B.flags[k] & PF_DEAD) {
@@ -395,7 +395,6 @@ __global__ void k_build_nlist(StepParams P, const uint32_t* cstart, const uint32
     const uint32_t ok = carry_history ? perm[k] : 0u;
     const uint32_t ocnt = carry_history ? O.ncnt[ok] : 0u;
     const uint32_t* orow = O.nbr + (size_t)ok * P.cap;
-    const size_t plane_old = plane_new;
     for (int zz = 0; zz < no[2]; ++zz)
       for (int yy = 0; yy < no[1]; ++yy)
         for (int xx = 0; xx < no[0]; ++xx) {
@@ -431,14 +430,14 @@ __global__ void k_build_nlist(StepParams P, const uint32_t* cstart, const uint32
                     if (orow[q] == oj) {
                       size_t oi = (size_t)ok * P.cap + q;
                       h0 = O.hist[oi];
-                      h1 = O.hist[plane_old + oi];
-                      h2 = O.hist[2 * plane_old + oi];
+                      h1 = O.hist[plane + oi];
+                      h2 = O.hist[2 * plane + oi];
                       break;
                     }
                   size_t ni = (size_t)k * P.cap + cnt;
                   B.hist[ni] = h0;
-                  B.hist[plane_new + ni] = h1;
-                  B.hist[2 * plane_new + ni] = h2;
+                  B.hist[plane + ni] = h1;
+                  B.hist[2 * plane + ni] = h2;
                   if (cnt < 64 && (__double_as_longlong(h0) | __double_as_longlong(h1) | __double_as_longlong(h2)))
                     hm |= 1ull << cnt;
                 }

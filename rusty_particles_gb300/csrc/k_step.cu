@@ -1226,7 +1226,7 @@ __global__ void __launch_bounds__(128) k_force(StepParams P) {
   if (C->halt) return;
   const Bank B = P.bank[C->bank];
   const bool adh = (P.nmodel == 3 || P.nmodel == 4);
-  const size_t plane = (size_t)P.n * P.cap;
+  const size_t plane = P.hplane;
   const float margin = pretest_margin(P, C);
   bool excess = false;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < P.n; k += gridDim.x * blockDim.x) {
@@ -1482,7 +1482,7 @@ __device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const 
   const bool zdrop_any = P.drop_zero && P.nmodel == 3;
   // the same for sJKR, whose zero region is explicit (no iteration to certify)
   const bool sdrop = P.drop_zero && P.nmodel == 4;
-  const size_t plane = (size_t)P.n * P.cap;
+  const size_t plane = P.hplane;
   const float margin = pretest_margin(P, C);
   const int lane = threadIdx.x & 31;
   const bool kick = !COHERENT && C->spin_due != 0, fuse = C->pending != 0;
@@ -1826,7 +1826,7 @@ __device__ __forceinline__ uint32_t back_record(const StepParams& P, uint32_t j,
 template <bool PHYS, bool HIST, typename R, bool JKR>
 __device__ __forceinline__ bool contact_eval(const StepParams& P, const Bank& B, uint4 it, float guess,
                                              bool can_defer, bool newton, bool& excess, uint32_t* tally) {
-  const size_t plane = (size_t)P.n * P.cap;
+  const size_t plane = P.hplane;
   const bool adh = (P.nmodel == 3 || P.nmodel == 4);
   const uint32_t k = it.x, j = it.y, m = it.z & 0xFFFFu;
   const int vij = (it.z >> 16) & 0xFF, vji = crec_vji(it.z);

@@ -108,7 +108,7 @@ struct Bank {
   float4* xf;       // FP32 mirror of (position, radius) for the pair pretest
   uint32_t* nbr;    // neighbour rows, cap entries per slot
   uint32_t* ncnt;   // row lengths
-  double* hist;     // physical-mode tangential spring per row entry: 3 planes of N*cap
+  double* hist;     // physical-mode tangential spring per row entry: 3 planes of StepParams::hplane
   // physical mode: bit m set when the spring of row entry m (< 64) may hold a
   // value other than +0 (entries past 64 are always treated as live)
   unsigned long long* hmask;
@@ -143,6 +143,7 @@ struct MlpInfer;
 struct StepParams {
   int n;  // slots
   int cap;
+  size_t hplane;   // entries a plane of Bank::hist (allocated slots x cap: stays as slots come and go)
   int force_path;  // 0: contact-parallel (default), 1: one thread per particle
   // launch shapes of the force pass (chosen by the autotuner): threads per
   // block of the filter, pair and accumulate kernels (<= 256), and the

@@ -1,8 +1,10 @@
-"""Spheres that leave while others hold them in their lists.
+"""Spheres that leave (or join) while others hold them in their lists.
 
 A sphere that crosses an open face is dropped at once (src/simulation.rs:199-219),
 while the rows of the spheres next to it name it until the lists are rebuilt:
-nothing of it may reach them, whichever of the two has the higher slot.
+nothing of it may reach them, whichever of the two has the higher slot. Between
+stepping calls the slots are compacted or appended to, and every remaining
+contact keeps its tangential spring (src/contact.rs:4-17).
 
 Positions to 1e-12 m; forces and torques to 1e-9 of a particle's sum of
 contact-force magnitudes (FP64), 1e-5 (mixed, whose pair law is in FP32).
@@ -11,6 +13,7 @@ import numpy as np
 import pytest
 
 from tests import parity_util as pu
+from tests.test_gpu_history import sheared_bed
 
 pytestmark = pytest.mark.gpu
 
@@ -123,3 +126,43 @@ def test_partner_drops_out_of_the_grid_of_a_thin_bed(rp, oracle_mod, loop):
         assert np.all(np.abs(sg["acceleration"] - so["a"]).max(1) <= 1e-9 * (FS / so["m"] + 10.0)), step
         crossed |= bool((so["x"][1:48:2, 1] < 0).any()) and g.stats()["neighbor_rebuilds"] == 1
     assert crossed and (so["x"][1:48:2, 1] < 0).all()
+
+
+@pytest.mark.parametrize("change", ["removal", "insertion", "both"])
+@pytest.mark.parametrize("tangential", [2, 1], ids=["mindlin", "linear_spring"])
+def test_springs_survive_a_change_of_the_bed(rp, oracle_mod, tangential, change):
+    # a sheared bed with loaded springs; between stepping calls some spheres
+    # have left it (the slots are compacted) or join it (appended)
+    lo, hi = (-0.25, -0.25, -0.25), (0.25, 0.25, 0.25)
+    st = sheared_bed(71 + tangential, 1900, lo, hi)
+    if change != "insertion":
+        out = np.random.default_rng(2).choice(1900, 9, replace=False)
+        st["position"][out] = np.stack([np.full(9, 1.2499), np.linspace(-0.2, 0.2, 9), np.linspace(-0.2, 0.2, 9)], 1)
+        st["velocity"][out] = np.stack([np.linspace(0.3, 3.0, 9), np.zeros(9), np.zeros(9)], 1)  # one after the other
+    dt = 1e-5
+    o = pu.oracle_sim(oracle_mod, st, dt, lo, hi, 1, tangential, mode=1)
+    g = pu.gpu_sim(rp, st, dt, lo, hi, 1, tangential, mode=1)
+    g.set_skin(3e-5)  # rebuilds every few steps
+    inserted = 0
+    for call in range(12):
+        o.steps(4)
+        g.steps(4)
+        assert g.get_particle_count() == o.get_particle_count()
+        so, sg = o.state(), g.get_state()
+        assert float(np.max(np.abs(sg["position"] - so["x"]))) <= 1e-12, call
+        FS, TS = o.last_force_scale()
+        To = so["tau"]
+        assert np.all(np.abs(sg["acceleration"] - so["a"]).max(1) <= 1e-9 * (FS / so["m"] + 10.0)), call
+        assert np.all(np.abs(sg["torque"] - To).max(1) <= 1e-9 * TS + 1e-25), call
+        assert np.count_nonzero(np.linalg.norm(To, axis=1) > 1e-6 * TS) > 400  # loaded springs
+        if change != "removal" and call % 4 == 1:
+            p = np.array([[0.5, 0.1 * inserted, 0.0]])  # away from the bed
+            g.add_particles(p, np.array([0.009]), np.array([0.008]))
+            o.add_particle(p[0, 0], p[0, 1], p[0, 2], 0.009, 0.008)
+            inserted += 1
+    s = g.stats()
+    assert s["state_uploads"] == 1
+    if change != "insertion":
+        assert s["compactions"] >= 2 and s["removed"] >= 5
+    if change != "removal":
+        assert s["device_inserts"] == inserted == 3
