@@ -385,7 +385,8 @@ int Engine::alloc_walls(size_t cap) {
 int Engine::alloc_lists(int cap, bool keep_current) {
   const bool need_hist = (mode == RP_MODE_PHYSICAL && tmodel != RP_TANGENTIAL_COULOMB);
   const size_t na = n_alloc_;
-  const int cur = keep_current ? last_.bank : 0;
+  // (the bank of the last rebuild: a call that halted may have flipped it since last_)
+  const int cur = keep_current ? ctrl_h_->bank : 0;
   uint32_t* old_nbr = keep_current ? bank_[cur].nbr : nullptr;
   double* old_hist = keep_current ? bank_[cur].hist : nullptr;
   const int old_cap = cap_;
