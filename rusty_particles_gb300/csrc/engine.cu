@@ -1282,6 +1282,7 @@ int Engine::step(uint64_t n) {
     return RP_OK;
   }
   host_valid_ = false;
+  rec_kept_ = false;
   int r = (use_graph_ && !profiling) ? launch_steps_graph(n) : launch_steps(n);
   if (r != RP_OK) return r;
   if (last_.pending) {  // the host issued the last step (a graph ends with this itself)
@@ -1290,7 +1291,10 @@ int Engine::step(uint64_t n) {
     TRY(sync_ctrl());
     last_.pending = ctrl_h_->pending;
   }
-  if (last_.removed > 0) TRY(compact_removed());
+  if (last_.removed > 0) {
+    if (debug) TRY(keep_recording());
+    TRY(compact_removed());
+  }
   return RP_OK;
 }
 
@@ -1727,10 +1731,29 @@ int Engine::bed_statistics(double out[3]) {
 }
 
 // ------------------------------------------------------------ diagnostics
+int Engine::keep_recording() {
+  size_t n = count(), np = 0;
+  rec_f_.resize(3 * n);
+  rec_t_.resize(3 * n);
+  TRY(debug_forces(rec_f_.data(), rec_t_.data()));
+  TRY(debug_pairs(nullptr, nullptr, nullptr, 0, &np));
+  rec_i_.resize(np);
+  rec_j_.resize(np);
+  rec_v_.resize(np);
+  TRY(debug_pairs(rec_i_.data(), rec_j_.data(), rec_v_.data(), np, &np));
+  rec_kept_ = true;
+  return RP_OK;
+}
+
 int Engine::debug_forces(double* F, double* T) {
   if (!gpu_ || !debug) {
     set_error("debug recording is off (call rp_set_debug before stepping)");
     return RP_E_INVALID_ARG;
+  }
+  if (rec_kept_) {
+    std::copy(rec_f_.begin(), rec_f_.end(), F);
+    std::copy(rec_t_.begin(), rec_t_.end(), T);
+    return RP_OK;
   }
   TRY(sync_ctrl());
   const Bank& B = bank_[ctrl_h_->bank];
@@ -1761,6 +1784,16 @@ int Engine::debug_pairs(int64_t* pi, int64_t* pj, int32_t* visits, size_t capaci
   if (!gpu_ || !debug || !dbgMult_) {
     set_error("debug recording is off (call rp_set_debug before stepping)");
     return RP_E_INVALID_ARG;
+  }
+  if (rec_kept_) {
+    const size_t m = std::min(capacity, rec_i_.size());
+    if (pi) {
+      std::copy_n(rec_i_.begin(), m, pi);
+      std::copy_n(rec_j_.begin(), m, pj);
+      std::copy_n(rec_v_.begin(), m, visits);
+    }
+    *nout = rec_i_.size();
+    return RP_OK;
   }
   TRY(sync_ctrl());
   const Bank& B = bank_[ctrl_h_->bank];

@@ -193,6 +193,13 @@ class Engine {
   int compact_removed();
   int append_on_device(size_t n, const double* xyz, const double* r, const double* m, const uint8_t* fixed,
                        bool& done);
+  // debug recording of a call that removed particles, by id: taken before the
+  // compaction moves the slots, dropped by the next stepping call
+  bool rec_kept_ = false;
+  std::vector<double> rec_f_, rec_t_;
+  std::vector<int64_t> rec_i_, rec_j_;
+  std::vector<int32_t> rec_v_;
+  int keep_recording();
   int n_upload_ = 0;          // upload positions (device tags index them); > n_ after compactions
   double rmax_dev_ = 0.0;     // largest radius of the uploaded set (sizes the grids)
   uint64_t uploads_ = 0, downloads_ = 0, compactions_ = 0, device_inserts_ = 0;

@@ -166,3 +166,29 @@ def test_springs_survive_a_change_of_the_bed(rp, oracle_mod, tangential, change)
         assert s["compactions"] >= 2 and s["removed"] >= 5
     if change != "removal":
         assert s["device_inserts"] == inserted == 3
+
+
+def test_diagnostics_of_a_call_that_removed_spheres(rp, oracle_mod):
+    # forces and contact pairs of the last step in the ids of the spheres that
+    # remain (removals are compacted when the call ends, which moves the slots)
+    lo, hi = (-0.2, -0.2, -0.2), (0.2, 0.2, 0.2)
+    st = pu.random_bed(53, 1500, lo, hi, 0.008, 0.012, ascale=0.0)
+    out = np.arange(0, 1500, 50)
+    st["position"][out, 0] = 1.19999
+    st["velocity"][out, 0] = np.linspace(0.5, 3.0, len(out))
+    o = pu.oracle_sim(oracle_mod, st, 1e-5, lo, hi, 1, 0)
+    g = pu.gpu_sim(rp, st, 1e-5, lo, hi, 1, 0)
+    for steps in (2, 1, 1):
+        n0 = o.get_particle_count()
+        o.steps(steps)
+        g.steps(steps)
+        assert g.get_particle_count() == o.get_particle_count()
+        Fo, To = o.last_forces()
+        Fg, Tg = g.debug_forces()
+        FS, TS = o.last_force_scale()
+        assert len(Fg) == len(Fo)
+        assert np.all(np.linalg.norm(Fg - Fo, axis=1) <= 1e-9 * FS)
+        assert np.all(np.linalg.norm(Tg - To, axis=1) <= 1e-9 * TS + 1e-25)
+        assert pu.pair_counter_gpu(g) == pu.pair_counter_oracle(o)
+        assert o.get_particle_count() < n0 or steps == 1
+    assert g.stats()["compactions"] >= 1
