@@ -173,13 +173,17 @@ __device__ __forceinline__ double relu(double x) {
   return b > 0 && b <= 0x7FF0000000000000ll ? x : 0.0;
 }
 __device__ __forceinline__ float relu(float x) { return fmax(x, 0.0f); }
-// a < b for a >= 0 or NaN (false) and b >= 0
+// a < b for a >= 0 or NaN (false, whichever its sign: inf - inf has it set) and
+// b >= 0. As unsigned words, a NaN of either sign lies above infinity.
 __device__ __forceinline__ bool less_nn(double a, double b) {
-  return __double_as_longlong(a) < __double_as_longlong(b);
+  return (unsigned long long)__double_as_longlong(a) < (unsigned long long)__double_as_longlong(b);
 }
 __device__ __forceinline__ bool less_nn(float a, float b) { return a < b; }
-// x <= 0 (false for a NaN with a clear sign bit, as the comparison)
-__device__ __forceinline__ bool not_positive(double x) { return __double_as_longlong(x) <= 0; }
+// x <= 0 (false for NaN)
+__device__ __forceinline__ bool not_positive(double x) {
+  const long long b = __double_as_longlong(x);
+  return b <= 0 && (unsigned long long)b <= 0xFFF0000000000000ull;
+}
 __device__ __forceinline__ bool not_positive(float x) { return x <= 0.0f; }
 // whether an overlap exceeds 0.2 min(r_i, r_j); below an eighth of both radii
 // the exponents decide it

@@ -10,6 +10,8 @@ lies closest to a rounding boundary, built with integers:
 * reciprocals of a root s: s m = 2^106 - r for an odd m and a small r;
 * roots: (M + 1/2)^2 = M^2 + M + 1/4, so the 53-bit numbers M^2 + M + j with a
   small even j are the ones whose root lies next to a midpoint.
+
+Comparisons stand for the floating ones, which are false for a NaN of either sign.
 """
 import ctypes
 import os
@@ -177,3 +179,20 @@ def test_conversions(probe):
     with np.errstate(all="ignore"):
         want = f.astype(np.float64)
     _same(probe(7, u.astype(U)), want, f)
+
+
+def test_comparisons(probe):
+    rng = np.random.default_rng(4)
+    a = np.concatenate([_doubles(rng, 100_000), SPECIAL])
+    with np.errstate(all="ignore"):
+        np.testing.assert_array_equal(probe(9, a) != 0, a <= 0)  # false for a NaN of either sign
+        np.testing.assert_array_equal(_bits(probe(10, a)), _bits(np.where(a > 0, a, 0.0)))
+        np.testing.assert_array_equal(probe(11, a) != 0, np.isfinite(a))
+        _same(probe(12, a), np.where(a == 0, 0.0, a), a)
+        # a >= 0 or NaN against b >= 0
+        x = rng.permutation(np.abs(a[~np.isnan(a)]))
+        y = rng.permutation(x)
+        x[:8] = np.tile(SPECIAL[np.isnan(SPECIAL)], 2)
+        y[:8] = [0.0, 1.0, np.inf, 1e-8, 1e-300, 5e-324, 1e300, 2.0]
+        x[8:2000] = y[8:2000]
+        np.testing.assert_array_equal(probe(8, x, y) != 0, x < y)
