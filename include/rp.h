@@ -108,6 +108,7 @@ typedef struct rp_stats {
 #define RP_STATUS_NAN_FORCE 2u  /* a non-finite particle force */
 #define RP_STATUS_NLIST_GROW 4u /* a neighbour list outgrew its capacity (recovered) */
 #define RP_STATUS_WALL_GROW 8u  /* the wall contact candidates outgrew their buffer (recovered) */
+#define RP_STATUS_STUCK 16u     /* the blocks of a small bed's step loop did not meet in time (the call fails) */
 
 /* --- lifecycle: Simulation.create (src/lib.rs:57, src/simulation.rs:62-91) */
 rp_sim* rp_create(double dt, const double min_xyz[3], const double max_xyz[3], size_t particle_capacity);
@@ -210,6 +211,10 @@ int rp_measure_fp64_peak(double* fma_per_s, double* add_per_s);
 /* --- diagnostics for parity checks (no reference counterpart) */
 /* Record per-particle force/torque and contact multiplicities during steps. */
 int rp_set_debug(rp_sim* sim, int enable);
+/* The step loop of small beds waits at its barriers for this many blocks more
+ * than it has (0: none): its bounded wait runs out and the call returns
+ * RP_E_DEVICE_FLAG, as it would if blocks were not running together. */
+int rp_debug_absent_blocks(rp_sim* sim, int blocks);
 /* Per-particle (f_total, torque_total) of the last step, before division by
  * mass (src/simulation.rs:317-526), in id order; 3N doubles each. */
 int rp_debug_last_forces(rp_sim* sim, double* force, double* torque);

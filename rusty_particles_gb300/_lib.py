@@ -165,6 +165,7 @@ SIGNATURES = {
     "rp_last_error": (ctypes.c_char_p, []),
     "rp_version": (ctypes.c_char_p, []),
     "rp_set_debug": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
+    "rp_debug_absent_blocks": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     "rp_debug_last_forces": (ctypes.c_int, [ctypes.c_void_p, _dp, _dp]),
     "rp_debug_contact_pairs": (ctypes.c_int, [ctypes.c_void_p, _i64p, _i64p, _i32p, ctypes.c_size_t,
                                               ctypes.POINTER(ctypes.c_size_t)]),

@@ -504,6 +504,7 @@ int Engine::build_params() {
   P.mode = mode;
   P.prec = prec;
   P.debug = debug;
+  P.absent_blocks = absent_blocks;
   P.dt = dt;
   for (int k = 0; k < 3; ++k) {
     P.periodic[k] = periodic[k] ? 1 : 0;
@@ -1231,6 +1232,8 @@ int Engine::launch_steps(uint64_t n) {
     }
   }
   uint64_t remaining = n;
+  lim_h_[0] = last_.steps_done + n;  // the closing second half waits for it
+  CK(cudaMemcpyAsync(&ctrl_->target, lim_h_, sizeof(unsigned long long), cudaMemcpyHostToDevice, stream_));
   while (remaining > 0) {
     const uint64_t chunk = std::min(remaining, CHUNK);
     const uint64_t before = last_.steps_done;
@@ -1284,7 +1287,12 @@ int Engine::step(uint64_t n) {
   host_valid_ = false;
   rec_kept_ = false;
   int r = (use_graph_ && !profiling) ? launch_steps_graph(n) : launch_steps(n);
-  if (r != RP_OK) return r;
+  if (r != RP_OK) {
+    // the halt and the particles that this call has lost count for what reads
+    // the state next (it goes over the host then)
+    if (sync_ctrl() == RP_OK) finish_step_accounting();
+    return r;
+  }
   if (last_.pending) {  // the host issued the last step (a graph ends with this itself)
     launches_ += launch_second_half(P_, stream_);
     CK(cudaGetLastError());

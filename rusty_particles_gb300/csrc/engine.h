@@ -45,6 +45,7 @@ class Engine {
   double href = 1.0;
   double skin_user = -1.0;
   int debug = 0;
+  int absent_blocks = 0;  // see StepParams
   int profiling = 0;
   int force_path = 0;  // 0 contact-parallel, 1 one thread per particle
 

@@ -2143,14 +2143,14 @@ __device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
   return v;
 }
 
-// All blocks of the launch; `gen` counts the barriers passed. False when the
-// others did not arrive in time.
-__device__ __forceinline__ bool grid_barrier(Ctrl* C, unsigned& gen) {
+// All blocks of the launch (`blocks`); `gen` counts the barriers passed. False
+// when the others did not arrive in time.
+__device__ __forceinline__ bool grid_barrier(Ctrl* C, unsigned& gen, unsigned blocks) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     ++gen;
-    const unsigned want = gen * gridDim.x;
+    const unsigned want = gen * blocks;
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&C->bar), "r"(1u) : "memory");
     bool here = load_acquire(&C->bar) >= want;
     for (unsigned n = 0; !here && n < SMALL_SPINS; ++n) here = load_acquire(&C->bar) >= want;
@@ -2368,6 +2368,7 @@ __global__ void __launch_bounds__(SMALL_BLOCK, 1) k_steps(StepParams P) {
   const Span sp{(int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + lane, (int)(gridDim.x * blockDim.x)};
   const int quad0 = (sp.at - lane) >> 2, quad_all = sp.all >> 2;  // of the warp
   unsigned gen = 0;
+  const unsigned blocks = gridDim.x + (unsigned)P.absent_blocks;
   for (unsigned s = 0; s < SMALL_STEPS && done < target; ++s) {
     uint32_t* ctot = P.ctot + (s & 1u) * CTOT_WORDS;
     if (!resume) {
@@ -2381,7 +2382,7 @@ __global__ void __launch_bounds__(SMALL_BLOCK, 1) k_steps(StepParams P) {
         rebuild = first_half_pass<FP64, true>(P, C, B, fuse, sp);
       }
       if (rebuild) W->rebuild = 1;
-      if (!grid_barrier(C, gen)) return;
+      if (!grid_barrier(C, gen, blocks)) return;
       if (W->rebuild) {
         if (first) W->resume = 1;
         return;
@@ -2389,7 +2390,7 @@ __global__ void __launch_bounds__(SMALL_BLOCK, 1) k_steps(StepParams P) {
     }
     resume = false;
     filter_pass<PHYS, HIST, true>(P, C, B, ctot, sp);
-    if (!grid_barrier(C, gen)) return;
+    if (!grid_barrier(C, gen, blocks)) return;
     if (W->halt) {  // the wall candidates outgrew their buffer: the host finishes this step
       if (first) W->resume = 0;
       return;
@@ -2397,7 +2398,7 @@ __global__ void __launch_bounds__(SMALL_BLOCK, 1) k_steps(StepParams P) {
     contact_pass<PHYS, HIST, R, false>(P, C, B, ctot, sp);
     // the next step's counters, last read two barriers ago
     if (blockIdx.x == 0 && threadIdx.x < CTOT_WORDS) P.ctot[((s + 1u) & 1u) * CTOT_WORDS + threadIdx.x] = 0u;
-    if (!grid_barrier(C, gen)) return;
+    if (!grid_barrier(C, gen, blocks)) return;
     if (quads) {
       for (int b = quad0; b < P.n; b += quad_all) {
         const int k = b + (lane >> 2);

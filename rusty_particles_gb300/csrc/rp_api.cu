@@ -601,6 +601,16 @@ int rp_set_debug(rp_sim* s, int enable) {
   s->e->config_changed();
   return RP_OK;
 }
+int rp_debug_absent_blocks(rp_sim* s, int blocks) {
+  SIM_OR_FAIL(s);
+  if (blocks < 0 || blocks > 1024) {
+    set_error("absent blocks must be in [0, 1024]");
+    return RP_E_INVALID_ARG;
+  }
+  s->e->absent_blocks = blocks;
+  s->e->config_changed();
+  return RP_OK;
+}
 int rp_debug_last_forces(rp_sim* s, double* force, double* torque) {
   SIM_OR_FAIL(s);
   if (!force || !torque) {

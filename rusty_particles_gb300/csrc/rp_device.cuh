@@ -150,6 +150,7 @@ struct StepParams {
   // largest grid of their grid-stride loops
   int bs_filter, bs_force, bs_accum, grid_cap;
   int nsm;  // multiprocessors of the device (sizes the default grids)
+  int absent_blocks;  // diagnostics: blocks that k_steps's barriers wait for beyond those launched
   // contact-parallel buffers (recomputed every step)
   CRec* crec;       // n*cap records, row k at k*cap
   uint32_t* ccnt;   // records per particle
