@@ -80,12 +80,10 @@ __device__ __forceinline__ double f2d_exact(float f) {
 //   starts with five ones; every upper word measured, the lower one is not read),
 //   so y is within 0.5 + 2^52 seed^3 = 0.5045 (0.5036) ulp of 1/b and q + r y
 //   within 2^-51 ulp of a/b. It can round the wrong way only with a midpoint that
-//   close, which is half or three halves of an ulp from q. At half an ulp
-//   |r| / b is a power of two to 2^-50, so the upper mantissas of r and b agree to
-//   one; three halves need a y, and so the mantissas of a and b, above 1.985.
-//   Those go to the library; without that, 28 of 8 million operands built to lie
-//   next to a midpoint came out an ulp off. The test costs the reference's JKR
-//   Newton (four quotients a round) 2 %, the Hertz beds nothing measurable.
+//   close, which is half or three halves of an ulp from q; three halves need a
+//   y, and so the mantissas of a and b, above 1.985. Such quotients go to the
+//   library; without that, 28 of 8 million operands built to lie next to a
+//   midpoint came out an ulp off.
 // * Reciprocal of the root: one correction from within two ulp misses 1/s only
 //   where s m = 2^106 - 1 for a 54-bit m, that is for s = 2 - 2^-52 and its
 //   multiples by powers of two, which go to the library.
@@ -125,28 +123,34 @@ __device__ __forceinline__ double sqrt_rn(double x) {
 __device__ __forceinline__ float sqrt_rn(float x) { return sqrt(x); }
 // sqrt(x) and the rounded 1/sqrt(x) of that rounded root
 __device__ __forceinline__ double sqrt_rn(double x, double& inv) {
-  if (!exponent_in(x, EXP_LO, EXP_HI)) {
+  // (the roots that round to s = 2 - 2^-52 are those of the last two x below a power of four)
+  if (!exponent_in(x, EXP_LO, EXP_HI) || (uint32_t)__double2loint(x) >= 0xFFFFFFFCu) {
     const double s = sqrt(x);
     inv = 1.0 / s;
     return s;
   }
   double y;
   const double s = sqrt_step(x, y);
-  if (__double2loint(s) == -1) inv = 1.0 / s;
-  else inv = fma(y, fma(-s, y, 1.0), y);
+  inv = fma(y, fma(-s, y, 1.0), y);
   return s;
 }
-// whether the corrected quotient of a and b, r = a - b q, may lie next to a midpoint
-__device__ __forceinline__ bool near_midpoint(double a, double b, double r) {
-  return ((__double2hiint(r) - __double2hiint(b) + 1) & 0x000FFFFF) < 3 ||
-         (__double2hiint(a) & __double2hiint(b) & 0x000FC000) == 0x000FC000;
+// Whether the corrected quotient of a and b may lie next to a midpoint (q before
+// the correction, r = a - b q): |r| = b ulp(q) / 2 to one unit of the upper word,
+// or three times that. (|r| = b ulp(q), an exact quotient missed by one, is common
+// where a wall's normal is formed along an axis: taken for a midpoint it cost a
+// bed of 1,000 spheres 25.1 -> 27.0 us a step.)
+__device__ __forceinline__ bool near_midpoint(double a, double b, double q, double r) {
+  const uint32_t hr = (uint32_t)__double2hiint(r) & 0x7FFFFFFFu, hb = (uint32_t)__double2hiint(b) & 0x7FFFFFFFu,
+                 ha = (uint32_t)__double2hiint(a), eq = (uint32_t)__double2hiint(q) & 0x7FF00000u;
+  return hr - hb - eq + (1076u << 20) + 1u < 3u ||
+         ((ha & hb & 0x000FC000u) == 0x000FC000u && (hr & 0x7FF00000u) + (52u << 20) >= (ha & 0x7FF00000u));
 }
 __device__ __forceinline__ double div_rn(double a, double b) {
   if (!(exponent_in(fabs(a), QUOT_LO, QUOT_HI) && exponent_in(fabs(b), QUOT_LO, QUOT_HI))) return a / b;
   const double y = rcp_step(b);
   const double q = a * y;
   const double r = fma(-b, q, a);
-  if (near_midpoint(a, b, r)) return a / b;
+  if (near_midpoint(a, b, q, r)) return a / b;
   return fma(r, y, q);
 }
 __device__ __forceinline__ float div_rn(float a, float b) { return a / b; }
@@ -161,7 +165,7 @@ __device__ __forceinline__ V div_rn(V a, double b) {
   const double y = rcp_step(b);
   const V q = vmk(a.x * y, a.y * y, a.z * y);
   const V r = vmk(fma(-b, q.x, a.x), fma(-b, q.y, a.y), fma(-b, q.z, a.z));
-  if (near_midpoint(a.x, b, r.x) || near_midpoint(a.y, b, r.y) || near_midpoint(a.z, b, r.z)) return a / b;
+  if (near_midpoint(a.x, b, q.x, r.x) || near_midpoint(a.y, b, q.y, r.y) || near_midpoint(a.z, b, q.z, r.z)) return a / b;
   return vmk(zx ? a.x : fma(r.x, y, q.x), zy ? a.y : fma(r.y, y, q.y), zz ? a.z : fma(r.z, y, q.z));
 }
 // Comparisons of FP64 values as integers, off the FP64 pipe (a comparison
