@@ -1357,15 +1357,15 @@ __device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const 
           }
           near &= valid;
         } else {
-          near = valid;
+          // a removed partner shows by its flag: its own row is not walked, so
+          // it evaluates nothing for this end
+          for (uint32_t m = 0; m < ce; ++m)
+            if (!(B.flags[__ldg(row + c0 + m)] & PF_DEAD)) near |= 1u << m;
         }
         uint32_t kept = 0u;
         for (uint32_t left = near; left; left &= left - 1u) {
           const uint32_t b = (uint32_t)__ffs((int)left) - 1u, m = c0 + b;
           const uint32_t j = __ldg(row + m);
-          // without the pretest a removed partner shows by its flag: its own
-          // row is not walked, so it evaluates nothing for this end
-          if (!P.pretest && (B.flags[j] & PF_DEAD)) continue;
           uint32_t hint = 0u;
           if (P.nmodel >= 3) {  // pairs never cross groups (the lists exclude them)
             const Law lw = law_of(P, B, k);
