@@ -657,6 +657,13 @@ int Engine::build_params() {
     for (int k = 0; k < 3; ++k) lm = std::max(lm, P.bsize[k]);
     P.home_margin = (float)(2e-6 * (xb + lm + 4.0 * rmax * adh + href));
   }
+  {
+    double bmag = 0.0;
+    for (int k = 0; k < 3; ++k) bmag = std::max(bmag, std::max(std::fabs(bmin[k]), std::fabs(bmax[k])));
+    const double gap = 2.0 * (2.0 * rmax * adh + skin), out = bmag + (double)P.lmax + 2.0 * gap;
+    P.xhome = (float)(bmag + gap);
+    P.xnear = (float)(out + 2e-6 * (out + gap));  // (twice the margin there on top)
+  }
   P.xbound = (float)xb;
   P.fncells = (uint32_t)((uint64_t)P.fdims[0] * P.fdims[1] * P.fdims[2]);
   rb_.key_bits = bits_for(P.fncells);

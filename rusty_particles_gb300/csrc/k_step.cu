@@ -1006,11 +1006,20 @@ __device__ __forceinline__ void wall_forces(const StepParams& P, const Law& L, u
 // the largest coordinate, L the largest periodic length), so d2f <= cut^2 +
 // 3.47 e cut + 3 e^2 + 12 u cut^2 there; (cut + m)^2 with m = 2.1 e + 1e-6 cut
 // lies above that, and a pair beyond it is certainly outside the exact FP64
-// test. One margin for all pairs (the largest X and cut) keeps the test short
-// and symmetric bit for bit, so both ends keep a pair or drop it together.
-__device__ __forceinline__ float pretest_margin(const StepParams& P, const Ctrl* C) {
-  const float X = __uint_as_float(C->xmax);
+// test. Both ends must keep a pair or drop it together, so the margin is the
+// same bit for bit at both: one for all pairs, from the largest |coordinate|
+// seen but at most StepParams::xnear, and for pairs of two spheres outside
+// StepParams::xhome the pair's own as well. A sphere inside xhome
+// and one beyond xnear are no pair, image or not, so a sphere that has flown
+// off widens nothing but its own pairs (with the largest coordinate alone, one
+// sphere 10,000 km above a hopper of 524,288 made every row entry a candidate:
+// 613 us a step against 352 without it; 356 now).
+__device__ __forceinline__ float margin_at(const StepParams& P, float X) {
   return 2.1f * (6.0e-8f * (2.0f * X + 2.0f * P.cutmaxf + P.lmax)) + 1.0e-6f * P.cutmaxf;
+}
+__device__ __forceinline__ float largest(float4 x) { return fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fabsf(x.z)); }
+__device__ __forceinline__ float pretest_margin(const StepParams& P, const Ctrl* C) {
+  return margin_at(P, fminf(__uint_as_float(C->xmax), P.xnear));
 }
 __device__ __forceinline__ bool pretest_near(const StepParams& P, float4 xi, float4 xj, bool image, float margin) {
   float fx = xi.x - xj.x, fy = xi.y - xj.y, fz = xi.z - xj.z;
@@ -1023,6 +1032,12 @@ __device__ __forceinline__ bool pretest_near(const StepParams& P, float4 xi, flo
   const float rsum = xi.w + xj.w;
   const float t = fminf(rsum * P.cut_a, rsum + P.cut_b) + margin;
   return d2 <= t * t;  // a removed partner's mirror is NaN: not near, from either end
+}
+// the same for a sphere xi outside xhome, with the pair's own margin (its rows
+// are walked again with this one, so that the others' loop stays as it is)
+__device__ __forceinline__ bool pretest_far_near(const StepParams& P, float4 xi, float4 xj) {
+  const float X = largest(xj);
+  return X > P.xhome && pretest_near(P, xi, xj, true, margin_at(P, fmaxf(largest(xi), X)));
 }
 
 // ---------------------------------------------------------------- forces
@@ -1054,10 +1069,12 @@ __global__ void __launch_bounds__(128) k_force(StepParams P) {
     const uint32_t* row = B.nbr + (size_t)k * P.cap;
     unsigned long long hm = 0ull;  // springs this row writes (the live-spring mask)
     const float4 xif = B.xf[k];
+    const bool far = largest(xif) > P.xhome;
     for (uint32_t m = 0; m < cnt; ++m) {
       const uint32_t j = row[m];
       if (P.pretest) {
-        if (!pretest_near(P, xif, B.xf[j], true, margin)) {
+        const float4 xjf = B.xf[j];
+        if (!pretest_near(P, xif, xjf, true, margin) && !(far && pretest_far_near(P, xif, xjf))) {
           const size_t hi = (size_t)k * P.cap + m;
           if (HIST) {
             B.hist[hi] = 0.0;
@@ -1315,6 +1332,7 @@ __device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const 
       const int same_c = !PHYS && !onecell && ref_inside(P, ci) ? same : 0;
       xif = B.xf[k];
       const bool image = !(flk & PF_NOIMAGE);
+      Xi = largest(xif);
       const uint32_t cnt = B.ncnt[k];
       const uint32_t* row = B.nbr + (size_t)k * P.cap;
       CRec* out = P.crec + (size_t)k * P.cap;
@@ -1355,6 +1373,11 @@ __device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const 
                                (pretest_near(P, xif, x3, image, margin) ? 8u : 0u);
             near |= q << m;
           }
+          if (Xi > P.xhome) {
+#pragma unroll 1
+            for (uint32_t m = 0; m < ce; ++m)
+              if (pretest_far_near(P, xif, load_xf<COHERENT>(B.xf + __ldg(row + c0 + m)))) near |= 1u << m;
+          }
           near &= valid;
         } else {
           // a removed partner shows by its flag: its own row is not walked, so
@@ -1370,7 +1393,6 @@ __device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const 
           if (P.nmodel >= 3) {  // pairs never cross groups (the lists exclude them)
             const Law lw = law_of(P, B, k);
             const float4 xjf = load_xf<COHERENT>(B.xf + j);
-            Xi = fmaxf(fmaxf(fabsf(xif.x), fabsf(xif.y)), fabsf(xif.z));
             const bool adhesive = lw.gamma_pp > 0.0;
             if (zdrop_any && adhesive && jkr_far_zero(P, lw.jkr_Cf, xif, Xi, xjf)) continue;
             if (sdrop && sjkr_far_zero(P, lw, xif, Xi, xjf)) continue;
@@ -1421,7 +1443,6 @@ __device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const 
       // wall candidates: the triangles of its triangle-grid cell that pass
       // the FP32 pretest, counted here and listed once the arena is reserved
       if (walled) {
-        Xi = fmaxf(fmaxf(fabsf(xif.x), fabsf(xif.y)), fabsf(xif.z));
         gi = P.ngroups > 1 ? B.grp[k] : 0u;
         for (uint32_t t = ts; t < te; t += 4) {
           const uint32_t pass = wall_pretest4(P, t, te, gi, xif, Xi);

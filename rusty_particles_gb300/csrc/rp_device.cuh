@@ -204,6 +204,9 @@ struct StepParams {
   // cut_b); the lists hold it plus the skin
   float cut_a, cut_b;
   float cutmaxf;     // the largest such distance: 2 r_max cut_a
+  // |coordinate| up to which a sphere counts as inside or next to the box, and
+  // one beyond which a sphere is out of reach of those, images included
+  float xhome, xnear;
   // adhesive pairs whose normal force is certainly zero are left out: their
   // tangential force vanishes too (Coulomb with |F_n| = 0; physical springs
   // reset out of contact), while parity-mode springs (G* = 0, NaN for Mindlin

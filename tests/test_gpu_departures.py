@@ -192,3 +192,54 @@ def test_diagnostics_of_a_call_that_removed_spheres(rp, oracle_mod):
         assert pu.pair_counter_gpu(g) == pu.pair_counter_oracle(o)
         assert o.get_particle_count() < n0 or steps == 1
     assert g.stats()["compactions"] >= 1
+
+
+def test_spheres_that_have_flown_off_touch(rp, oracle_mod):
+    # nothing is removed above the box: pairs from the box's top to 200 m above
+    # it, turned every way, touching by 1e-6 to 1e-3 of a radius or just apart
+    # (the pretest's margin is its own for pairs outside the box and one for all
+    # inside, and both ends of a pair must take the same one)
+    rng = np.random.default_rng(17)
+    lo, hi = np.array([-0.2, -0.2, -0.2]), np.array([0.2, 0.2, 0.2])
+    x, r = [], []
+    for k in range(600):
+        y = 10.0 ** rng.uniform(-1.2, 2.3) if k % 2 else rng.uniform(0.2, 0.45)
+        c = np.array([0.05 * (k % 8) - 0.18, y, 0.05 * (k // 8 % 8) - 0.18])
+        u = rng.normal(size=3)
+        u /= np.linalg.norm(u)
+        ra = rng.uniform(0.008, 0.012, 2)
+        gap = ra.sum() * (1.0 + rng.choice([-1, 1]) * 10.0 ** rng.uniform(-6, -3))
+        x += [c, c + gap * u]
+        r += list(ra)
+    x, r = np.array(x), np.array(r)
+    st = _state(x, r, rng.normal(0, 0.1, (len(x), 3)), rng.normal(0, 1.0, (len(x), 3)))
+    o = pu.oracle_sim(oracle_mod, st, 1e-6, lo, hi, 1, 0, mode=1)
+    g = pu.gpu_sim(rp, st, 1e-6, lo, hi, 1, 0, mode=1)
+    for step in range(5):
+        o.step()
+        g.step()
+        so, sg = o.state(), g.get_state()
+        FS, TS = o.last_force_scale()
+        assert np.all(np.abs(sg["acceleration"] - so["a"]).max(1) <= 1e-9 * (FS / so["m"] + 10.0)), step
+        assert np.all(np.abs(sg["torque"] - so["tau"]).max(1) <= 1e-9 * TS + 1e-25), step
+    assert pu.pair_counter_gpu(g) == pu.pair_counter_oracle(o)
+    assert np.count_nonzero((FS > 0) & (so["x"][:, 1] > 1.0)) > 50
+
+
+def test_sphere_far_away_slows_nobody(rp):
+    lo, hi = (-0.6, -0.6, -0.6), (0.6, 0.6, 0.6)
+    st = pu.random_bed(6, 300_000, lo, hi, 0.0085, 0.0088, vscale=0.05, ascale=0.0, tscale=0.0)
+    took = []
+    for far in (False, True):
+        g = pu.gpu_sim(rp, st, 1e-6, lo, hi, 1, 0)
+        g.set_debug(False)
+        if far:
+            g.add_particle(0.0, 1e7, 0.0, 0.001, 1.0, True)
+        g.steps(20)
+        t = []
+        for _ in range(7):
+            a = g.stats()["device_ms"]
+            g.steps(20)
+            t.append(g.stats()["device_ms"] - a)
+        took.append(sorted(t)[3])
+    assert took[1] < 1.2 * took[0], took
