@@ -108,6 +108,7 @@ typedef struct rp_stats {
 #define RP_STATUS_NAN_FORCE 2u  /* a non-finite particle force */
 #define RP_STATUS_NLIST_GROW 4u /* a neighbour list outgrew its capacity (recovered) */
 #define RP_STATUS_WALL_GROW 8u  /* the wall contact candidates outgrew their buffer (recovered) */
+#define RP_STATUS_PAIR_GROW 32u /* the list of evaluated contacts outgrew its capacity (recovered) */
 #define RP_STATUS_STUCK 16u     /* the blocks of a small bed's step loop did not meet in time (the call fails) */
 
 /* --- lifecycle: Simulation.create (src/lib.rs:57, src/simulation.rs:62-91) */

@@ -149,7 +149,8 @@ void Engine::free_device() {
   dfree(id_part_);
   io_n_ = 0;
   jq_alloc_ = 0;
-  jfb_alloc_ = 0;
+  jfb_alloc_ = jhard_alloc_ = 0;
+  ccap_ = hcap_ = 0;
   dfree(ctrl_);
   if (ctrl_h_) cudaFreeHost(ctrl_h_);
   if (pin_buf_) cudaFreeHost(pin_buf_);
@@ -421,27 +422,52 @@ int Engine::alloc_lists(int cap, bool keep_current) {
     dfree(dbgMult_);
   }
   TRY(dalloc(&crec_, na * (size_t)cap));
-  TRY(dalloc(&clist_, na * (size_t)cap));
   TRY(dalloc(&cres_, 6 * na * (size_t)cap));
   cap_ = cap;
   graph_dirty_ = true;
-  refresh_list_ptrs();
-  TRY(ensure_jkr_buffers());
+  TRY(alloc_pairs(0, 0));
   return RP_OK;
 }
 
-// Network queue and per-record predictions (one entry per possible
-// evaluating record) and the device copy of the network, for the learned
-// JKR solver only.
+// The lists of evaluating records: clist_ and, for the certified JKR solvers,
+// jhard_ and the buffers indexed like them. At most one end of a pair evaluates
+// it and rows have room to spare (32 places, while touching equal spheres have at
+// most 12 neighbours, 6 pairs a sphere), so they start at a quarter of the rows'
+// places, jhard_ at an eighth of that, and a filter that finds them
+// full halts the step (HALT_PAIRS) and recover_halt grows them. A record in
+// clist_ takes 16 bytes: with a place of its own for each of the rows' a
+// million spheres took 384 MB more, two million adhesive ones 1.9 GB.
+int Engine::alloc_pairs(size_t cap, size_t hard) {
+  const size_t places = std::min<size_t>(n_alloc_ * (size_t)std::max(cap_, 1), 0xFFFFFFF0u);
+  cap = std::min(std::max({cap, ccap_, places / 4, std::min<size_t>(places, 65536)}), places);
+  hard = std::min(std::max({hard, hcap_, cap / 8, std::min<size_t>(places, 16384)}), places);
+  if (!clist_ || cap != ccap_) {
+    ccap_ = 0;
+    TRY(dalloc(&clist_, cap));
+    ccap_ = cap;
+  }
+  hcap_ = hard;
+  graph_dirty_ = true;
+  refresh_list_ptrs();
+  return ensure_jkr_buffers();
+}
+
+// The certified JKR solvers' lists beside clist_ and, for the learned one, the
+// network queue, the predictions and the device copy of the network.
 int Engine::ensure_jkr_buffers() {
   // pairs left to the reference's Newton by the certified solvers
   const bool defer = gpu_ && jkr_solver != RP_JKR_NEWTON && nmodel == RP_NORMAL_JKR;
   if (defer) {
-    const size_t need = std::max<size_t>(n_alloc_ * (size_t)std::max(cap_, 1), 1);
-    if (jfb_alloc_ < need) {
-      TRY(dalloc(&jfb_, need));
-      TRY(dalloc(&jhard_, need));
-      jfb_alloc_ = need;
+    if (jfb_alloc_ < ccap_) {
+      jfb_alloc_ = 0;
+      TRY(dalloc(&jfb_, ccap_));
+      jfb_alloc_ = ccap_;
+      graph_dirty_ = true;
+    }
+    if (jhard_alloc_ < hcap_) {
+      jhard_alloc_ = 0;
+      TRY(dalloc(&jhard_, hcap_));
+      jhard_alloc_ = hcap_;
       graph_dirty_ = true;
     }
     P_.jfb = jfb_;
@@ -453,11 +479,11 @@ int Engine::ensure_jkr_buffers() {
     P_.mlp = nullptr;
     return RP_OK;
   }
-  const size_t need = std::max<size_t>(n_alloc_ * (size_t)std::max(cap_, 1), 1);
-  if (jq_alloc_ < need) {
-    TRY(dalloc(&jq_, need));
-    TRY(dalloc(&jguess_, need));
-    jq_alloc_ = need;
+  if (jq_alloc_ < ccap_) {
+    jq_alloc_ = 0;
+    TRY(dalloc(&jq_, ccap_));
+    TRY(dalloc(&jguess_, ccap_));
+    jq_alloc_ = ccap_;
     graph_dirty_ = true;
   }
   if (!mlp_d_) {
@@ -480,6 +506,8 @@ void Engine::refresh_list_ptrs() {
   P_.dbgMult = dbgMult_;
   P_.crec = crec_;
   P_.clist = clist_;
+  P_.ccap = (uint32_t)ccap_;
+  P_.hcap = (uint32_t)hcap_;
   P_.cres = cres_;
   P_.cresf = reinterpret_cast<float*>(cres_);
   P_.ccnt = ccnt_;
@@ -913,7 +941,7 @@ int Engine::upload() {
   if (n > n_alloc_ || n_alloc_ == 0) TRY(alloc_slots(n));
   if (cap_ == 0) cap_ = 32;
   const bool need_hist = (mode == RP_MODE_PHYSICAL && tmodel != RP_TANGENTIAL_COULOMB);
-  if (!bank_[0].nbr || (need_hist && !bank_[0].hist) || (debug && !dbgMult_)) TRY(alloc_lists(cap_, false));
+  if (!bank_[0].nbr || !crec_ || !cres_ || !clist_ || (need_hist && !bank_[0].hist) || (debug && !dbgMult_)) TRY(alloc_lists(cap_, false));
   // pack
   const size_t na = std::max<size_t>(n, 1);
   std::vector<D4> a8[8];
@@ -1071,12 +1099,21 @@ int Engine::recover_halt() {
       CK(cudaMemcpyAsync(&ctrl_->spin_due, &none, sizeof(int), cudaMemcpyHostToDevice, stream_));
       tot_.status |= ST_WALL_GROW;
     }
+    if (ctrl_h_->halt & HALT_PAIRS) {
+      TRY(alloc_pairs(ctrl_h_->pair_need > ccap_ ? std::max<size_t>(2 * ccap_, (size_t)ctrl_h_->pair_need * 5 / 4) : ccap_,
+                      ctrl_h_->hard_need > hcap_ ? std::max<size_t>(2 * hcap_, (size_t)ctrl_h_->hard_need * 5 / 4) : hcap_));
+      const int none = 0;  // that filter has kicked the spins
+      CK(cudaMemcpyAsync(&ctrl_->spin_due, &none, sizeof(int), cudaMemcpyHostToDevice, stream_));
+      tot_.status |= ST_PAIR_GROW;
+    }
     graph_dirty_ = true;
     int zero = 0;
     unsigned zu = 0;
     CK(cudaMemcpyAsync(&ctrl_->halt, &zero, sizeof(int), cudaMemcpyHostToDevice, stream_));
     CK(cudaMemcpyAsync(&ctrl_->max_count, &zu, sizeof(unsigned), cudaMemcpyHostToDevice, stream_));
     CK(cudaMemcpyAsync(&ctrl_->wall_need, &zu, sizeof(unsigned), cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpyAsync(&ctrl_->pair_need, &zu, sizeof(unsigned), cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpyAsync(&ctrl_->hard_need, &zu, sizeof(unsigned), cudaMemcpyHostToDevice, stream_));
     CK(cudaStreamSynchronize(stream_));
     launches_ += launch_rebuild(P_, rb_, stream_);
     launches_ += launch_force(P_, stream_, side_);

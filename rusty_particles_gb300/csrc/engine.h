@@ -163,6 +163,8 @@ class Engine {
   uint8_t* wok_ = nullptr;      // their contact flags
   uint32_t *woff_ = nullptr, *wcnt_ = nullptr;
   size_t wcap_ = 0;
+  size_t ccap_ = 0, hcap_ = 0;  // entries of clist_ (and the buffers beside it) and of jhard_
+  int alloc_pairs(size_t cap, size_t hard);
   uint32_t *ctot_ = nullptr;
   double* cres_ = nullptr;
   void refresh_list_ptrs();
@@ -179,7 +181,7 @@ class Engine {
   uint32_t* jfb_ = nullptr;    // pairs deferred to the reference-Newton pass
   uint4* jhard_ = nullptr;  // pairs that the filter sends to it at once
   SideStream side_;
-  size_t jfb_alloc_ = 0;
+  size_t jfb_alloc_ = 0, jhard_alloc_ = 0;
   int ensure_jkr_buffers();
   int step_kernels_ = 4;  // kernels of one device-loop step outside the rebuild chain
   TriRec* tri_d_ = nullptr;

@@ -1498,6 +1498,12 @@ __device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const 
       P.woff[k] = wb;
     }
     if (ncmp + nhard == 0) continue;
+    if (q + ncmp > P.ccap || (hint_any && qh + nhard > P.hcap)) {  // the host grows the lists and runs the step again
+      atomicMax(&C->pair_need, q + ncmp);
+      if (hint_any) atomicMax(&C->hard_need, qh + nhard);
+      atomicOr(&C->halt, HALT_PAIRS);
+      continue;
+    }
     // the evaluating records into the compact list, read back from the row that
     // this thread just wrote
     const CRec* out = P.crec + (size_t)k * P.cap;
@@ -1527,7 +1533,7 @@ __device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const 
 template <bool PHYS, bool HIST>
 __global__ void __launch_bounds__(256, 4) k_contact_filter(StepParams P) {
   Ctrl* C = P.ctrl;
-  // a full wall buffer that another block reports must not keep this one from
+  // a full buffer that another block reports must not keep this one from
   // its spin kicks (the device loop ends with the step that halts)
   if (C->spin_due ? (C->halt & HALT_LISTS) : C->halt) return;
   filter_pass<PHYS, HIST, false>(P, C, P.bank[C->bank], P.ctot, grid_span());
@@ -2373,7 +2379,7 @@ template <bool PHYS, bool HIST, typename R>
 __global__ void __launch_bounds__(SMALL_BLOCK, 1) k_steps(StepParams P) {
   Ctrl* C = P.ctrl;
   volatile Ctrl* W = C;
-  // (a resumed launch filters before its first barrier: a full wall buffer that
+  // (a resumed launch filters before its first barrier: a full buffer that
   // another block reports meanwhile must not keep this one from the barrier)
   if (W->halt & (HALT_LISTS | HALT_STUCK)) return;
   constexpr bool FP64 = sizeof(R) == sizeof(double);
@@ -2412,7 +2418,7 @@ __global__ void __launch_bounds__(SMALL_BLOCK, 1) k_steps(StepParams P) {
     resume = false;
     filter_pass<PHYS, HIST, true>(P, C, B, ctot, sp);
     if (!grid_barrier(C, gen, blocks)) return;
-    if (W->halt) {  // the wall candidates outgrew their buffer: the host finishes this step
+    if (W->halt) {  // a buffer of the filter is full: the host finishes this step
       if (first) W->resume = 0;
       return;
     }

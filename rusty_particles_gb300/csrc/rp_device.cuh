@@ -27,7 +27,7 @@ struct alignas(32) D4 {
 //              cell (parity mode; implies PF_NOIMAGE)
 enum : uint32_t { PF_FIXED = 1u, PF_DEAD = 2u, PF_WALLFAR = 4u, PF_NOIMAGE = 8u, PF_ONECELL = 16u };
 
-enum : unsigned { ST_OVERLAP = 1u, ST_NAN = 2u, ST_NLIST_GROW = 4u, ST_WALL_GROW = 8u, ST_STUCK = 16u };
+enum : unsigned { ST_OVERLAP = 1u, ST_NAN = 2u, ST_NLIST_GROW = 4u, ST_WALL_GROW = 8u, ST_STUCK = 16u, ST_PAIR_GROW = 32u };
 
 // Device control block: written by kernels, read by the host after a chunk.
 struct Ctrl {
@@ -43,6 +43,7 @@ struct Ctrl {
   unsigned long long overlap_steps;
   int pending;                    // the last completed step still owes its second half kick
   unsigned int wall_need;         // wall candidates a halted filter wanted room for
+  unsigned int pair_need, hard_need;  // and evaluating records, for clist and jhard
   int spin_due;                   // the step's first half left the spin kicks to the contact filter
   unsigned int bar;               // k_steps: blocks that have arrived at its grid barriers
   int resume;                     // k_steps: the current step's first half is done (it stopped for a rebuild)
@@ -83,6 +84,8 @@ constexpr int HALT_LISTS = 1;
 constexpr int HALT_WALLS = 2;
 // a grid barrier of k_steps ran out of its bounded wait (an error, not recovered)
 constexpr int HALT_STUCK = 4;
+// the evaluating records outgrew their list (contact filter)
+constexpr int HALT_PAIRS = 8;
 
 // A rigid surface velocity V + W x (p - C) of a set of triangles whose geometry
 // stays put (a surface of revolution turning about its own axis, a belt). The
@@ -163,6 +166,7 @@ struct StepParams {
   uint32_t wcap;    // wall candidate capacity
   uint32_t* coff;   // first result slot of particle k (its ccnt results are contiguous)
   uint4* clist;     // compact list of evaluating records: slot, partner, m and visits, result slot
+  uint32_t ccap, hcap;  // capacity of clist (and of jfb, jq, jguess) and of jhard
   // [0] records, [1] evaluating records, [2] network queue, [3] deferred pairs, [4] wall candidates, [5] hard pairs
   uint32_t* ctot;   // (k_steps alternates between two such sets)
   uint32_t* jfb;    // entries of clist deferred to the reference-Newton pass (null: no deferral)
