@@ -961,6 +961,8 @@ int Engine::upload() {
     // correctly rounded division the step would do)
     a8[7][i] = D4{p.wres[0], p.wres[1], p.wres[2], 1.0 / (0.4 * p.m * p.r * p.r)};
     flags[i] = p.fixed ? PF_FIXED : 0u;
+    if (!(std::isfinite(p.w[0]) && std::isfinite(p.w[1]) && std::isfinite(p.w[2]) && std::isfinite(a8[7][i].w)))
+      flags[i] |= PF_KICK;
     tags[i] = (uint32_t)i;  // the device tag is the id at upload; the insertion tag stays on the host
   }
   up_tags_.resize(n);
@@ -1424,6 +1426,7 @@ int Engine::append_on_device(size_t k, const double* xyz, const double* r, const
     a8[6][i] = D4{0.0, 0.0, 0.0, 1.0 / m[i]};
     a8[7][i] = D4{0.0, 0.0, 0.0, 1.0 / (0.4 * m[i] * r[i] * r[i])};
     flags[i] = (fixed && fixed[i]) ? PF_FIXED : 0u;
+    if (!std::isfinite(a8[7][i].w)) flags[i] |= PF_KICK;
     tags[i] = (uint32_t)(n_upload_ + i);
     xf[i] = make_float4((float)xyz[3 * i], (float)xyz[3 * i + 1], (float)xyz[3 * i + 2], (float)r[i]);
   }

@@ -707,7 +707,7 @@ __device__ __forceinline__ bool first_half_pass(const StepParams& P, Ctrl* C, co
       // away and, where that holds for a whole warp, 30 of the ~90 FP64
       // instructions (decided by the warp: lanes going apart cost more)
       if (SPIN) {
-        own_spin = some_bits(tau) || (KAHAN && some_bits(wres));
+        own_spin = some_bits(tau) || (KAHAN && some_bits(wres)) || (fl & PF_KICK);
         spin = __any_sync(__activemask(), own_spin);
       }
       if (spin) dw = KAHAN ? (tau * inv_inertia) * kdt : tau * (inv_inertia * kdt);
@@ -804,11 +804,11 @@ __global__ void __launch_bounds__(KAHAN ? 128 : 256, KAHAN ? (SPIN ? 5 : 7) : 5)
 // FP64 form only (us a step with / without: hopper 1 M 687 / 716, gas 1 M 270 /
 // 305, boxes 1.6 M 907 / 945): the mixed form's spin is 9 FP64 instructions, not
 // 30, and the filter's extra traffic costs more (drum 4.2 M 1499 / 1450).
-__device__ __forceinline__ void spin_kick(const StepParams& P, const Bank& B, int k, bool fuse) {
+__device__ __forceinline__ void spin_kick(const StepParams& P, const Bank& B, int k, uint32_t fl, bool fuse) {
   const D4 wr4 = B.wres[k];
   const V tau = xyz(B.tq[k]);
   V wres = xyz(wr4);
-  if (!(some_bits(tau) || some_bits(wres))) return;
+  if (!(some_bits(tau) || some_bits(wres) || (fl & PF_KICK))) return;
   double* at = &B.wc[k].x;
   const double2 w0 = *reinterpret_cast<const double2*>(at);
   V w = vmk(w0.x, w0.y, at[2]);
@@ -1336,7 +1336,7 @@ __device__ __forceinline__ void filter_pass(const StepParams& P, Ctrl* C, const 
       const uint32_t cnt = B.ncnt[k];
       const uint32_t* row = B.nbr + (size_t)k * P.cap;
       CRec* out = P.crec + (size_t)k * P.cap;
-      if (kick && !(flk & PF_FIXED)) spin_kick(P, B, k, fuse);
+      if (kick && !(flk & PF_FIXED)) spin_kick(P, B, k, flk, fuse);
       const bool wide = (P.cap & 3) == 0;  // rows on 16 bytes
       // where latency is all that counts, the first eight entries come with the
       // particle itself (a dilute bed of a million would read rows it does not have)
@@ -2242,7 +2242,7 @@ __device__ __forceinline__ bool first_half_quad(const StepParams& P, Ctrl* C, co
     }
   }
   const double dt = P.dt, hdt = P.hdt, inv_inertia = quad_word(wres, 3);
-  const unsigned spinning = __ballot_sync(ALL, moving && (nonzero_bits(tau) || (KAHAN && nonzero_bits(wres))));
+  const unsigned spinning = __ballot_sync(ALL, moving && (nonzero_bits(tau) || (KAHAN && nonzero_bits(wres)) || (fl & PF_KICK)));
   const bool own_spin = (spinning & quad_mask()) != 0;
   const double kdt = (!KAHAN && fuse) ? dt : hdt;
   const double dv = a * kdt;
@@ -2780,6 +2780,11 @@ __global__ void k_state_scatter(StepParams P, const uint32_t* slot_of, StateIO i
         d.z = io.v[q][3 * (size_t)i + 2];
         dst[q][k] = d;
       }
+    if (io.v[2]) {
+      const uint32_t fl = B.flags[k] & ~PF_KICK;
+      const V w = xyz(B.wc[k]);
+      B.flags[k] = finite_bits(w.x) && finite_bits(w.y) && finite_bits(w.z) && finite_bits(B.wres[k].w) ? fl : fl | PF_KICK;
+    }
     if (io.v[0]) {
       const D4 x = B.xr[k];
       B.xf[k] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);

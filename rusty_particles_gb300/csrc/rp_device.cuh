@@ -25,7 +25,9 @@ struct alignas(32) D4 {
 //   PF_NOIMAGE no pair of the slot is a periodic image
 //   PF_ONECELL every partner within reach lies in the slot's own reference
 //              cell (parity mode; implies PF_NOIMAGE)
-enum : uint32_t { PF_FIXED = 1u, PF_DEAD = 2u, PF_WALLFAR = 4u, PF_NOIMAGE = 8u, PF_ONECELL = 16u };
+// Set with the state: PF_KICK, an infinite or NaN spin or 1 / I, whose kick by a
+// torque of zero is not nothing (inf - inf, 0 inf)
+enum : uint32_t { PF_FIXED = 1u, PF_DEAD = 2u, PF_WALLFAR = 4u, PF_NOIMAGE = 8u, PF_ONECELL = 16u, PF_KICK = 32u };
 
 enum : unsigned { ST_OVERLAP = 1u, ST_NAN = 2u, ST_NLIST_GROW = 4u, ST_WALL_GROW = 8u, ST_STUCK = 16u, ST_PAIR_GROW = 32u };
 

@@ -99,3 +99,35 @@ def test_odd_velocities_at_a_wall(rp, oracle_mod):
     so, sg = o.state(), g.get_state()
     for k, q in (("acceleration", "a"), ("torque", "tau"), ("velocity", "v")):
         np.testing.assert_array_equal(_kind(sg[k]), _kind(so[q]), err_msg=k)
+
+
+@pytest.mark.parametrize("steps", [1, 4])
+@pytest.mark.parametrize("n,normal", [(40, 1), (9000, 1), (300, 3)], ids=["quads", "scalar", "kernels"])
+def test_infinite_spins_in_flight(rp, oracle_mod, n, normal, steps):
+    # spheres that touch nothing: kicked by no torque, an infinite spin turns
+    # into NaN by its compensated sum; set before the first step and in between
+    m = int(np.ceil(n ** (1 / 3)))
+    g3 = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    rng = np.random.default_rng(n)
+    w = rng.normal(0, 1.0, (n, 3))
+    w[::5, 0], w[1::5, 1], w[2::5, 2] = np.inf, -np.inf, np.nan
+    r = np.full(n, 0.005)
+    st = {"position": g3 * 0.02 - 0.25, "radius": r, "mass": 2500.0 * 4.0 / 3.0 * np.pi * r ** 3,
+          "velocity": rng.normal(0, 0.1, (n, 3)), "angular_velocity": w, "acceleration": np.zeros((n, 3)),
+          "torque": np.zeros((n, 3)), "fixed": np.zeros(n, np.uint8)}
+    lo, hi = (-0.6,) * 3, (0.6,) * 3
+    for late in (False, True):
+        first = dict(st, angular_velocity=np.zeros((n, 3))) if late else st
+        o = pu.oracle_sim(oracle_mod, first, 1e-7, lo, hi, normal, 0)
+        g = pu.gpu_sim(rp, first, 1e-7, lo, hi, normal, 0)
+        g.set_debug(False)
+        if late:
+            o.step()
+            g.step()
+            o.set_state({"w": w})
+            g.set_state({"angular_velocity": w})
+        o.steps(steps)
+        g.steps(steps)
+        so, sg = o.state(), g.get_state()
+        for k, q in (("angular_velocity", "w"), ("angular_velocity_residual", "wres"), ("velocity", "v")):
+            np.testing.assert_array_equal(sg[k], so[q], err_msg=k)
