@@ -2787,7 +2787,16 @@ __global__ void k_state_scatter(StepParams P, const uint32_t* slot_of, StateIO i
     }
     if (io.v[0]) {
       const D4 x = B.xr[k];
-      B.xf[k] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
+      const float4 xf = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
+      B.xf[k] = xf;
+      // farther beyond a periodic face than a step leaves it, the minimum image
+      // of its displacement does not show where it is: the lists are rebuilt,
+      // and with them the flags that rule images out
+      const float p[3] = {xf.x, xf.y, xf.z};
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+        if (P.periodic[a] && ((float)P.bmin[a] - p[a] > P.half_skinf || p[a] - (float)P.bmax[a] > P.half_skinf))
+          P.ctrl->rebuild = 1;
     }
   }
 }

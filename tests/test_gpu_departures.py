@@ -233,6 +233,7 @@ def test_sphere_far_away_slows_nobody(rp):
     for far in (False, True):
         g = pu.gpu_sim(rp, st, 1e-6, lo, hi, 1, 0)
         g.set_debug(False)
+        g.set_skin(0.009)  # rows of 18, six of them near
         if far:
             g.add_particle(0.0, 1e7, 0.0, 0.001, 1.0, True)
         g.steps(20)
@@ -243,3 +244,32 @@ def test_sphere_far_away_slows_nobody(rp):
             t.append(g.stats()["device_ms"] - a)
         took.append(sorted(t)[3])
     assert took[1] < 1.2 * took[0], took
+
+
+@pytest.mark.parametrize("skin", [0.0, 0.03])
+def test_sphere_written_whole_periods_away(rp, oracle_mod, skin):
+    # positions written between calls that lie two box lengths off: the step
+    # wraps them by one, so the spheres meet their neighbours as periodic images
+    # in the middle of the box, although nothing has moved by the minimum image
+    lo, hi = (-0.2, -0.2, -0.2), (0.2, 0.2, 0.2)
+    st = pu.random_bed(19, 3000, lo, hi, 0.0125, 0.0135, vscale=0.05, ascale=0.0, tscale=0.0)
+    per = (True, False, True)
+    o = pu.oracle_sim(oracle_mod, st, 1e-6, lo, hi, 1, 0, per, mode=1)
+    g = pu.gpu_sim(rp, st, 1e-6, lo, hi, 1, 0, per, mode=1)
+    if skin:
+        g.set_skin(skin)
+    o.step()
+    g.step()
+    x = g.get_state()["position"]
+    x[::7, 0] += 0.8
+    x[3::7, 2] -= 0.8
+    o.set_state({"x": x})
+    g.set_state({"position": x})
+    for step in range(3):
+        o.step()
+        g.step()
+        so, sg = o.state(), g.get_state()
+        FS, TS = o.last_force_scale()
+        np.testing.assert_allclose(sg["position"], so["x"], rtol=0, atol=1e-12)
+        assert np.all(np.abs(sg["acceleration"] - so["a"]).max(1) <= 1e-9 * (FS / so["m"] + 10.0)), step
+    assert np.count_nonzero(FS[::7]) > 100
