@@ -2,12 +2,14 @@
 // step's second half kick, boundary rule, half kick + drift), the pair/wall
 // force gather, the end-of-step bookkeeping and the closing second half kick.
 //
-// This translation unit is compiled with -fmad=false: every double operation
-// rounds exactly as the oracle's (-ffp-contract=off), so positions after the
-// first half, cutoff decisions, normals and relative velocities are
-// bit-identical to the reference algorithm evaluated in FP64 from the same
-// state. Force magnitudes differ only where a transcendental is evaluated
-// differently (delta^1.5 as delta*sqrt(delta)), well inside 1e-9 relative.
+// This translation unit is compiled with -fmad=false: in parity mode every
+// double operation rounds exactly as the oracle's (-ffp-contract=off), so
+// positions after the first half, cutoff decisions, normals and relative
+// velocities are bit-identical to the reference algorithm evaluated in FP64 from
+// the same state. Force magnitudes differ only where a transcendental is
+// evaluated differently (delta^1.5 as delta*sqrt(delta)), well inside 1e-9
+// relative. Physical mode has no such counterpart: its FP64 pair law is written
+// with fused multiply-adds (pair_contact_fused).
 //
 // Precision forms of the pair force (StepParams::prec):
 //   FP64  — all pair math in double.
@@ -30,8 +32,8 @@ __device__ __forceinline__ V xyz(const D4& d) { return V{d.x, d.y, d.z}; }
 // with the products that every contact of a group would form again: (4/3) E*,
 // 2 E* and 1.5 pi gamma, each rounded as the laws' own left-to-right product.
 // With the reduced mass formed only by the laws that damp with it and the
-// quotients below in the wall contact: 96 beds of 10,648 adhesive spheres 887
-// to 855 us a step, 22,680 of them 33.0 to 31.8, 4.2 million Hertz spheres in
+// quotients below in the wall contact: 1,636,935 adhesive spheres in 96 boxes 887
+// to 855 us a step, 23,457 in one 33.0 to 31.8, 4.2 million Hertz spheres in
 // mixed precision 1391 to 1354.
 template <typename R> __device__ __forceinline__ R law_mu(const Law& L) { return sizeof(R) == 4 ? (R)L.muf : (R)L.mu; }
 template <typename R> __device__ __forceinline__ R law_gs(const Law& L) { return sizeof(R) == 4 ? (R)L.gs_ppf : (R)L.gs_pp; }
@@ -1223,7 +1225,7 @@ __device__ __forceinline__ bool jkr_far_zero(const StepParams& P, float Cf, floa
   const float c23 = jkr_c23(c);
   const float d = sqrtf(fx * fx + fy * fy + fz * fz);
   const float X = fmaxf(Xi, fmaxf(fmaxf(fabsf(xjf.x), fabsf(xjf.y)), fabsf(xjf.z)));
-  // per-axis FP32 difference error <= 6e-8 (2X + 2 cut + L) (as in pretest_far),
+  // per-axis FP32 difference error <= 6e-8 (2X + 2 cut + L) (as in pretest_near),
   // so |d_f - d| <= 1.8e-7 (2X + 3 r_sum + L) + 4e-7 d, radii rounded too
   const float e = (1.8e-7f * (2.0f * X + 3.0f * rsum + P.lmax) + 4e-7f * (d + rsum)) / rs;
   const float x = (rsum - d) / rs;
@@ -1991,33 +1993,6 @@ int launch_accum_order(const StepParams& P, cudaStream_t s) {
   return 1;
 }
 
-// Exclusive scan of one value per thread (blockDim.x a multiple of 32, at
-// most 256); the block total goes to *total. Contains two __syncthreads.
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* wsum, uint32_t* total) {
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  uint32_t inc = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= (uint32_t)o) inc += t;
-  }
-  if (lane == 31) wsum[warp] = inc;
-  __syncthreads();
-  if (warp == 0) {
-    const uint32_t w = lane < nw ? wsum[lane] : 0u;
-    uint32_t wi = w;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, wi, o);
-      if (lane >= (uint32_t)o) wi += t;
-    }
-    if (lane < nw) wsum[lane] = wi - w;
-    if (lane == nw - 1) *total = wi;
-  }
-  __syncthreads();
-  return inc - v + wsum[warp];
-}
-
 // a = g + F (1/m) and tau = 0 + T for one particle, with the debug record and
 // the non-finite check (on the integer pipe, as the +0 of 0 + T).
 __device__ __forceinline__ void finish_particle(const StepParams& P, const Bank& B, Ctrl* C, int k, V F, V T) {
@@ -2200,7 +2175,6 @@ __device__ __forceinline__ bool grid_barrier(Ctrl* C, unsigned& gen, unsigned bl
 __device__ __forceinline__ double quad_word(double v, int word) { return __shfl_sync(0xFFFFFFFFu, v, word, 4); }
 __device__ __forceinline__ float quad_word(float v, int word) { return __shfl_sync(0xFFFFFFFFu, v, word, 4); }
 __device__ __forceinline__ unsigned quad_mask() { return 7u << (threadIdx.x & 28); }  // the three components' lanes
-__device__ __forceinline__ bool nonzero_bits(double x) { return (__double_as_longlong(x) << 1) != 0; }
 __device__ __forceinline__ void kahan_add(double& s, double& r, double d) {
   const double y = d - r;
   const double t = s + y;
@@ -2242,7 +2216,7 @@ __device__ __forceinline__ bool first_half_quad(const StepParams& P, Ctrl* C, co
     }
   }
   const double dt = P.dt, hdt = P.hdt, inv_inertia = quad_word(wres, 3);
-  const unsigned spinning = __ballot_sync(ALL, moving && (nonzero_bits(tau) || (KAHAN && nonzero_bits(wres)) || (fl & PF_KICK)));
+  const unsigned spinning = __ballot_sync(ALL, moving && (!is_zero(tau) || (KAHAN && !is_zero(wres)) || (fl & PF_KICK)));
   const bool own_spin = (spinning & quad_mask()) != 0;
   const double kdt = (!KAHAN && fuse) ? dt : hdt;
   const double dv = a * kdt;
@@ -2518,7 +2492,7 @@ __global__ void k_kinetic(StepParams P, double* out) {
 // rotational, I = 2/5 m r^2), out[1] the summed sphere volumes, *pairs the
 // overlapping pairs counted from both ends over the Verlet lists (the exact
 // FP64 test d^2 < (r_i + r_j)^2 on the minimum image; every such pair is in
-// the lists, which hold all pairs within the cutoff plus the skin).
+// the lists, which reach beyond r_i + r_j by the skin at least).
 __global__ void k_bed_stats(StepParams P, double* out, unsigned long long* pairs) {
   const Bank B = P.bank[P.ctrl->bank];
   double e = 0.0, vol = 0.0;

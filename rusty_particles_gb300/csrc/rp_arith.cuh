@@ -27,11 +27,10 @@ template <typename R, typename S> __device__ __forceinline__ T3<R> cvt(T3<S> a) 
 using V = T3<double>;
 using Vf = T3<float>;
 __device__ __forceinline__ V vmk(double x, double y, double z) { return V{x, y, z}; }
-// isfinite(x) and 0.0 + x from the bits, off the FP64 pipe
+// isfinite(x), x == 0 and 0.0 + x from the bits, off the FP64 pipe
 __device__ __forceinline__ bool finite_bits(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
-__device__ __forceinline__ double plus_zero(double x) {
-  return (__double_as_longlong(x) << 1) == 0 ? 0.0 : x;
-}
+__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+__device__ __forceinline__ double plus_zero(double x) { return is_zero(x) ? 0.0 : x; }
 // whether any component has a bit other than its sign set (is not +-0)
 __device__ __forceinline__ bool some_bits(V a) {
   return ((__double_as_longlong(a.x) | __double_as_longlong(a.y) | __double_as_longlong(a.z)) << 1) != 0;
@@ -156,7 +155,6 @@ __device__ __forceinline__ double div_rn(double a, double b) {
 __device__ __forceinline__ float div_rn(float a, float b) { return a / b; }
 // a / b for each component (b > 0), the divisor's reciprocal formed once. A
 // plane's normal along an axis leaves zeros: they are their own quotients.
-__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
 __device__ __forceinline__ V div_rn(V a, double b) {
   const bool zx = is_zero(a.x), zy = is_zero(a.y), zz = is_zero(a.z);
   if (!((zx || exponent_in(fabs(a.x), QUOT_LO, QUOT_HI)) && (zy || exponent_in(fabs(a.y), QUOT_LO, QUOT_HI)) &&

@@ -52,7 +52,7 @@ struct Ctrl {
   unsigned int xmax;              // bits of the largest |coordinate| of the FP32 mirror since the upload
   unsigned int xout;              // list rebuild: bits of the farthest distance of a particle outside the periodic faces
   unsigned long long target;      // device step loop: run while steps_done < target
-  unsigned long long iters;       // device step loop iterations (bounded by target + 4)
+  unsigned long long iters;       // device step loop iterations (bounded by target + 4; k_steps: 2 target + 8)
   // learned JKR tallies (pair evaluations): network/certified-solver results
   // accepted, certified zeros, reference-Newton fallbacks, network rows, FP32
   // Newton steps, closed-form walks
