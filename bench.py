@@ -958,6 +958,50 @@ def settled_state(rp, wl, mode, precision, jkr, settle, device, log):
     return st
 
 
+FORM_COLUMNS = ["value", "ms_per_step", "e2e", "force_err_sum_scale"]
+
+
+def short_line(line):
+    """The printed line: everything the headline is judged by, the other forms as
+    one row each (FORM_COLUMNS). What explains them (counts, notes, per-form
+    clocks and beds) is in the full record only: 13 KB of it on the line had been
+    cut off by what captures the output, and the value with it."""
+    out = {k: v for k, v in line.items() if k not in ("forms", "stats", "bed", "autotune", "jkr", "roofline", "cpu_baseline",
+                                                      "cpu_baseline_literal", "e2e", "force_err")}
+    out["config"] = {**line["config"], "describe": line["config"].get("describe", "")[:260]}
+
+    def pick(d, keys):
+        return {k: d[k] for k in keys if k in d} if isinstance(d, dict) else d
+
+    roof = line.get("roofline")
+    out["roofline"] = pick(roof, ("bound", "achieved", "peak", "unit", "frac", "traffic", "avg_launch_ms", "peak_source"))
+    if isinstance(roof, dict) and isinstance(roof.get("fp64"), dict):
+        out["roofline"]["fp64"] = pick(roof["fp64"], ("achieved", "peak_fma_per_s", "frac"))
+    for k in ("cpu_baseline", "cpu_baseline_literal"):
+        out[k] = pick(line.get(k), ("value", "unit", "cores", "kind"))
+    out["e2e"] = pick(line.get("e2e"), ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "wall_ms"))
+    out["force_err"] = pick(line.get("force_err"), ("force_rel_sum", "force_rel_net", "torque_rel_sum", "error"))
+    if isinstance(line.get("forms"), dict):
+        rows = {}
+        for bed, forms in line["forms"].items():
+            if not isinstance(forms, dict):
+                rows[bed] = forms
+                continue
+            for name, f in forms.items():
+                if not isinstance(f, dict):
+                    continue
+                if "value" not in f:
+                    if bed == "errors" or name == "errors":
+                        rows[f"{bed}/{name}"] = f
+                    continue
+                fe = f.get("force_err")
+                err = fe.get("force_rel_sum") if isinstance(fe, dict) else None
+                cells = (f["value"], f.get("ms_per_step"), (f.get("e2e") or {}).get("value"), err)
+                rows[f"{bed}/{name}"] = [None if c is None else float(f"{c:.4g}") for c in cells]
+        out["forms"] = {"columns": FORM_COLUMNS, "rows": rows}
+    return out
+
+
 def run_forms(rp, args, dist, device, log, headline_state, hopper_wl, cache, threads, deadline):
     """Every spec form beside the plain one, each on its own benchmark
     workload (see the module docstring); each entry carries its own value,
@@ -1221,7 +1265,12 @@ def run_ours(args, log):
     if forms is not None:
         line["forms"] = forms
     line["bench_wall_s"] = round(time.time() - t_start, 1)
-    print(json.dumps(line), flush=True)
+    try:
+        with open(args.details, "w") as f:
+            json.dump(line, f, indent=1)
+    except OSError as ex:
+        log(f"full record not written: {ex}")
+    print(json.dumps(short_line(line)), flush=True)
     barrier(dist)
     return 0
 
@@ -1260,6 +1309,8 @@ def main():
     ap.add_argument("--host-loop", action="store_true", help="host-issued kernels instead of the device loop")
     ap.add_argument("--skin", type=float, default=None,
                     help="Verlet skin in m for the timed simulations (default: 0.2 of the largest radius)")
+    ap.add_argument("--details", default=os.path.join(ROOT, "bench_details.json"),
+                    help="file for the full record (per-form clocks, counts, notes); the printed line is its summary")
     ap.add_argument("--profile-only", action="store_true", help="warm-up + timed steps only (for ncu)")
     args = ap.parse_args()
     log = (lambda m: print(m, file=sys.stderr, flush=True))
