@@ -82,7 +82,8 @@ __device__ __forceinline__ double f2d_exact(float f) {
 //   close, which is half or three halves of an ulp from q; three halves need a
 //   y, and so the mantissas of a and b, above 1.985. Such quotients go to the
 //   library; without that, 28 of 8 million operands built to lie next to a
-//   midpoint came out an ulp off.
+//   midpoint came out an ulp off. The test costs the reference's JKR Newton, four
+//   quotients a round, 2.7 % (262,144 spheres, 1489 to 1530 us a call of 8 steps).
 // * Reciprocal of the root: one correction from within two ulp misses 1/s only
 //   where s m = 2^106 - 1 for a 54-bit m, that is for s = 2 - 2^-52 and its
 //   multiples by powers of two, which go to the library.
