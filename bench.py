@@ -439,7 +439,9 @@ def relax(rp, wl, stages=9, steps_per_stage=100, settle=300, log=None):
 
 # ------------------------------------------------------------------- clocks
 class ClockSampler:
-    """nvidia-smi samples (200 ms) while the timed region runs."""
+    """nvidia-smi samples (50 ms) from just before the timed region to just after
+    it: a short region (20 steps of the hopper take 7 ms) ends before nvidia-smi
+    has started, so the region waits for the first sample and the end for one more."""
 
     FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
               "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
@@ -455,7 +457,7 @@ class ClockSampler:
         try:
             self.proc = subprocess.Popen(
                 ["nvidia-smi", f"--id={self.device}", f"--query-gpu={self.FIELDS}", "--format=csv,noheader,nounits",
-                 "-lms", "200"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
+                 "-lms", "50"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
         except (OSError, ValueError):
             self.proc = None
             return
@@ -465,6 +467,12 @@ class ClockSampler:
     def _read(self):
         for line in self.proc.stdout:
             self.lines.append(line.strip())
+
+    def wait(self, samples, limit_s=3.0):
+        """Until that many samples are in (or the limit, or nvidia-smi has ended)."""
+        end = time.perf_counter() + limit_s
+        while self.proc and self.proc.poll() is None and len(self.lines) < samples and time.perf_counter() < end:
+            time.sleep(0.002)
 
     def stop(self):
         if not self.proc:
@@ -792,11 +800,14 @@ def timed(sim, steps, dist, device):
     barrier(dist)
     torch.cuda.synchronize()
     clocks.start()
+    clocks.wait(1)
+    barrier(dist)
     t0 = time.perf_counter()
     sim.steps(steps)
     torch.cuda.synchronize()
     wall = time.perf_counter() - t0
     barrier(dist)
+    clocks.wait(len(clocks.lines) + 1, 0.5)
     ck = clocks.stop()
     s1 = sim.stats()
     return s0, s1, wall, ck

@@ -70,3 +70,19 @@ def test_line_without_forms():
     line = bench.short_line(full)
     assert "forms" not in line and line["cpu_baseline"] is None and "fp64" not in line["roofline"]
     assert json.loads(json.dumps(line))["value"] == NUMBER
+
+
+def test_clock_sampler_waits_for_samples(tmp_path, monkeypatch):
+    # a stand-in for nvidia-smi that starts slowly: a region shorter than its start still has samples
+    fake = tmp_path / "nvidia-smi"
+    fake.write_text("#!/bin/sh\nsleep 0.2\nwhile true; do echo '0, 1950, 2070, 700, 0x0, Not Active, Not Active, Not Active, Active'; "
+                    "sleep 0.05; done\n")
+    fake.chmod(0o755)
+    monkeypatch.setenv("PATH", f"{tmp_path}:{os.environ['PATH']}")
+    ck = bench.ClockSampler()
+    ck.start()
+    ck.wait(1)
+    ck.wait(len(ck.lines) + 1, 2.0)
+    got = ck.stop()
+    assert got["samples"] >= 2 and got["sm_mhz"] == 1950.0 and got["sm_max_mhz"] == 2070.0
+    assert got["reasons"] == ["sw_power_cap"]
