@@ -484,13 +484,13 @@ __device__ __forceinline__ double normal_mag_fused(int model, const Law& L, doub
   if (model == 1) {
     // (4/3) E* s delta = (2/3) k_t delta with k_t = 2 E* s, s = sqrt(R* delta)
     if (overlap <= 0.0) return 0.0;
-    const double ms = div_rn(mi * mj, mi + mj);
+    const double ms = div_near(mi * mj, mi + mj);
     const double kt = (2.0 * es) * sqrt_rn(rs * overlap);
     const double cn = sqrt_rn(ms * kt) * (2.0 * L.beta_abs);
     return relu(fma(-cn, vn, (kt * overlap) * (2.0 / 3.0)));
   }
   if (model == 0) {
-    const double ms = div_rn(mi * mj, mi + mj);
+    const double ms = div_near(mi * mj, mi + mj);
     const double kn = es * rs;
     return relu(fma(kn, overlap, -(0.5 * sqrt_rn(ms * kn)) * vn));
   }
@@ -545,7 +545,7 @@ __device__ __forceinline__ void pair_contact_fused(const StepParams& P, const La
                    fma(n.x, W.y, fma(-W.x, n.y, u.z)));
   const double vn = dot_fma(rv, n);
   const V vt = mad(-vn, n, rv);
-  const double rs = div_rn(ri * rj, rsum);
+  const double rs = div_near(ri * rj, rsum);
   double fm = 0.0;
   if (JKR) {
     int kind = JKR_FALLBACK;
@@ -585,7 +585,7 @@ __device__ __forceinline__ void pair_contact_fused(const StepParams& P, const La
       V ft = trial;
       if (t2 > fc * fc) {
         ft = t2 > 1e-12 ? (fc * rsqrt(t2)) * trial : vmk(0.0, 0.0, 0.0);
-        xi = (-div_rn(1.0, kt)) * ft;
+        xi = (-div_near(1.0, kt)) * ft;
       }
       nf = cross_fma(n, ft);
       f = f + ft;

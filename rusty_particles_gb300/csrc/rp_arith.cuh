@@ -145,6 +145,14 @@ __device__ __forceinline__ bool near_midpoint(double a, double b, double q, doub
   return hr - hb - eq + (1076u << 20) + 1u < 3u ||
          ((ha & hb & 0x000FC000u) == 0x000FC000u && (hr & 0x7FF00000u) + (52u << 20) >= (ha & 0x7FF00000u));
 }
+// a / b, rounded the other way at most next to a midpoint: for physical mode's
+// fused law, which has no counterpart to agree with bit for bit
+__device__ __forceinline__ double div_near(double a, double b) {
+  if (!(exponent_in(fabs(a), QUOT_LO, QUOT_HI) && exponent_in(fabs(b), QUOT_LO, QUOT_HI))) return a / b;
+  const double y = rcp_step(b);
+  const double q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
 __device__ __forceinline__ double div_rn(double a, double b) {
   if (!(exponent_in(fabs(a), QUOT_LO, QUOT_HI) && exponent_in(fabs(b), QUOT_LO, QUOT_HI))) return a / b;
   const double y = rcp_step(b);

@@ -22,6 +22,7 @@ __global__ void k_probe(int op, size_t n, const double* a, const double* b, doub
       case 10: r = relu(a[i]); break;
       case 11: r = finite_bits(a[i]) ? 1.0 : 0.0; break;
       case 12: r = plus_zero(a[i]); break;
+      case 13: r = div_near(a[i], b[i]); break;
     }
     out[i] = r;
   }

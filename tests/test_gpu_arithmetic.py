@@ -117,6 +117,10 @@ def test_quotients(probe):
     with np.errstate(all="ignore"):
         want = ra / rb
     _same(probe(3, ra, rb), want, ra, rb)
+    near = probe(13, ra, rb)  # physical mode's: an ulp off at most, and only next to a midpoint
+    off = np.where(np.isfinite(want), np.abs(_bits(near).astype(np.int64) - _bits(want).astype(np.int64)), 0)
+    assert off.max() <= 1 and np.count_nonzero(off[n:n + 2 * R]) == 0  # (none among the random operands)
+    np.testing.assert_array_equal(np.isnan(near), np.isnan(want))
     pos = rb > 0  # the vector form divides by a positive length
     for op in (4, 5):
         _same(probe(op, ra[pos], rb[pos]), want[pos], ra[pos], rb[pos])
