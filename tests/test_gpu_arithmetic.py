@@ -15,7 +15,6 @@ Comparisons stand for the floating ones, which are false for a NaN of either sig
 """
 import ctypes
 import os
-import shutil
 import subprocess
 
 import numpy as np
